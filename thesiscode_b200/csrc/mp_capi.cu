@@ -399,6 +399,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
         unsigned long long* kex = cv.take<unsigned long long>(PL * shards);
         unsigned long long* kid = cv.take<unsigned long long>(PL * shards);
         double* thr = cv.take<double>(PL + kFp64ThrPad);
+        unsigned* counter = cv.take<unsigned>(1);
         double* d2 = o_dev ? dist2_out : cv.take<double>(PL);
         int64_t* ix = o_dev ? idx_out : cv.take<int64_t>(PL);
 
@@ -455,6 +456,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             P.thr = thr;
             P.thr_eps = fp64_threshold_eps(P.idx_bits);
             P.thr_tiny = fp64_threshold_tiny(P.m);
+            P.counter = counter;
             launch_band(R, P, st);
             MP_LAUNCHED(ctx);
         }
@@ -882,6 +884,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     double* sv = cv.take<double>(T);
     double* mv = cv.take<double>(T);
     double* thr = cv.take<double>(region + kFp64ThrPad);
+    unsigned* counter = cv.take<unsigned>(1);
     const cudaMemcpyKind K = cudaMemcpyDefault;
     MP_CUDA(ctx, cudaMemcpyAsync(ah, A_hor, 8 * (T + m), K, st));
     MP_CUDA(ctx, cudaMemcpyAsync(av, A_vert, 8 * (T + m), K, st));
@@ -939,6 +942,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     P.thr = thr;
     P.thr_eps = fp64_threshold_eps(ib);
     P.thr_tiny = fp64_threshold_tiny(P.m);
+    P.counter = counter;
     launch_band(R, P, st);
     MP_LAUNCHED(ctx);
     block_finalize_kernel<<<grid_for(region), kThreads, 0, st>>>(kex, kid, region, 1, region, ib,

@@ -16,30 +16,48 @@
 //
 // Work layout (B200): lane l of a warp owns diagonals g0 + a, a < R,
 // g0 = band start + l*R; all lanes walk the same column j.  Per step a lane
-// evaluates R cells: the column maximum over the warp comes from two warp
-// reductions (high, then low word of the ordered score), the row maxima
-// accumulate in registers for R steps and then pass through a per-warp shared
-// memory ring (one writer per slot per chunk, no atomics) until the warp's
-// lowest lane has seen the row.  Finished rows and columns go to global
-// memory as 64-bit max reductions into one of several key shards.  One
-// resident wave of warps walks the bands in a snake order (band b to warp
-// b mod W in even rounds, W-1 - b mod W in odd ones), so every warp's bands
-// add up to nearly the same length -- the reference's triv_par balance rule
-// (ScrimpTrivialPar.cpp:200-224) carried over any number of rounds.
+// evaluates R cells; no two of a step's 32*R cells share a row.  The best cell
+// of every row alive in the band sits in the warp's shared memory until the
+// warp's lowest lane has met the row; a column is complete in one step.
+// Finished rows and columns go to global memory as 64-bit max reductions into
+// one of several key shards.  One resident wave of warps takes the bands
+// from a list (fp64_band_of).
 //
 // Selection thresholds: every merge also raises a per-entry threshold to a
 // value just below the merged score (fp64_threshold_below: the margin is wider
-// than the index key's resolution).  A lane's row partials start at their
-// rows' thresholds, and in the branch-free chunks each column step first
-// evaluates its cells and compares them with their row partials and with the
-// column's threshold; only when some cell of the warp exceeds one does the
-// step run the (score, index) selection.  A cell that exceeds neither can
-// raise neither key of its row or column (its score is below a score already
-// merged there, by more than the index key resolves), so the result is the
-// same as selecting every cell.  Thresholds are read as they stand (a stale
-// one is only a lower bound), so the arithmetic and the keys -- and therefore
-// the output -- do not depend on timing.
+// than the index key's resolution).  A row's best cell starts at its row's
+// threshold with no source.  A cell that exceeds neither its row's best nor its
+// column's threshold can raise neither key of its row or column (its score is
+// below a score already merged there, by more than the index key resolves), so
+// the result is the same as selecting every cell.  Thresholds are read as they
+// stand (a stale one is only a lower bound), so the arithmetic and the keys --
+// and therefore the output -- do not depend on timing.
+//
+// Bands of one wave run side by side, and a row's first candidates come from
+// the band whose diagonals reach it first.  If the wave holds the longest bands
+// only, every row past its last band is new to all of them: the band next to
+// those rows selects in nearly every step, the ones behind catch up with it, and
+// soon the whole wave selects (n = 1,048,576: 16% of the steps had a cell above
+// its row's best).  So the first wave takes every spread-th band of the whole
+// list; the bands between them then meet rows whose bests are nearly final.
+//
+// Passes inside the 4-wide part test in integers, once per kU * R columns: a lane
+// takes the maximum of its scores' high words and compares it with the smallest
+// high word among the best scores of the rows and the thresholds of the columns
+// that it meets in the pass (fp64_gate; high words order like non-negative
+// doubles, and a negative bound opens the gate).  When some lane of the warp
+// passes, the pass is evaluated again with the selection.  That takes R/2 integer
+// maxima per column in place of 2R FP64 compares and two votes, and no branch
+// between the columns.
+//
+// What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 5
+// per cell (40 of a step's 62 instructions at R = 8); other instructions cost it
+// about 0.7 cycles each.  n = 1,048,576, m = 256: 262 ms, from 441 ms with the
+// selection tested per step in FP64 and the bands in order of length (spread
+// alone: 269 ms, with the gate per step).  3 CTAs of 4 warps per SM at 168
+// registers spill and run at 273 ms.
 #include <float.h>
+#include <limits.h>
 
 #include <algorithm>
 #include <atomic>
@@ -58,94 +76,12 @@ __device__ __forceinline__ double4 ring_rec(const char* p) {
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-// Which parts of a column step need the selection, voted over the warp: bit 0
-// when some lane has a cell above its row partial, bit 1 when some cell is
-// above the column's threshold.  Chains of predicated compares per lane
-// (setp ... .or; with R = 8 two chains of 4 per test, interleaved, so the
-// dependent compares are half as deep) and two votes; NaN compares false, so
-// NaN cells never select.
-template <int R>
-__device__ __forceinline__ unsigned step_hits(const double (&sc)[R], const double (&acc)[2 * R - 1],
-                                              int b, double tc) {
-    bool row = false, col = false;
-#pragma unroll
-    for (int a = 0; a < R; ++a) {
-        row |= sc[a] > acc[b + a];
-        col |= sc[a] > tc;
-    }
-    return (__any_sync(kFullMask, row) ? 1u : 0u) | (__any_sync(kFullMask, col) ? 2u : 0u);
-}
-template <>
-__device__ __forceinline__ unsigned step_hits<4>(const double (&sc)[4], const double (&acc)[7],
-                                                 int b, double tc) {
-    unsigned r;
-    asm volatile(
-        "{\n\t.reg .pred pr, pc, qr, qc;\n\t"
-        "setp.gt.f64 pr, %1, %5;\n\t"
-        "setp.gt.or.f64 pr, %2, %6, pr;\n\t"
-        "setp.gt.or.f64 pr, %3, %7, pr;\n\t"
-        "setp.gt.or.f64 pr, %4, %8, pr;\n\t"
-        "setp.gt.f64 pc, %1, %9;\n\t"
-        "setp.gt.or.f64 pc, %2, %9, pc;\n\t"
-        "setp.gt.or.f64 pc, %3, %9, pc;\n\t"
-        "setp.gt.or.f64 pc, %4, %9, pc;\n\t"
-        "vote.sync.any.pred qr, pr, 0xffffffff;\n\t"
-        "vote.sync.any.pred qc, pc, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, qr;\n\t"
-        "@qc or.b32 %0, %0, 2;\n\t"
-        "}"
-        : "=r"(r)
-        : "d"(sc[0]), "d"(sc[1]), "d"(sc[2]), "d"(sc[3]), "d"(acc[b]), "d"(acc[b + 1]),
-          "d"(acc[b + 2]), "d"(acc[b + 3]), "d"(tc));
-    return r;
-}
-template <>
-__device__ __forceinline__ unsigned step_hits<8>(const double (&sc)[8], const double (&acc)[15],
-                                                 int b, double tc) {
-    unsigned r;
-    asm volatile(
-        "{\n\t.reg .pred pr, pc, pr2, pc2, qr, qc;\n\t"
-        "setp.gt.f64 pr, %1, %9;\n\t"
-        "setp.gt.f64 pr2, %5, %13;\n\t"
-        "setp.gt.f64 pc, %1, %17;\n\t"
-        "setp.gt.f64 pc2, %5, %17;\n\t"
-        "setp.gt.or.f64 pr, %2, %10, pr;\n\t"
-        "setp.gt.or.f64 pr2, %6, %14, pr2;\n\t"
-        "setp.gt.or.f64 pc, %2, %17, pc;\n\t"
-        "setp.gt.or.f64 pc2, %6, %17, pc2;\n\t"
-        "setp.gt.or.f64 pr, %3, %11, pr;\n\t"
-        "setp.gt.or.f64 pr2, %7, %15, pr2;\n\t"
-        "setp.gt.or.f64 pc, %3, %17, pc;\n\t"
-        "setp.gt.or.f64 pc2, %7, %17, pc2;\n\t"
-        "setp.gt.or.f64 pr, %4, %12, pr;\n\t"
-        "setp.gt.or.f64 pr2, %8, %16, pr2;\n\t"
-        "setp.gt.or.f64 pc, %4, %17, pc;\n\t"
-        "setp.gt.or.f64 pc2, %8, %17, pc2;\n\t"
-        "or.pred pr, pr, pr2;\n\t"
-        "or.pred pc, pc, pc2;\n\t"
-        "vote.sync.any.pred qr, pr, 0xffffffff;\n\t"
-        "vote.sync.any.pred qc, pc, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, qr;\n\t"
-        "@qc or.b32 %0, %0, 2;\n\t"
-        "}"
-        : "=r"(r)
-        : "d"(sc[0]), "d"(sc[1]), "d"(sc[2]), "d"(sc[3]), "d"(sc[4]), "d"(sc[5]), "d"(sc[6]),
-          "d"(sc[7]), "d"(acc[b]), "d"(acc[b + 1]), "d"(acc[b + 2]), "d"(acc[b + 3]),
-          "d"(acc[b + 4]), "d"(acc[b + 5]), "d"(acc[b + 6]), "d"(acc[b + 7]), "d"(tc));
-    return r;
-}
-
-// Asynchronous copies global -> shared (both addresses aligned to the size):
-// 16 bytes through L2 only, 8 bytes through L1.
+// Asynchronous 16-byte copy global -> shared through L2 only (both addresses
+// 16-byte aligned).
 __device__ __forceinline__ void cp_async16(char* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-
 // A threshold as it stands (other warps raise it with atomics meanwhile; any
 // value it has held is a valid lower bound).
 __device__ __forceinline__ double ld_thr(const double* p) {
@@ -166,54 +102,67 @@ __device__ __forceinline__ void flush_fp64(const Fp64BandParams& P, int shard, i
     if (t >= 0.0) atomicMax(reinterpret_cast<long long*>(P.thr + slot), __double_as_longlong(t));
 }
 
-// Per-warp ring of row thresholds in shared memory, indexed like the record
-// ring (row t of the band at slot t % kRecRing), one double of padding after
-// every 8 so that lanes reading rows 8 apart hit distinct banks.  Slots
-// kRecRing .. kRecRing + kThrMirror - 1 mirror slots 0 .. kThrMirror - 1, so
-// the 16 consecutive rows a lane starts in one chunk never wrap: with R = 8
-// their offsets are one base plus compile-time constants.
-constexpr int kThrMirror = 16;
-constexpr int kThrRingDoubles = (kRecRing + kThrMirror) + (kRecRing + kThrMirror) / 8;
-__device__ __forceinline__ int thr_pos(int s) { return s + (s >> 3); }
-__device__ __forceinline__ int thr_off(int t) { return thr_pos(t % kRecRing); }
-__device__ __forceinline__ void thr_store(double* tring, int t, double v) {
-    const int s = t % kRecRing;
-    tring[thr_pos(s)] = v;
-    if (s < kThrMirror) tring[thr_pos(s + kRecRing)] = v;
+// A bound's high word for the integer gate: scores at or above a non-negative
+// bound have a high word at or above its high word (as signed integers); a
+// negative bound lets every cell through.
+__device__ __forceinline__ int fp64_gate(double bound) {
+    const int h = __double2hiint(bound);
+    return h < 0 ? INT_MIN : h;
 }
 
-// The (score, index) selection of one column step: row partials (strict '>',
-// the reference's rule; a partial started at its row's threshold has no
-// source (RowSrc) until a cell beats it), then the column's best cell over
-// the warp from two REDUX instructions (high, then low word of the ordered
-// score); the lowest winning lane parks (score, row) in the warp's column slot
-// with a predicated store, so no divergent branch splits consecutive steps.
-// Where a lane's 2R - 1 row partials came from: the diagonal offset a < R of
-// the selected cell, as nibble k = a + 1, or 0 while partial k is still its
-// row's threshold (no candidate yet).  One 64-bit register pair instead of
-// 2R - 1 registers.
-struct RowSrc {
-    unsigned long long w;
-    __device__ __forceinline__ int get(int k) const { return (int)((w >> (4 * k)) & 15ull) - 1; }
-    __device__ __forceinline__ void set(int k, int a) {
-        w = (w & ~(15ull << (4 * k))) | ((unsigned long long)(a + 1) << (4 * k));
+// One warp's shared memory.  Rows of the band go in groups of R (row t of the
+// tile, counted from its first column's row on the band's first diagonal, is
+// element t % R of group t / R); kGroups slots of R rows form a ring, in which
+// chunk c reads groups c .. c + 32; a pass of kU chunks copies in the next kU
+// groups meanwhile.  Every
+// array is padded by one element per group, so that lanes reading the same
+// element of consecutive groups hit distinct banks (a multiple of 8 groups, so
+// that a wrap keeps that for the 16-byte halves of the records).
+constexpr int kGroups = 40;
+constexpr int kU = 2;  // chunks per pass
+static_assert(kGroups % kU == 0 && kGroups >= 32 + 2 * kU, "a pass's incoming groups fit the ring");
+__device__ __forceinline__ int wrap_group(int s) { return s < kGroups ? s : s - kGroups; }
+template <int R>
+struct BandSmem {
+    static constexpr int kRecStride = 32 * R + 16;  // bytes of a group's records
+    static constexpr int kUsed = kGroups * kRecStride + 2 * 32 * R * kU +
+                                 kGroups * (R + 1) * (int)(sizeof(double) + sizeof(int)) +
+                                 2 * R * kU * (int)sizeof(double) + kGroups * (int)sizeof(int);
+    static constexpr int kBytes = (kUsed + 15) / 16 * 16;  // warps' areas stay aligned
+    char* rec;     // row records
+    char* col;     // column records, two buffers of kU * R
+    double* best;  // best score of each row (its threshold while src < 0)
+    double* cthr;  // column thresholds, two buffers of kU * R
+    int* src;      // its column, -1: none yet
+    int* gate;     // per group: smallest gate among the rows' best scores
+    __device__ __forceinline__ BandSmem(char* p) {
+        rec = p;
+        p += kGroups * kRecStride;
+        col = p;
+        p += 2 * 32 * R * kU;
+        best = reinterpret_cast<double*>(p);
+        p += kGroups * (R + 1) * sizeof(double);
+        cthr = reinterpret_cast<double*>(p);
+        p += 2 * R * kU * sizeof(double);
+        src = reinterpret_cast<int*>(p);
+        p += kGroups * (R + 1) * sizeof(int);
+        gate = reinterpret_cast<int*>(p);
+    }
+    // smallest gate among the R rows of the group in slot s
+    __device__ __forceinline__ int group_gate(int s) const {
+        int g = INT_MAX;
+#pragma unroll
+        for (int k = 0; k < R; ++k) g = min(g, fp64_gate(best[s * (R + 1) + k]));
+        return g;
     }
 };
+
+// The column's best cell over the warp, from two REDUX instructions (high, then
+// low word of the ordered score; ties go to the smallest diagonal); the winning
+// lane merges it.
 template <int R>
-__device__ __forceinline__ void select_rows(int b, const double (&sc)[R], double (&acc_s)[2 * R - 1],
-                                            RowSrc& acc_a) {
-    static_assert(2 * R - 1 <= 16, "2R - 1 nibbles fit 64 bits");
-#pragma unroll
-    for (int a = 0; a < R; ++a) {
-        if (sc[a] > acc_s[b + a]) {
-            acc_s[b + a] = sc[a];
-            acc_a.set(b + a, a);
-        }
-    }
-}
-template <int R>
-__device__ __forceinline__ void select_column(const Fp64BandParams& P, int b, const double (&sc)[R],
-                                              int64_t g0, int lane, double* cslot_s, int* cslot_r) {
+__device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard, unsigned j,
+                                              const double (&sc)[R], int64_t g0, int lane) {
     // lane's best cell of the column: pairwise tree, left wins ties.  A NaN
     // cell (a constant window) never selects under the reference's '>'; as
     // -DBL_MAX it also cannot hide the cell it is paired with in the tree.
@@ -239,266 +188,268 @@ __device__ __forceinline__ void select_column(const Fp64BandParams& P, int b, co
     const unsigned mlo = __reduce_max_sync(kFullMask, hi == mhi ? lo : 0u);
     const bool top = (hi == mhi) && (lo == mlo) && (mhi != 0u);
     const unsigned tops = __ballot_sync(kFullMask, top);
-    if (top && (tops & ((1u << lane) - 1u)) == 0u) {
-        cslot_s[b] = cbest;
-        cslot_r[b] = (int)(b + g0 + ca[0]);  // row - jc (rows < 2^31)
-    }
-}
-template <int R>
-__device__ __forceinline__ void select_step(const Fp64BandParams& P, int b, const double (&sc)[R],
-                                            double (&acc_s)[2 * R - 1], RowSrc& acc_a,
-                                            int64_t g0, int lane, double* cslot_s, int* cslot_r) {
-    select_rows<R>(b, sc, acc_s, acc_a);
-    select_column<R>(P, b, sc, g0, lane, cslot_s, cslot_r);
+    if (top && (tops & ((1u << lane) - 1u)) == 0u)
+        flush_fp64(P, shard, j + P.col_key_off, cbest, j + g0 + ca[0] + P.row_nb_off);
 }
 
-// One chunk = R consecutive columns.  FAST chunks hold only cells of the
-// reference's 4-wide (fused) part; each step there evaluates its R cells per
-// lane, and the selection runs only when some cell of the warp exceeds its row
-// partial or the column's threshold cthr[b] (a warp vote).  Other chunks
-// evaluate every cell with its own geometry and always select.  Returns
-// whether any step selected (uniform over the warp).
-template <int R, bool FAST>
-__device__ __forceinline__ bool chunk_fp64(const Fp64BandParams& P, int64_t jc, const char* rring,
-                                           const char* rbase, int tbase, double4 (&rwin)[R], double (&qt)[R],
-                                           const int* lgeo,
-                                           double (&acc_s)[2 * R - 1], RowSrc& acc_a,
-                                           int64_t g0, int lane, double* cslot_s, int* cslot_r,
-                                           const double* cthr, const char* ccur) {
-    bool selected = !FAST;
+// Selection of one column step: every cell above its row's best replaces it
+// (strict '>', the reference's rule; a step's cells lie in distinct rows), and
+// a column with a cell above its threshold tc is reduced over the warp.  Cell a
+// of column b is element b + a of the lane's two groups, in slots s0 and s1.
+template <int R>
+__device__ __forceinline__ void select_step(const Fp64BandParams& P, int shard, int b, unsigned j,
+                                            const double (&sc)[R], const BandSmem<R>& sm, int s0,
+                                            int s1, double tc, int64_t gb, int lane) {
+    __syncwarp();  // rows move from lane to lane between steps
+    bool col = false;
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+        const int e = b + a < R ? s0 * (R + 1) + b + a : s1 * (R + 1) + b + a - R;
+        if (sc[a] > sm.best[e]) {
+            sm.best[e] = sc[a];
+            sm.src[e] = (int)j;
+        }
+        col |= sc[a] > tc;
+    }
+    if (__any_sync(kFullMask, col)) select_column<R>(P, shard, j, sc, gb + lane * R, lane);
+}
+
+// One chunk = R consecutive columns, in one of three ways:
+//   kGate    only cells of the reference's 4-wide (fused) part, no selection:
+//            returns the largest high word of the lane's scores
+//   kSelect  the same cells again with the selection, for a chunk whose gate
+//            opened: per step behind the gate
+//   kEdge    any cells, each with its own geometry; every step selects
+// On entry rwin holds the records of the lane's first group, on return those of
+// its second.
+// (sel: set when a step selected).
+enum ChunkWay { kGate, kSelect, kEdge };
+template <int R, ChunkWay WAY>
+__device__ __forceinline__ int chunk_fp64(const Fp64BandParams& P, int shard, unsigned jc,
+                                          const BandSmem<R>& sm, int s0, int s1,
+                                          const char* col, const double* cthr,
+                                          double4 (&rwin)[R], double (&qt)[R], int gate,
+                                          unsigned geo, int64_t gb, int lane, bool& sel) {
+    const int len0 = (int)(P.Tbase - gb) - lane * R;  // columns of the lane's first diagonal
+    int top = INT_MIN;
+    const char* rec1 = sm.rec + s1 * BandSmem<R>::kRecStride;
+    double4 cv = ring_rec(col);
 #pragma unroll
     for (int b = 0; b < R; ++b) {
-        const int64_t j = jc + b;
-        // record tbase + b + R - 1 (tbase = jc + lane*R): with R = 8 the slot of
-        // record tbase + R - 1 is 7 mod 8 and the step offsets are constants
-        if (R == 8)
-            rwin[(b + R - 1) % R] = ring_rec(rbase + rec_step<7>(b));
-        else
-            rwin[(b + R - 1) % R] =
-                ring_rec(rring + rec_off(rec_slot(tbase + b + R - 1)));
-        const double4 cv = ring_rec(ccur + 32 * b);  // column record, staged a chunk ahead
+        const unsigned j = jc + b;
+        double4 cn = cv;
+        if (b + 1 < R) cn = ring_rec(col + 32 * (b + 1));
         double sc[R];
-        if (FAST) {
-            const double tc = cthr[b];
 #pragma unroll
-            for (int a = 0; a < R; ++a) {
-                const double4 rv = rwin[(b + a) % R];
-                // 4-wide part of the reference kernel (kernels.cpp:206-225)
+        for (int a = 0; a < R; ++a) {
+            const double4 rv = rwin[(b + a) % R];
+            // the window moves on: element b + R replaces element b
+            if (a == 0) rwin[b] = ring_rec(rec1 + 32 * b);
+            double score = -DBL_MAX;
+            const unsigned code = (geo >> (4 * a)) & 15u;
+            if (WAY != kEdge || (code != 15u && (int64_t)j < len0 - a)) {
                 const double ss = __dmul_rn(rv.z, cv.z);
-                const double mm = __dmul_rn(cv.w, rv.w);
-                sc[a] = __fma_rn(qt[a], ss, -mm);
-                qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
-            }
-            const unsigned hits = step_hits<R>(sc, acc_s, b, tc);
-            if (hits) {
-                selected = true;
-                if (hits & 1u) select_rows<R>(b, sc, acc_s, acc_a);
-                if (hits & 2u) select_column<R>(P, b, sc, g0, lane, cslot_s, cslot_r);
-            }
-        } else {
-#pragma unroll
-            for (int a = 0; a < R; ++a) {
-                const double4 rv = rwin[(b + a) % R];
-                double score;
-                if (j < lgeo[a * 32]) {
-                    const double ss = __dmul_rn(rv.z, cv.z);
-                    if (j <= lgeo[(R + a) * 32]) {
-                        const double mm = __dmul_rn(cv.w, rv.w);
-                        score = __fma_rn(qt[a], ss, -mm);
-                        qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
-                    } else {
-                        // scalar remainder (kernels.cpp:282-289), no fusion
-                        score = __dsub_rn(__dmul_rn(qt[a], ss), __dmul_rn(rv.w, cv.w));
-                        qt[a] = __dsub_rn(__dadd_rn(qt[a], __dmul_rn(rv.y, cv.y)),
-                                          __dmul_rn(rv.x, cv.x));
-                    }
+                if (WAY != kEdge || (code != 7u && (int64_t)j <= len0 - a - 4 + (int)code)) {
+                    // 4-wide part of the reference kernel (kernels.cpp:206-225)
+                    const double mm = __dmul_rn(cv.w, rv.w);
+                    score = __fma_rn(qt[a], ss, -mm);
+                    qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
                 } else {
-                    score = -DBL_MAX;
+                    // scalar remainder (kernels.cpp:282-289), no fusion
+                    score = __dsub_rn(__dmul_rn(qt[a], ss), __dmul_rn(rv.w, cv.w));
+                    qt[a] = __dsub_rn(__dadd_rn(qt[a], __dmul_rn(rv.y, cv.y)),
+                                      __dmul_rn(rv.x, cv.x));
                 }
-                sc[a] = score;
             }
-            select_step<R>(P, b, sc, acc_s, acc_a, g0, lane, cslot_s, cslot_r);
+            sc[a] = score;
+        }
+        cv = cn;
+        if (WAY != kEdge) {
+            if (WAY == kSelect) top = INT_MIN;
+            if (R == 1) top = max(top, __double2hiint(sc[0]));
+#pragma unroll
+            for (int a = 0; a + 1 < R; a += 2)
+                top = __vimax3_s32(top, __double2hiint(sc[a]), __double2hiint(sc[a + 1]));
+        }
+        if (WAY == kEdge || (WAY == kSelect && __any_sync(kFullMask, top >= gate))) {
+            select_step<R>(P, shard, b, j, sc, sm, s0, s1, cthr[b], gb, lane);
+            sel = true;
         }
     }
-    return selected;
+    return top;
 }
 
 template <int R>
 __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band, int lane,
-                                          int shard, double* ring_s, int* ring_c, char* rring,
-                                          double* cslot_s, int* cslot_r, double* tring,
-                                          double* cthr, char* ccol, int* lgeo) {
-    constexpr int RING = 32 * R;
-    const int64_t gb = P.g_lo + band * (int64_t)RING;
+                                          int shard, const BandSmem<R>& sm) {
+    constexpr int RS = BandSmem<R>::kRecStride;
+    const int64_t gb = P.g_lo + band * (int64_t)(32 * R);
     const int64_t g0 = gb + (int64_t)lane * R;
-    const int64_t jmax = P.Tbase - gb;  // length of the band's longest diagonal
+    const int jmax = (int)(P.Tbase - gb);  // length of the band's longest diagonal
     if (jmax <= 0) return;
 
-    // Per diagonal a of the lane: len = its column count, psw = its last
-    // column of the reference's 4-wide part (-1: none), kept in the lane's
-    // slots of shared memory (lgeo[a*32], lgeo[(R+a)*32]; columns < 2^31,
-    // checked by the host): only the chunks near a diagonal's end read them.
+    // Diagonal g has len = Tbase - g columns; with delta its offset in its block,
+    // its last column of the reference's 4-wide part is len - 4 + delta % 4, or
+    // none when delta >= B & ~3.  geo holds delta % 4 (or 7) of the lane's
+    // diagonals, 15 for one past g_hi, as nibbles: only the chunks near a
+    // diagonal's end read them.  A diagonal past g_hi carries -inf, which stays
+    // below every bound, so it does not cost the band its branch-free chunks.
     double qt[R];
-    int minpsw = INT32_MAX;
+    unsigned geo = 0;
+    int minpsw = INT_MAX;
 #pragma unroll
     for (int a = 0; a < R; ++a) {
         const int64_t g = g0 + a;
-        int len = 0, psw = -1;
+        unsigned code = 15;
+        qt[a] = -__longlong_as_double(0x7ff0000000000000ll);
         if (g < P.g_hi) {
             const int64_t delta = (g - P.blk_origin) % P.B;
-            const int64_t T = P.Tbase - (g - delta);
             qt[a] = P.qt0[g - P.g_lo];
-            len = (int)(T - delta);
-            psw = (delta < (P.B & ~3ll)) ? (int)(T - 4 * (delta / 4 + 1)) : -1;
-        } else {
-            qt[a] = 0.0;
+            code = delta < (P.B & ~3ll) ? (unsigned)(delta & 3) : 7u;
+            minpsw = min(minpsw, code == 7u ? -1 : (int)(P.Tbase - g) - 4 + (int)code);
         }
-        lgeo[a * 32] = len;
-        lgeo[(R + a) * 32] = psw;
-        minpsw = min(minpsw, psw);
+        geo |= code << (4 * a);
     }
+    minpsw = __reduce_min_sync(kFullMask, minpsw);
 
-    // ring of row partials, slot = (r - gb) mod RING; column slots of a chunk
-    for (int k = lane; k < RING; k += 32) {
-        ring_s[k] = -DBL_MAX;
-        ring_c[k] = 0;
-    }
-    if (lane < R) cslot_s[lane] = -DBL_MAX;
-
-    // row records of the band (t = row - gb) and their rows' thresholds staged
-    // in the warp's shared-memory rings; before chunk jc they hold t < fill
+    // Groups 0 .. 32 + kU - 1 and the first pass's columns.  In a pass of kU
+    // chunks, lanes 0 - 15 bring in the next rows' thresholds, lanes 16 - 31 the
+    // next columns': part = lane % 16.
+    const int part = lane & 15;
+    const bool isrow = lane < 16;
     const uint4* rsrc = reinterpret_cast<const uint4*>(P.rowrec + gb);
-    const double* tsrc = P.thr + gb + P.row_key_off;  // threshold of band row t
+    const uint4* crec = reinterpret_cast<const uint4*>(P.colrec);
+    const double* tsrc = P.thr + gb + P.row_key_off;  // threshold of row t
     const double* csrc = P.thr + P.col_key_off;       // threshold of column j
-    int fill = 34 * R;
-    for (int i = lane; i < 2 * fill; i += 32) rec_store(rring, i >> 1, i & 1, __ldg(rsrc + i));
-    for (int i = lane; i < fill; i += 32) thr_store(tring, i, ld_thr(tsrc + i));
-    if (lane < R) cthr[lane] = ld_thr(csrc + lane);
-    // column records of a chunk in shared memory, double-buffered: R records of
-    // 32 bytes per buffer, the next chunk's loaded while this one runs
-    const uint4* csrc_rec = reinterpret_cast<const uint4*>(P.colrec);
-    if (lane < 2 * R) *reinterpret_cast<uint4*>(ccol + 16 * lane) = __ldg(csrc_rec + lane);
-    int cbuf = 0;
+    for (int i = lane; i < (32 + kU) * 2 * R; i += 32)
+        *reinterpret_cast<uint4*>(sm.rec + (i / (2 * R)) * RS + 16 * (i % (2 * R))) =
+            __ldg(rsrc + i);
+    for (int i = lane; i < (32 + kU) * R; i += 32) {
+        sm.best[(i / R) * (R + 1) + i % R] = ld_thr(tsrc + i);
+        sm.src[(i / R) * (R + 1) + i % R] = -1;
+    }
+    if (lane < 2 * R * kU) *reinterpret_cast<uint4*>(sm.col + 16 * lane) = __ldg(crec + lane);
+    int cgate = INT_MAX;
+    if (lane < R * kU) {
+        const double t = ld_thr(csrc + lane);
+        sm.cthr[lane] = t;
+        cgate = fp64_gate(t);
+    }
+    cgate = __reduce_min_sync(kFullMask, cgate);
     __syncwarp();
-    // register window of row records: slot (k mod R) holds row g0 + jc + k
+    sm.gate[lane] = sm.group_gate(lane);
+    if (lane < kU) sm.gate[32 + lane] = sm.group_gate(32 + lane);
+    __syncwarp();
+    // register window of row records: slot (k mod R) holds element k of the
+    // lane's first group
     double4 rwin[R];
 #pragma unroll
-    for (int k = 0; k < R - 1; ++k) rwin[k] = ring_rec(rring + rec_off(rec_slot(lane * R + k)));
-    // row partials: slot k holds row g0 + jc + k, starting at the row's
-    // threshold with no source (no candidate yet)
-    double acc_s[2 * R - 1];
-    RowSrc acc_a{0ull};
-#pragma unroll
-    for (int k = 0; k < 2 * R - 1; ++k) {
-        acc_s[k] = tring[thr_off(lane * R + k)];
-    }
+    for (int k = 0; k < R; ++k) rwin[k] = ring_rec(sm.rec + lane * RS + 32 * k);
 
-    bool sel_prev = false;
-    for (int64_t jc = 0; jc < jmax; jc += R) {
-        // Prefetch what the next chunk appends -- R row records and their
-        // rows' thresholds into ring slots this chunk does not read (it reads
-        // rows below fill - 1), R column records and column thresholds into
-        // the other buffers -- copied straight into shared memory while the
-        // chunk runs.  A threshold copied through L1 may be older than the
-        // value in L2; any value it has held is a valid lower bound.
-        if (lane < 2 * R) {
-            const int sr = rec_slot(fill + (lane >> 1));
-            const uint4* src = rsrc + 2 * fill + lane;
-            cp_async16(rring + rec_off(sr) + 16 * (lane & 1), src);
-            if (sr < kRecMirror) cp_async16(rring + rec_off(sr + kRecRing) + 16 * (lane & 1), src);
-            cp_async16(ccol + (cbuf ^ 1) * (32 * R) + 16 * lane, csrc_rec + 2 * (jc + R) + lane);
+    // what the lane copies in next: records of groups c + 32 + kU .. and of the
+    // next pass's columns, and their thresholds
+    const uint4* nrow = rsrc + (32 + kU) * 2 * R + lane;
+    const uint4* ncol = crec + kU * 2 * R + lane;
+    const double* nthr = isrow ? tsrc + (32 + kU) * R + part : csrc + kU * R + part;
+    int s0 = lane;  // slot of the lane's first group
+    int sf = 0;     // slot of group c, the first that the pass finishes
+    int cbuf = 0;
+    bool sel = false;
+    for (unsigned jc = 0; jc < (unsigned)jmax; jc += kU * R) {
+        const int sn = wrap_group(sf + 32 + kU);  // slots of the incoming groups (kU divides kGroups)
+        double t = 0.0;
+        if (lane < 2 * R * kU) {
+            cp_async16(sm.rec + (sn + lane / (2 * R)) * RS + 16 * (lane % (2 * R)), nrow);
+            cp_async16(sm.col + (cbuf ^ 1) * (32 * R * kU) + 16 * lane, ncol);
         }
-        if (lane < R) {
-            const int st = (fill + lane) % kRecRing;
-            cp_async8(tring + thr_pos(st), tsrc + fill + lane);
-            if (st < kThrMirror) cp_async8(tring + thr_pos(st + kRecRing), tsrc + fill + lane);
-            cp_async8(cthr + (cbuf ^ 1) * R + lane, csrc + jc + R + lane);
-        }
+        if (part < R * kU) t = ld_thr(nthr);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-        const char* ccur = ccol + cbuf * (32 * R);
-        const int tbase = (int)jc + lane * R;
-        const char* rbase = rring + rec_off(rec_slot(tbase + R - 1));
-        const bool fast = __all_sync(kFullMask, jc + R - 1 <= minpsw);
-        bool sel;
-        if (fast)
-            sel = chunk_fp64<R, true>(P, jc, rring, rbase, tbase, rwin, qt, lgeo, acc_s, acc_a,
-                                      g0, lane, cslot_s, cslot_r, cthr + cbuf * R, ccur);
-        else
-            sel = chunk_fp64<R, false>(P, jc, rring, rbase, tbase, rwin, qt, lgeo, acc_s, acc_a,
-                                       g0, lane, cslot_s, cslot_r, cthr + cbuf * R, ccur);
-        __syncwarp();
-        // the chunk's column maxima (one per column, parked by the winning lane)
-        if (sel && lane < R) {
-            const double cs = cslot_s[lane];
-            if (cs > P.floor)
-                flush_fp64(P, shard, jc + lane + P.col_key_off, cs,
-                           jc + cslot_r[lane] + P.row_nb_off);
-            cslot_s[lane] = -DBL_MAX;
-        }
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        cbuf ^= 1;
-        fill += R;
-        // rows jc + g0 + [0, R) are done for this lane: merge its candidates
-        // (selected in this chunk or the previous one) into the ring
-        if (sel || sel_prev) {
-            const int base = (int)(((jc / R) + lane) % 32) * R;
+        nrow += kU * 2 * R;
+        ncol += kU * 2 * R;
+        nthr += kU * R;
+        int gate = cgate;
 #pragma unroll
-            for (int k = 0; k < R; ++k) {
-                const int a = acc_a.get(k);
-                if (a >= 0 && acc_s[k] > ring_s[base + k]) {
-                    ring_s[base + k] = acc_s[k];
-                    ring_c[base + k] = (int)(jc + k - a);
+        for (int u = 0; u <= kU; ++u) gate = min(gate, sm.gate[wrap_group(s0 + u)]);
+        const char* col = sm.col + cbuf * (32 * R * kU);
+        const double* cthr = sm.cthr + cbuf * (R * kU);
+        if ((int64_t)jc + (kU * R - 1) <= minpsw) {
+            bool open = sel;  // a pass after one that selected goes straight to selecting
+            if (!open) {
+                double q0[R];
+#pragma unroll
+                for (int a = 0; a < R; ++a) q0[a] = qt[a];
+                int top = INT_MIN;
+#pragma unroll 1
+                for (int u = 0; u < kU; ++u)
+                    top = max(top, chunk_fp64<R, kGate>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
+                                                        col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, open));
+                open = __any_sync(kFullMask, top >= gate);
+                if (open) {
+#pragma unroll
+                    for (int a = 0; a < R; ++a) {
+                        qt[a] = q0[a];
+                        rwin[a] = ring_rec(sm.rec + s0 * RS + 32 * a);
+                    }
                 }
             }
-        }
-        sel_prev = sel;
-        __syncwarp();
-        // rows jc + gb + [0, R) have now met every lane: flush and free
-        if (lane < R) {
-            const int e = (int)((jc / R) % 32) * R + lane;
-            const double s = ring_s[e];
-            if (s > P.floor) flush_fp64(P, shard, jc + gb + lane + P.row_key_off, s,
-                                     ring_c[e] + P.col_nb_off);
-            ring_s[e] = -DBL_MAX;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int k = 0; k < R - 1; ++k) acc_s[k] = acc_s[k + R];
-        acc_a.w >>= 4 * R;  // and the new rows' nibbles are 0
-        // new rows jc + R + g0 + k start at their thresholds
-        if (R == 8) {
-            // rows tbase + 8 + k: slot s0 + k with s0 = (tbase + 8) % kRecRing a
-            // multiple of 8 and k < 16 (the mirror keeps them from wrapping)
-            const double* tb = tring + thr_pos((tbase + 8) % kRecRing);
-#pragma unroll
-            for (int k = R - 1; k < 2 * R - 1; ++k) {
-                acc_s[k] = tb[k + (k >> 3)];
+            sel = false;
+            if (open) {
+#pragma unroll 1
+                for (int u = 0; u < kU; ++u)
+                    chunk_fp64<R, kSelect>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
+                                           col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, sel);
             }
         } else {
-#pragma unroll
-            for (int k = R - 1; k < 2 * R - 1; ++k) {
-                acc_s[k] = tring[thr_off(tbase + R + k)];
+            sel = true;
+#pragma unroll 1
+            for (int u = 0; u < kU; ++u)
+                chunk_fp64<R, kEdge>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
+                                     col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, sel);
+        }
+        __syncwarp();
+        // groups c .. c + kU - 1 have met every lane: merge their rows
+        if (lane < R * kU) {
+            const int e = (sf + lane / R) * (R + 1) + lane % R;
+            const int j = sm.src[e];
+            if (j >= 0) {
+                const double s = sm.best[e];
+                if (s > P.floor) flush_fp64(P, shard, jc + gb + lane + P.row_key_off, s, j + P.col_nb_off);
             }
         }
+        // the incoming groups and columns begin at their thresholds
+        if (part < R * kU) {
+            if (isrow) {
+                const int e = (sn + part / R) * (R + 1) + part % R;
+                sm.best[e] = t;
+                sm.src[e] = -1;
+            } else {
+                sm.cthr[(cbuf ^ 1) * (R * kU) + part] = t;
+            }
+        }
+        const int x = part < R * kU ? fp64_gate(t) : INT_MAX;
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int g = __reduce_min_sync(kFullMask, isrow && part / R == u ? x : INT_MAX);
+            if (lane == 0) sm.gate[sn + u] = g;
+        }
+        cgate = __reduce_min_sync(kFullMask, isrow ? INT_MAX : x);
+        s0 = wrap_group(s0 + kU);
+        if (sel) sm.gate[s0] = sm.group_gate(s0);  // best scores of groups c + kU .. c + kU + 31 rose
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncwarp();
+        sf = wrap_group(sf + kU);
+        cbuf ^= 1;
     }
 
-    // drain: carried rows jend + g0 + [0, R-1) into the ring, then every slot
-    const int64_t jend = ((jmax + R - 1) / R) * R;
-    const int base = (int)(((jend / R) + lane) % 32) * R;
-#pragma unroll
-    for (int k = 0; k < R - 1; ++k) {
-        const int a = acc_a.get(k);
-        if (a >= 0 && acc_s[k] > ring_s[base + k]) {
-            ring_s[base + k] = acc_s[k];
-            ring_c[base + k] = (int)(jend + k - a);
-        }
-    }
-    __syncwarp();
-    for (int e = lane; e < RING; e += 32) {
-        const double s = ring_s[e];
-        if (s > P.floor) {
-            const int64_t rel = ((int64_t)e - jend % RING + RING) % RING;
-            flush_fp64(P, shard, jend + gb + rel + P.row_key_off, s, ring_c[e] + P.col_nb_off);
+    // drain: rows of groups c .. c + 31 (the last chunk's second groups)
+    const int64_t tend = ((int64_t)jmax + kU * R - 1) / (kU * R) * (kU * R);  // row t of group c
+    for (int i = lane; i < 32 * R; i += 32) {
+        const int s = wrap_group(sf + i / R);
+        const int e = s * (R + 1) + i % R;
+        const int j = sm.src[e];
+        if (j >= 0) {
+            const double v = sm.best[e];
+            if (v > P.floor) flush_fp64(P, shard, tend + gb + i + P.row_key_off, v, j + P.col_nb_off);
         }
     }
     __syncwarp();
@@ -512,54 +463,33 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
 
 template <int R>
 constexpr int fp64_smem_bytes() {
-    return kFp64WarpsPerBlock *
-           (kRecRingBytes + 2 * 32 * R + (32 * R + R) * (int)(sizeof(double) + sizeof(int)) +
-            (kThrRingDoubles + 2 * R) * (int)sizeof(double) + 2 * R * 32 * (int)sizeof(int));
+    return kFp64WarpsPerBlock * BandSmem<R>::kBytes;
 }
 
 template <int R>
-__global__ void __launch_bounds__(32 * kFp64WarpsPerBlock) fp64_band_kernel(const Fp64BandParams P) {
+__global__ void __launch_bounds__(32 * kFp64WarpsPerBlock, R == 8 ? 2 : 4)
+    fp64_band_kernel(const Fp64BandParams P) {
     extern __shared__ __align__(128) char smem_fp64[];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
-    constexpr int kW = kFp64WarpsPerBlock;
-    char* p = smem_fp64;
-    char* rring = p + w * kRecRingBytes;
-    p += kW * kRecRingBytes;
-    char* ccol = p + w * (2 * 32 * R);
-    p += kW * 2 * 32 * R;
-    double* tring = reinterpret_cast<double*>(p) + w * kThrRingDoubles;
-    p += kW * kThrRingDoubles * sizeof(double);
-    double* ring_s = reinterpret_cast<double*>(p) + w * 32 * R;
-    p += kW * 32 * R * sizeof(double);
-    double* cslot_s = reinterpret_cast<double*>(p) + w * R;
-    p += kW * R * sizeof(double);
-    double* cthr = reinterpret_cast<double*>(p) + w * 2 * R;  // two buffers of R
-    p += kW * 2 * R * sizeof(double);
-    int* ring_c = reinterpret_cast<int*>(p) + w * 32 * R;
-    p += kW * 32 * R * sizeof(int);
-    int* cslot_r = reinterpret_cast<int*>(p) + w * R;
-    p += kW * R * sizeof(int);
-    int* lgeo = reinterpret_cast<int*>(p) + w * 2 * R * 32 + lane;
-    // One resident wave of W warps.  Band b (longest first: band lengths fall
-    // with b) goes to warp b mod W in even rounds and W-1 - (b mod W) in odd
-    // rounds, so every warp's bands add up to nearly the same length -- the
-    // reference's (k, nbands-1-k) pairing carried over any number of rounds.
-    const int64_t W = (int64_t)gridDim.x * kFp64WarpsPerBlock;
+    const BandSmem<R> sm(smem_fp64 + w * BandSmem<R>::kBytes);
+    // One resident wave of W warps takes the bands by rank (fp64_band_of): warp
+    // w starts with rank w, later ranks come from one counter (no waiting on
+    // anything).
     const int64_t wid = (int64_t)blockIdx.x * kFp64WarpsPerBlock + w;
     const int shard = (int)(wid % P.shards);
-    for (int64_t r = 0;; ++r) {
-        const int64_t band = r * W + ((r & 1) ? W - 1 - wid : wid);
-        if (band >= P.nbands) break;
-        band_fp64<R>(P, band, lane, shard, ring_s, ring_c, rring, cslot_s, cslot_r, tring, cthr,
-                     ccol, lgeo);
+    for (int64_t rank = wid; rank < P.nbands;) {
+        band_fp64<R>(P, fp64_band_of(rank, P.nbands, P.spread), lane, shard, sm);
+        unsigned next = 0;
+        if (lane == 0) next = atomicAdd(P.counter, 1u);
+        rank = (int64_t)gridDim.x * kFp64WarpsPerBlock + __shfl_sync(kFullMask, next, 0);
     }
 }
 
 }  // namespace
 
 template <int R>
-void launch_fp64_band(const Fp64BandParams& P, cudaStream_t s) {
+void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
     constexpr int smem = fp64_smem_bytes<R>();
     // per-device attribute and occupancy, idempotent: see launch_fp32_join
     static std::atomic<unsigned long long> configured{0};
@@ -581,9 +511,13 @@ void launch_fp64_band(const Fp64BandParams& P, cudaStream_t s) {
     }
     // one resident wave, fewer CTAs when there are fewer bands than warps
     const int64_t wave = (int64_t)sm_count() * resident[dev & 63].load(std::memory_order_relaxed);
-    const int64_t want = (P.nbands + kFp64WarpsPerBlock - 1) / kFp64WarpsPerBlock;
+    const int64_t want = (Q.nbands + kFp64WarpsPerBlock - 1) / kFp64WarpsPerBlock;
     const int64_t blocks = std::min<int64_t>(want, wave);
-    if (blocks > 0) fp64_band_kernel<R><<<(unsigned)blocks, 32 * kFp64WarpsPerBlock, smem, s>>>(P);
+    if (blocks <= 0) return;
+    Fp64BandParams P = Q;
+    P.spread = (P.nbands + blocks * kFp64WarpsPerBlock - 1) / (blocks * kFp64WarpsPerBlock);
+    cudaMemsetAsync(P.counter, 0, sizeof(unsigned), s);
+    fp64_band_kernel<R><<<(unsigned)blocks, 32 * kFp64WarpsPerBlock, smem, s>>>(P);
 }
 
 template void launch_fp64_band<1>(const Fp64BandParams&, cudaStream_t);

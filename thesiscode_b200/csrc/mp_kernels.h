@@ -65,7 +65,17 @@ struct Fp64BandParams {
     double* thr;
     double thr_eps;   // relative margin, wider than the index key's resolution
     double thr_tiny;  // absolute margin near v = m - score = 0
+    unsigned* counter;  // ranks handed out beyond the first wave (zeroed by the launch)
+    int64_t spread;     // set by the launch: every spread-th band is in the first wave
 };
+// Order of the bands: every spread-th band first (longest to shortest), then
+// the others, longest first.
+__host__ __device__ inline int64_t fp64_band_of(int64_t rank, int64_t nbands, int64_t spread) {
+    const int64_t first = (nbands + spread - 1) / spread;
+    if (rank < first) return rank * spread;
+    rank -= first;
+    return rank / (spread - 1) * spread + 1 + rank % (spread - 1);
+}
 constexpr int kFp64WarpsPerBlock = 4;
 constexpr int64_t kFp64ThrPad = 64 * 8 + 64;  // >= the 34R + R rows staged past a band's end
 // Threshold stored after merging `score` (see Fp64BandParams::thr): below the
