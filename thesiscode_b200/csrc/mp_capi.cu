@@ -130,6 +130,20 @@ int reserve(mp_context* ctx, size_t bytes) {
 }
 
 
+// reserve() of `base` bytes and, where the budget, a lent scratch and the device
+// have room, `extra` more from align_up(base) on that the call can do without
+// (`has_extra`: they are there).
+int reserve_with(mp_context* ctx, size_t base, size_t extra, bool& has_extra) {
+    has_extra = false;
+    const size_t all = align_up(base) + extra;
+    if (extra > 0 && (!ctx->budget || all <= ctx->budget) &&
+        (all <= ctx->arena_bytes || (!ctx->lent && reserve(ctx, all) == MP_OK))) {
+        has_extra = true;
+        return MP_OK;
+    }
+    return reserve(ctx, base);
+}
+
 // Key shards spread the 64-bit max reductions of concurrently running bands
 // (which all walk the same columns) over more addresses; kept small enough
 // (~32 MB of keys) to stay resident in L2.
@@ -386,7 +400,16 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
     if (precision == MP_PREC_FP64) {
         const int64_t B = blocklen > 0 ? blocklen : 500;
         const int shards = fp64_shards(PL);
-        rc = reserve(ctx, fp64_scratch(n, m, ndiag, !o_dev));
+        const size_t base = fp64_scratch(n, m, ndiag, !o_dev);
+        std::vector<Fp64Split> splits;
+        size_t extra = 0;
+        for (const DiagRange& r : ranges) {
+            const int R = pick_fp64_R(r.hi - r.lo);
+            splits.push_back(fp64_split_plan(PL, r.lo, r.hi, R));
+            extra = std::max(extra, fp64_split_bytes(splits.back(), r.hi - r.lo, R));
+        }
+        bool split = false;
+        rc = reserve_with(ctx, base, extra, split);
         if (rc) return rc;
         Carve cv{(char*)ctx->arena};
         double* Apad = cv.take<double>(n + 1);
@@ -457,6 +480,13 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             P.thr_eps = fp64_threshold_eps(P.idx_bits);
             P.thr_tiny = fp64_threshold_tiny(P.m);
             P.counter = counter;
+            if (split && splits[&r - ranges.data()].L > 0) {
+                P.split = splits[&r - ranges.data()];
+                fp64_split_carve(P.split, nd, R, (char*)ctx->arena + align_up(base));
+                launch_fp64_seeds(P, Apad, n + 1, Apad, n + 1, m, st);
+                MP_LAUNCHED(ctx);
+                ++ctx->launches;  // the rows that two tiles meet
+            }
             launch_band(R, P, st);
             MP_LAUNCHED(ctx);
         }
@@ -866,7 +896,10 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
                   2 * align_up(8 * (size_t)region) * 2 + 2 * align_up(8 * (size_t)(T + m)) +
                   4 * align_up(8 * (size_t)T) + align_up(8 * (size_t)(region + kFp64ThrPad)) +
                   4096;
-    int rc = reserve(ctx, need);
+    const int R = pick_fp64_R(nq);
+    Fp64Split split = fp64_split_plan(T, 0, nq, R);
+    bool has_split = false;
+    int rc = reserve_with(ctx, need, fp64_split_bytes(split, nq, R), has_split);
     if (rc) return rc;
     Carve cv{(char*)ctx->arena};
     double4* colrec = cv.take<double4>(nrec);
@@ -915,7 +948,6 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     MP_LAUNCHED(ctx);
 
     Fp64BandParams P{};
-    const int R = pick_fp64_R(nq);
     P.colrec = colrec;
     P.rowrec = rowrec;
     P.qt0 = q;
@@ -943,6 +975,13 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     P.thr_eps = fp64_threshold_eps(ib);
     P.thr_tiny = fp64_threshold_tiny(P.m);
     P.counter = counter;
+    if (has_split) {
+        P.split = split;
+        fp64_split_carve(P.split, nq, R, (char*)ctx->arena + align_up(need));
+        launch_fp64_seeds(P, ah, T + m, av, T + m, m, st);
+        MP_LAUNCHED(ctx);
+        ++ctx->launches;  // the rows that two tiles meet
+    }
     launch_band(R, P, st);
     MP_LAUNCHED(ctx);
     block_finalize_kernel<<<grid_for(region), kThreads, 0, st>>>(kex, kid, region, 1, region, ib,

@@ -52,15 +52,17 @@
 //
 // What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 5
 // per cell (40 of a step's 62 instructions at R = 8); other instructions cost it
-// about 0.7 cycles each.  n = 1,048,576, m = 256: 262 ms, from 441 ms with the
-// selection tested per step in FP64 and the bands in order of length (spread
-// alone: 269 ms, with the gate per step).  3 CTAs of 4 warps per SM at 168
-// registers spill and run at 273 ms.
+// about 0.7 cycles each.  n = 1,048,576, m = 256: 254 ms, from 441 ms with the
+// selection tested per step in FP64 and the bands in order of length (gate per
+// step 269 ms; a pass's two chunks as a loop 271 ms; 3 CTAs of 4 warps per SM at
+// 168 registers spill, 273 ms).  With fewer bands than resident warps the longest
+// band sets the time; then the bands are cut into tiles (Fp64Split).
 #include <float.h>
 #include <limits.h>
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "mp_common.cuh"
 #include "mp_kernels.h"
@@ -102,6 +104,29 @@ __device__ __forceinline__ void flush_fp64(const Fp64BandParams& P, int shard, i
     if (t >= 0.0) atomicMax(reinterpret_cast<long long*>(P.thr + slot), __double_as_longlong(t));
 }
 
+// A row's best cell of the band: merged into its key slot.
+__device__ __forceinline__ void flush_row(const Fp64BandParams& P, int shard, int64_t r, double score,
+                                          int j) {
+    if (score > P.floor) flush_fp64(P, shard, r + P.row_key_off, score, j + P.col_nb_off);
+}
+// Row t of tile lt (its rows start at rb; seg > 0: the band has a tile before it;
+// more: one after it) has met the whole tile.
+template <int R>
+__host__ __device__ __forceinline__ bool seam_row(int64_t t, int64_t L, int64_t seg, bool more) {
+    return (seg > 0 && t < 32 * R) || (more && t >= L);
+}
+template <int R>
+__device__ __forceinline__ void finish_row(const Fp64BandParams& P, int shard, int64_t lt, int64_t seg,
+                                           bool more, int64_t rb, int64_t t, double score, int j) {
+    if (seam_row<R>(t, P.split.L, seg, more)) {
+        const int64_t i = lt * (P.split.L + 32 * R) + t;
+        P.split.seam_s[i] = score;
+        P.split.seam_j[i] = j;
+    } else if (j >= 0) {
+        flush_row(P, shard, rb + t, score, j);
+    }
+}
+
 // A bound's high word for the integer gate: scores at or above a non-negative
 // bound have a high word at or above its high word (as signed integers); a
 // negative bound lets every cell through.
@@ -133,7 +158,7 @@ struct BandSmem {
     char* col;     // column records, two buffers of kU * R
     double* best;  // best score of each row (its threshold while src < 0)
     double* cthr;  // column thresholds, two buffers of kU * R
-    int* src;      // its column, -1: none yet
+    int* src;      // column of a row's best score, -1: none yet
     int* gate;     // per group: smallest gate among the rows' best scores
     __device__ __forceinline__ BandSmem(char* p) {
         rec = p;
@@ -163,24 +188,16 @@ struct BandSmem {
 template <int R>
 __device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard, unsigned j,
                                               const double (&sc)[R], int64_t g0, int lane) {
-    // lane's best cell of the column: pairwise tree, left wins ties.  A NaN
-    // cell (a constant window) never selects under the reference's '>'; as
-    // -DBL_MAX it also cannot hide the cell it is paired with in the tree.
+    // lane's best cell of the column.  A NaN cell (a constant window) never
+    // selects under the reference's '>'; as -DBL_MAX it also cannot hide the
+    // cell it is paired with in the tree.
     double cb[R];
-    int ca[R];
 #pragma unroll
-    for (int a = 0; a < R; ++a) {
-        cb[a] = sc[a] == sc[a] ? sc[a] : -DBL_MAX;
-        ca[a] = a;
-    }
+    for (int a = 0; a < R; ++a) cb[a] = sc[a] == sc[a] ? sc[a] : -DBL_MAX;
 #pragma unroll
     for (int w = 1; w < R; w *= 2)
 #pragma unroll
-        for (int a = 0; a + w < R; a += 2 * w)
-            if (cb[a + w] > cb[a]) {
-                cb[a] = cb[a + w];
-                ca[a] = ca[a + w];
-            }
+        for (int a = 0; a + w < R; a += 2 * w) cb[a] = cb[a + w] > cb[a] ? cb[a + w] : cb[a];
     const double cbest = cb[0];
     const unsigned long long key = (cbest > P.floor) ? ord_f64(cbest) : 0ull;
     const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
@@ -188,55 +205,26 @@ __device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard
     const unsigned mlo = __reduce_max_sync(kFullMask, hi == mhi ? lo : 0u);
     const bool top = (hi == mhi) && (lo == mlo) && (mhi != 0u);
     const unsigned tops = __ballot_sync(kFullMask, top);
-    if (top && (tops & ((1u << lane) - 1u)) == 0u)
-        flush_fp64(P, shard, j + P.col_key_off, cbest, j + g0 + ca[0] + P.row_nb_off);
-}
-
-// Selection of one column step: every cell above its row's best replaces it
-// (strict '>', the reference's rule; a step's cells lie in distinct rows), and
-// a column with a cell above its threshold tc is reduced over the warp.  Cell a
-// of column b is element b + a of the lane's two groups, in slots s0 and s1.
-template <int R>
-__device__ __forceinline__ void select_step(const Fp64BandParams& P, int shard, int b, unsigned j,
-                                            const double (&sc)[R], const BandSmem<R>& sm, int s0,
-                                            int s1, double tc, int64_t gb, int lane) {
-    __syncwarp();  // rows move from lane to lane between steps
-    bool col = false;
+    if (top && (tops & ((1u << lane) - 1u)) == 0u) {
+        int ca = R - 1;
 #pragma unroll
-    for (int a = 0; a < R; ++a) {
-        const int e = b + a < R ? s0 * (R + 1) + b + a : s1 * (R + 1) + b + a - R;
-        if (sc[a] > sm.best[e]) {
-            sm.best[e] = sc[a];
-            sm.src[e] = (int)j;
-        }
-        col |= sc[a] > tc;
+        for (int a = R - 2; a >= 0; --a) ca = sc[a] == cbest ? a : ca;
+        flush_fp64(P, shard, j + P.col_key_off, cbest, j + g0 + ca + P.row_nb_off);
     }
-    if (__any_sync(kFullMask, col)) select_column<R>(P, shard, j, sc, gb + lane * R, lane);
 }
 
-// One chunk = R consecutive columns, in one of three ways:
-//   kGate    only cells of the reference's 4-wide (fused) part, no selection:
-//            returns the largest high word of the lane's scores
-//   kSelect  the same cells again with the selection, for a chunk whose gate
-//            opened: per step behind the gate
-//   kEdge    any cells, each with its own geometry; every step selects
-// On entry rwin holds the records of the lane's first group, on return those of
-// its second.
-// (sel: set when a step selected).
-enum ChunkWay { kGate, kSelect, kEdge };
-template <int R, ChunkWay WAY>
-__device__ __forceinline__ int chunk_fp64(const Fp64BandParams& P, int shard, unsigned jc,
-                                          const BandSmem<R>& sm, int s0, int s1,
-                                          const char* col, const double* cthr,
-                                          double4 (&rwin)[R], double (&qt)[R], int gate,
-                                          unsigned geo, int64_t gb, int lane, bool& sel) {
-    const int len0 = (int)(P.Tbase - gb) - lane * R;  // columns of the lane's first diagonal
+// One chunk = R consecutive columns, all their cells in the reference's 4-wide
+// (fused) part, without the selection: the largest high word of the lane's
+// scores.  On entry rwin holds the records of the lane's first group (slot s1 - 1),
+// on return those of its second.
+template <int R>
+__device__ __forceinline__ int gate_chunk(const BandSmem<R>& sm, int s1, const char* col,
+                                          double4 (&rwin)[R], double (&qt)[R]) {
     int top = INT_MIN;
     const char* rec1 = sm.rec + s1 * BandSmem<R>::kRecStride;
     double4 cv = ring_rec(col);
 #pragma unroll
     for (int b = 0; b < R; ++b) {
-        const unsigned j = jc + b;
         double4 cn = cv;
         if (b + 1 < R) cn = ring_rec(col + 32 * (b + 1));
         double sc[R];
@@ -245,12 +233,56 @@ __device__ __forceinline__ int chunk_fp64(const Fp64BandParams& P, int shard, un
             const double4 rv = rwin[(b + a) % R];
             // the window moves on: element b + R replaces element b
             if (a == 0) rwin[b] = ring_rec(rec1 + 32 * b);
+            // kernels.cpp:206-225
+            const double ss = __dmul_rn(rv.z, cv.z);
+            const double mm = __dmul_rn(cv.w, rv.w);
+            sc[a] = __fma_rn(qt[a], ss, -mm);
+            qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
+        }
+        cv = cn;
+        if (R == 1) top = max(top, __double2hiint(sc[0]));
+#pragma unroll
+        for (int a = 0; a + 1 < R; a += 2)
+            top = __vimax3_s32(top, __double2hiint(sc[a]), __double2hiint(sc[a + 1]));
+    }
+    return top;
+}
+
+// A pass of kU chunks with the selection, s0 the slot of the lane's first group:
+// EDGE evaluates every cell with its own geometry and selects in every step;
+// otherwise all cells are fused and a step selects behind the gate.  A step's
+// selection: every cell above its row's best replaces it (strict '>', the
+// reference's rule; a step's cells lie in distinct rows), and a column whose
+// largest high word reaches its threshold's is reduced over the warp.  Returns
+// whether a step selected.  One loop over the columns with the records read from
+// shared memory: unrolled like gate_chunk, this path's code pushed the passes
+// without selection out of the instruction cache.
+template <int R, bool EDGE>
+__device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, unsigned jc,
+                                            const BandSmem<R>& sm, int s0, const char* col,
+                                            const double* cthr, double (&qt)[R], int gate,
+                                            unsigned geo, int64_t gb, int lane) {
+    constexpr int RS = BandSmem<R>::kRecStride;
+    bool sel = false;
+#pragma unroll 1
+    for (int b = 0; b < kU * R; ++b) {
+        const unsigned j = jc + b;
+        const int k = b % R;  // cell a lies in element k + a of the lane's groups
+        const int sa = wrap_group(s0 + b / R), sb = wrap_group(sa + 1);
+        const char* rec0 = sm.rec + sa * RS + 32 * k;
+        const char* rec1 = sm.rec + sb * RS + 32 * (k - R);
+        const double4 cv = ring_rec(col + 32 * b);
+        double sc[R];
+        int top = INT_MIN;
+#pragma unroll
+        for (int a = 0; a < R; ++a) {
+            const double4 rv = ring_rec((k + a < R ? rec0 : rec1) + 32 * a);
             double score = -DBL_MAX;
             const unsigned code = (geo >> (4 * a)) & 15u;
-            if (WAY != kEdge || (code != 15u && (int64_t)j < len0 - a)) {
+            const int64_t left = P.Tbase - gb - (lane * R + a) - (int64_t)j;  // columns from j on
+            if (!EDGE || (code != 15u && left > 0)) {
                 const double ss = __dmul_rn(rv.z, cv.z);
-                if (WAY != kEdge || (code != 7u && (int64_t)j <= len0 - a - 4 + (int)code)) {
-                    // 4-wide part of the reference kernel (kernels.cpp:206-225)
+                if (!EDGE || (code != 7u && left >= 4 - (int)code)) {
                     const double mm = __dmul_rn(cv.w, rv.w);
                     score = __fma_rn(qt[a], ss, -mm);
                     qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
@@ -262,38 +294,51 @@ __device__ __forceinline__ int chunk_fp64(const Fp64BandParams& P, int shard, un
                 }
             }
             sc[a] = score;
+            top = max(top, __double2hiint(score));
         }
-        cv = cn;
-        if (WAY != kEdge) {
-            if (WAY == kSelect) top = INT_MIN;
-            if (R == 1) top = max(top, __double2hiint(sc[0]));
+        if (!EDGE && !__any_sync(kFullMask, top >= gate)) continue;
+        sel = true;
+        __syncwarp();  // rows move from lane to lane between steps
+        const int e0 = sa * (R + 1) + k, e1 = sb * (R + 1) + k - R;
+        double best[R];
 #pragma unroll
-            for (int a = 0; a + 1 < R; a += 2)
-                top = __vimax3_s32(top, __double2hiint(sc[a]), __double2hiint(sc[a + 1]));
-        }
-        if (WAY == kEdge || (WAY == kSelect && __any_sync(kFullMask, top >= gate))) {
-            select_step<R>(P, shard, b, j, sc, sm, s0, s1, cthr[b], gb, lane);
-            sel = true;
-        }
+        for (int a = 0; a < R; ++a) best[a] = sm.best[(k + a < R ? e0 : e1) + a];
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+            if (sc[a] > best[a]) {
+                sm.best[(k + a < R ? e0 : e1) + a] = sc[a];
+                sm.src[(k + a < R ? e0 : e1) + a] = (int)j;
+            }
+        if (__any_sync(kFullMask, top >= fp64_gate(cthr[b])))
+            select_column<R>(P, shard, j, sc, gb + lane * R, lane);
     }
-    return top;
+    return sel;
 }
 
+// Columns [j0, jend) of a band.  lt: the tile's number when the band is cut into
+// tiles (then jend - j0 = L, or less for the band's last tile).
 template <int R>
-__device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band, int lane,
-                                          int shard, const BandSmem<R>& sm) {
+__device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band, int64_t lt,
+                                          int64_t seg, int lane, int shard,
+                                          const BandSmem<R>& sm) {
     constexpr int RS = BandSmem<R>::kRecStride;
     const int64_t gb = P.g_lo + band * (int64_t)(32 * R);
     const int64_t g0 = gb + (int64_t)lane * R;
-    const int jmax = (int)(P.Tbase - gb);  // length of the band's longest diagonal
-    if (jmax <= 0) return;
+    const int64_t jmax = P.Tbase - gb;  // length of the band's longest diagonal
+    const int64_t L = P.split.L;
+    const unsigned j0 = (unsigned)(seg * L);
+    if ((int64_t)j0 >= jmax) return;
+    const bool more = L > 0 && j0 + L < jmax;  // the band goes on in the next tile
+    const unsigned jend = more ? j0 + (unsigned)L : (unsigned)jmax;
+    const int64_t rb = gb + j0;  // row t = 0 of the tile
 
     // Diagonal g has len = Tbase - g columns; with delta its offset in its block,
     // its last column of the reference's 4-wide part is len - 4 + delta % 4, or
     // none when delta >= B & ~3.  geo holds delta % 4 (or 7) of the lane's
     // diagonals, 15 for one past g_hi, as nibbles: only the chunks near a
-    // diagonal's end read them.  A diagonal past g_hi carries -inf, which stays
-    // below every bound, so it does not cost the band its branch-free chunks.
+    // diagonal's end read them.  A diagonal past g_hi, or one that ended before
+    // the tile, carries -inf, which stays below every bound, so it does not cost
+    // the tile its branch-free passes.
     double qt[R];
     unsigned geo = 0;
     int minpsw = INT_MAX;
@@ -302,9 +347,10 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         const int64_t g = g0 + a;
         unsigned code = 15;
         qt[a] = -__longlong_as_double(0x7ff0000000000000ll);
-        if (g < P.g_hi) {
+        if (g < P.g_hi && (int64_t)j0 < P.Tbase - g) {
             const int64_t delta = (g - P.blk_origin) % P.B;
-            qt[a] = P.qt0[g - P.g_lo];
+            qt[a] = seg == 0 ? P.qt0[g - P.g_lo]
+                             : P.split.seeds[(seg - 1) * (P.g_hi - P.g_lo) + (g - P.g_lo)];
             code = delta < (P.B & ~3ll) ? (unsigned)(delta & 3) : 7u;
             minpsw = min(minpsw, code == 7u ? -1 : (int)(P.Tbase - g) - 4 + (int)code);
         }
@@ -317,10 +363,10 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     // next columns': part = lane % 16.
     const int part = lane & 15;
     const bool isrow = lane < 16;
-    const uint4* rsrc = reinterpret_cast<const uint4*>(P.rowrec + gb);
-    const uint4* crec = reinterpret_cast<const uint4*>(P.colrec);
-    const double* tsrc = P.thr + gb + P.row_key_off;  // threshold of row t
-    const double* csrc = P.thr + P.col_key_off;       // threshold of column j
+    const uint4* rsrc = reinterpret_cast<const uint4*>(P.rowrec + rb);
+    const uint4* crec = reinterpret_cast<const uint4*>(P.colrec + j0);
+    const double* tsrc = P.thr + rb + P.row_key_off;  // threshold of row t
+    const double* csrc = P.thr + j0 + P.col_key_off;  // threshold of column j0
     for (int i = lane; i < (32 + kU) * 2 * R; i += 32)
         *reinterpret_cast<uint4*>(sm.rec + (i / (2 * R)) * RS + 16 * (i % (2 * R))) =
             __ldg(rsrc + i);
@@ -355,7 +401,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     int sf = 0;     // slot of group c, the first that the pass finishes
     int cbuf = 0;
     bool sel = false;
-    for (unsigned jc = 0; jc < (unsigned)jmax; jc += kU * R) {
+    for (unsigned jc = j0; jc < jend; jc += kU * R) {
         const int sn = wrap_group(sf + 32 + kU);  // slots of the incoming groups (kU divides kGroups)
         double t = 0.0;
         if (lane < 2 * R * kU) {
@@ -372,49 +418,36 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         for (int u = 0; u <= kU; ++u) gate = min(gate, sm.gate[wrap_group(s0 + u)]);
         const char* col = sm.col + cbuf * (32 * R * kU);
         const double* cthr = sm.cthr + cbuf * (R * kU);
-        if ((int64_t)jc + (kU * R - 1) <= minpsw) {
-            bool open = sel;  // a pass after one that selected goes straight to selecting
-            if (!open) {
-                double q0[R];
+        const bool fused = (int64_t)jc + (kU * R - 1) <= minpsw;
+        bool open = !fused || sel;  // a pass after one that selected goes straight to selecting
+        if (!open) {
+            double q0[R];
 #pragma unroll
-                for (int a = 0; a < R; ++a) q0[a] = qt[a];
-                int top = INT_MIN;
-#pragma unroll 1
-                for (int u = 0; u < kU; ++u)
-                    top = max(top, chunk_fp64<R, kGate>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
-                                                        col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, open));
-                open = __any_sync(kFullMask, top >= gate);
-                if (open) {
+            for (int a = 0; a < R; ++a) q0[a] = qt[a];
+            int top = INT_MIN;
 #pragma unroll
-                    for (int a = 0; a < R; ++a) {
-                        qt[a] = q0[a];
-                        rwin[a] = ring_rec(sm.rec + s0 * RS + 32 * a);
-                    }
-                }
-            }
-            sel = false;
-            if (open) {
-#pragma unroll 1
-                for (int u = 0; u < kU; ++u)
-                    chunk_fp64<R, kSelect>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
-                                           col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, sel);
-            }
-        } else {
-            sel = true;
-#pragma unroll 1
             for (int u = 0; u < kU; ++u)
-                chunk_fp64<R, kEdge>(P, shard, jc + u * R, sm, wrap_group(s0 + u), wrap_group(s0 + u + 1),
-                                     col + u * 32 * R, cthr + u * R, rwin, qt, gate, geo, gb, lane, sel);
+                top = max(top, gate_chunk<R>(sm, wrap_group(s0 + u + 1), col + u * 32 * R, rwin, qt));
+            open = __any_sync(kFullMask, top >= gate);
+            if (open) {
+#pragma unroll
+                for (int a = 0; a < R; ++a) qt[a] = q0[a];
+            }
+        }
+        sel = false;
+        if (open) {
+            sel = fused ? select_pass<R, false>(P, shard, jc, sm, s0, col, cthr, qt, gate, geo, gb, lane)
+                        : select_pass<R, true>(P, shard, jc, sm, s0, col, cthr, qt, gate, geo, gb, lane);
+            const char* r0 = sm.rec + wrap_group(s0 + kU) * RS;
+#pragma unroll
+            for (int a = 0; a < R; ++a) rwin[a] = ring_rec(r0 + 32 * a);
         }
         __syncwarp();
         // groups c .. c + kU - 1 have met every lane: merge their rows
         if (lane < R * kU) {
             const int e = (sf + lane / R) * (R + 1) + lane % R;
             const int j = sm.src[e];
-            if (j >= 0) {
-                const double s = sm.best[e];
-                if (s > P.floor) flush_fp64(P, shard, jc + gb + lane + P.row_key_off, s, j + P.col_nb_off);
-            }
+            finish_row<R>(P, shard, lt, seg, more, rb, (int64_t)(jc - j0) + lane, sm.best[e], j);
         }
         // the incoming groups and columns begin at their thresholds
         if (part < R * kU) {
@@ -442,22 +475,20 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     }
 
     // drain: rows of groups c .. c + 31 (the last chunk's second groups)
-    const int64_t tend = ((int64_t)jmax + kU * R - 1) / (kU * R) * (kU * R);  // row t of group c
+    const int64_t tend = ((int64_t)(jend - j0) + kU * R - 1) / (kU * R) * (kU * R);  // row t of group c
     for (int i = lane; i < 32 * R; i += 32) {
-        const int s = wrap_group(sf + i / R);
-        const int e = s * (R + 1) + i % R;
+        const int e = wrap_group(sf + i / R) * (R + 1) + i % R;
         const int j = sm.src[e];
-        if (j >= 0) {
-            const double v = sm.best[e];
-            if (v > P.floor) flush_fp64(P, shard, tend + gb + i + P.row_key_off, v, j + P.col_nb_off);
-        }
+        finish_row<R>(P, shard, lt, seg, more, rb, tend + i, sm.best[e], j);
     }
     __syncwarp();
 
-    if (P.qt_out) {
+    if (P.qt_out) {  // diagonals whose last column lies in the tile
 #pragma unroll
-        for (int a = 0; a < R; ++a)
-            if (g0 + a < P.g_hi) P.qt_out[g0 + a - P.g_lo] = qt[a];
+        for (int a = 0; a < R; ++a) {
+            const int64_t g = g0 + a, len = P.Tbase - g;
+            if (g < P.g_hi && (int64_t)j0 < len && len <= (int64_t)jend) P.qt_out[g - P.g_lo] = qt[a];
+        }
     }
 }
 
@@ -473,20 +504,291 @@ __global__ void __launch_bounds__(32 * kFp64WarpsPerBlock, R == 8 ? 2 : 4)
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const BandSmem<R> sm(smem_fp64 + w * BandSmem<R>::kBytes);
-    // One resident wave of W warps takes the bands by rank (fp64_band_of): warp
-    // w starts with rank w, later ranks come from one counter (no waiting on
-    // anything).
+    // One resident wave of W warps takes the bands by rank (fp64_band_of), or the
+    // tiles by number: warp w starts with rank w, later ranks come from one
+    // counter (no waiting on anything).
     const int64_t wid = (int64_t)blockIdx.x * kFp64WarpsPerBlock + w;
     const int shard = (int)(wid % P.shards);
-    for (int64_t rank = wid; rank < P.nbands;) {
-        band_fp64<R>(P, fp64_band_of(rank, P.nbands, P.spread), lane, shard, sm);
+    const int64_t count = P.split.L > 0 ? P.split.ntiles : P.nbands;
+    for (int64_t rank = wid; rank < count;) {
+        int64_t band, seg = 0;
+        bool any = true;
+        if (P.split.L > 0)
+            any = tile_of_pair(rank, P.Tbase, P.g_lo, P.split.L, P.nbands, P.split.seg_per_pair,
+                               32 * R, band, seg);
+        else
+            band = fp64_band_of(rank, P.nbands, P.spread);
+        if (any) band_fp64<R>(P, band, rank, seg, lane, shard, sm);
         unsigned next = 0;
         if (lane == 0) next = atomicAdd(P.counter, 1u);
         rank = (int64_t)gridDim.x * kFp64WarpsPerBlock + __shfl_sync(kFullMask, next, 0);
     }
 }
 
+// Rows met by several tiles of a band: the block of tile lt takes the rows whose
+// last tile (or the band's last) it is; the earlier tile's cell (smaller column)
+// wins ties, as within a tile.
+template <int R>
+__global__ void fp64_seam_kernel(const Fp64BandParams P) {
+    const int64_t lt = blockIdx.x, L = P.split.L, stride = L + 32 * R;
+    int64_t band, seg;
+    if (!tile_of_pair(lt, P.Tbase, P.g_lo, L, P.nbands, P.split.seg_per_pair, 32 * R, band, seg) ||
+        seg == 0)
+        return;
+    const int64_t gb = P.g_lo + band * (32 * R);
+    const int64_t last = (P.Tbase - gb + L - 1) / L - 1;  // the band's last tile
+    // rows x = t + seg L of the band: t < L, or all of the last tile's
+    const int64_t rows = min((int64_t)(32 * R), seg == last ? stride : L);
+    for (int64_t t = threadIdx.x; t < rows; t += blockDim.x) {
+        const int64_t x = seg * L + t;
+        double s = 0.0;
+        int j = -1;
+        for (int64_t k = max((int64_t)0, (x - stride) / L); k <= seg; ++k) {
+            const int64_t tk = x - k * L;
+            if (tk >= stride || !seam_row<R>(tk, L, k, k < last)) continue;
+            const int64_t i = (lt - (seg - k)) * stride + tk;
+            const int jk = P.split.seam_j[i];
+            if (jk >= 0 && (j < 0 || P.split.seam_s[i] > s)) {
+                s = P.split.seam_s[i];
+                j = jk;
+            }
+        }
+        if (j >= 0) flush_row(P, (int)(lt % P.shards), gb + x, s, j);
+    }
+}
+
+// ---- running dot products at the tiles' first columns ------------------------
+// The recurrence of a diagonal is a chain of two dependent FP64 operations per
+// column, 8 cycles each, and a thread per diagonal cannot run ahead of it: 16
+// cycles per column of the longest diagonal bound this kernel (n = 16,384: 0.14
+// ms, 0.28 measured; n = 65,536: 0.55 ms, 1.10 measured).  Above two blocks of
+// diagonals per SM a thread walks C = 4 adjacent ones, so that 4 chains overlap
+// and a value of the series read from shared memory serves 4.  Operands are
+// staged there a chunk ahead; row values lie C + 1 apart per C, so that lanes hit
+// distinct banks.
+constexpr int kSeedThreads = 128;
+constexpr int kSeedChunk = 128;
+
+// 8-byte asynchronous copy that writes zero where !inside.
+__device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
+                 "r"(inside ? 8 : 0)
+                 : "memory");
+}
+
+template <int C>
+__global__ void __launch_bounds__(kSeedThreads)
+    fp64_seed_kernel(const Fp64BandParams P, const double* __restrict__ Ah, int64_t nh,
+                     const double* __restrict__ Av, int64_t nv, int64_t m) {
+    constexpr int K = kSeedChunk, T = kSeedThreads;
+    static_assert(K == T && T % 8 == 0 && (C == 1 || C == 4), "a thread stages one row and one column per chunk");
+    // Ring of rows in blocks of K: a chunk reads rows [0, T*C + K) from its first
+    // while the next K arrive; block 0 is mirrored behind the ring (with 8 + C
+    // rows more, read ahead and not used), so a lane's rows of a chunk never wrap.
+    constexpr int kBlocks = C + 2;
+    constexpr int kRing = kBlocks * K + K + 16;
+    constexpr int kPad = C > 1 ? kRing / C : 0;
+    __shared__ double2 scol[2][K + 16];                   // {A[j], A[j+m]}
+    __shared__ double srow[2][kRing + kPad];              // A[r], A[r+m]
+    const int tid = threadIdx.x;
+    const int64_t d0 = (int64_t)blockIdx.x * (T * C);     // first diagonal, from g_lo
+    const int64_t nd = P.g_hi - P.g_lo, L = P.split.L;
+    const int64_t gb = P.g_lo + d0, g0 = gb + (int64_t)tid * C;
+    const int64_t jlast = (P.Tbase - gb - 1) / L * L;     // start of the longest diagonal's last tile
+    if (jlast <= 0) return;
+    double q[C];
+    int64_t psw[C], minpsw = P.Tbase;
+#pragma unroll
+    for (int a = 0; a < C; ++a) {
+        const int64_t g = g0 + a;
+        q[a] = 0.0;
+        psw[a] = P.Tbase;
+        if (g < P.g_hi) {
+            const int64_t delta = (g - P.blk_origin) % P.B;
+            q[a] = P.qt0[g - P.g_lo];
+            psw[a] = delta < (P.B & ~3ll) ? P.Tbase - g - 4 + (delta & 3) : -1;
+            // cells past a diagonal's last tile start feed nothing
+            if (P.Tbase - g > L) minpsw = min(minpsw, psw[a]);
+        }
+    }
+    // rows gb + i, i in block bi of the ring (i = K * (number of blocks before))
+    auto stage_rows = [&](int64_t i, int bi) {
+        const int64_t r = gb + i + tid;
+        const bool in0 = r < nv, in1 = r + m < nv;
+        const double *p0 = Av + (in0 ? r : 0), *p1 = Av + (in1 ? r + m : 0);
+        int e = bi * K + tid;
+        e += C > 1 ? e / C : 0;
+        cp_async8_or_zero(&srow[0][e], p0, in0);
+        cp_async8_or_zero(&srow[1][e], p1, in1);
+        if (bi == 0) {
+            e += kBlocks * K + (C > 1 ? kBlocks * K / C : 0);
+            cp_async8_or_zero(&srow[0][e], p0, in0);
+            cp_async8_or_zero(&srow[1][e], p1, in1);
+        }
+    };
+    auto stage_cols = [&](int64_t jc, int buf) {
+        const int64_t j = jc + tid;
+        const bool in0 = j < nh, in1 = j + m < nh;
+        cp_async8_or_zero(&scol[buf][tid].x, Ah + (in0 ? j : 0), in0);
+        cp_async8_or_zero(&scol[buf][tid].y, Ah + (in1 ? j + m : 0), in1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int bi = 0; bi <= C; ++bi) stage_rows((int64_t)bi * K, bi);
+    stage_cols(0, 0);
+    // dot products at a tile's first column (kFp64SplitUnit columns apart or more)
+    int64_t jnext = L;
+    double* out = P.split.seeds + d0 + (int64_t)tid * C;
+    auto leave = [&](int64_t j) {
+        if (j != jnext) return;
+#pragma unroll
+        for (int a = 0; a < C; ++a)
+            if (g0 + a < P.g_hi && j < P.Tbase - (g0 + a)) out[a] = q[a];
+        jnext += L;
+        out += nd;
+    };
+    int buf = 0;
+    int bl = 0;  // block of the chunk's first row
+    for (int64_t jc = 0;; jc += K, buf ^= 1, bl = bl + 1 == kBlocks ? 0 : bl + 1) {
+        if (jc > jlast) break;
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        // rows [T*C + K, T*C + 2K) from the chunk's first: the block before it
+        stage_rows(jc + T * C + K, bl == 0 ? kBlocks - 1 : bl - 1);
+        stage_cols(jc + K, buf ^ 1);
+        // lane's first row of the chunk: block bl, element tid * C, modulo the ring
+        int rs = bl * K + tid * C;
+        rs = rs < kBlocks * K ? rs : rs - kBlocks * K;
+        const double* ra = srow[0] + rs + (C > 1 ? rs / C : 0);
+        const double* rm = srow[1] + rs + (C > 1 ? rs / C : 0);
+        double wa[C], wm[C];  // rows of the current column: slot (column + a) % C
+#pragma unroll
+        for (int a = 0; a < C - 1; ++a) {
+            wa[a] = ra[a];
+            wm[a] = rm[a];
+        }
+        if (jc + K - 1 <= minpsw) {
+            // The next U columns' operands are read into the other half of the
+            // registers while these run, each read between the chain's dependent
+            // operations.
+            constexpr int U = 8;
+            static_assert(K % (2 * U) == 0 && U % C == 0 && kFp64SplitUnit % (2 * U) == 0, "tiles start at a round");
+            constexpr int kStep = C > 1 ? U + U / C : U;
+            double xa[2][U], xm[2][U];
+            double2 xc[2][U];
+            auto fetch = [&](int h, int k, const double* pa, const double* pm, const double2* pc) {
+                const int i = k + C - 1, e = C > 1 ? i + i / C : i;
+                xa[h][k] = pa[e];
+                xm[h][k] = pm[e];
+                xc[h][k] = pc[k];
+            };
+            const double2* pc = scol[buf];
+#pragma unroll
+            for (int k = 0; k < U; ++k) fetch(0, k, ra, rm, pc);
+            auto walk = [&](auto starts) {  // starts: a tile starts in the chunk
+#pragma unroll 1
+                for (int k0 = 0; k0 < K; k0 += 2 * U) {
+                    if (decltype(starts)::value) leave(jc + k0);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        ra += kStep;
+                        rm += kStep;
+                        pc += U;
+#pragma unroll
+                        for (int k = 0; k < U; ++k) {
+                            wa[(k + C - 1) % C] = xa[h][k];
+                            wm[(k + C - 1) % C] = xm[h][k];
+#pragma unroll
+                            for (int a = 0; a < C; ++a) q[a] = __fma_rn(wm[(k + a) % C], xc[h][k].y, q[a]);
+                            fetch(h ^ 1, k, ra, rm, pc);  // past the chunk: read, not used
+#pragma unroll
+                            for (int a = 0; a < C; ++a) q[a] = __fma_rn(-wa[(k + a) % C], xc[h][k].x, q[a]);
+                        }
+                    }
+                }
+            };
+            if (jnext < jc + K)
+                walk(std::true_type{});
+            else
+                walk(std::false_type{});
+        } else {
+#pragma unroll 1
+            for (int k0 = 0; k0 < K; k0 += 4) {
+                leave(jc + k0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = k + C - 1, e = C > 1 ? i + i / C : i;
+                    wa[i % C] = ra[e];
+                    wm[i % C] = rm[e];
+                    const double2 c = scol[buf][k0 + k];
+#pragma unroll
+                    for (int a = 0; a < C; ++a) {
+                        const double x = wa[(k + a) % C], y = wm[(k + a) % C];
+                        if (jc + k0 + k <= psw[a])
+                            q[a] = __fma_rn(-x, c.x, __fma_rn(y, c.y, q[a]));
+                        else  // the reference's scalar remainder
+                            q[a] = __dsub_rn(__dadd_rn(q[a], __dmul_rn(y, c.y)), __dmul_rn(x, c.x));
+                    }
+                }
+                ra += C > 1 ? 4 + 4 / C : 4;
+                rm += C > 1 ? 4 + 4 / C : 4;
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
 }  // namespace
+
+Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R) {
+    Fp64Split S{};
+    const int64_t span = 32 * R, nd = g_hi - g_lo;
+    if (nd <= 0) return S;
+    const int64_t nbands = (nd + span - 1) / span;
+    // Whole bands keep the chip busy once there are about as many as resident
+    // warps (8 per SM), and the dot products of the tiles' first columns cost two
+    // more FP64 operations per cell.  Join phase, tiles against whole bands: n =
+    // 2,500 0.11 / 0.83 ms; 16,384 0.57 / 2.2; 65,536 (256 bands) 2.8 / 6.6;
+    // 200,000 (780 bands) 17.1 / 19.5; 260,000 (1,015) 27.5 / 26.8; 300,000 36 / 31.
+    const int64_t warps = (int64_t)sm_count() * 8;
+    if (nbands > warps * 4 / 5) return S;
+    // About 5 tiles per warp (10 and 20 measured the same); at least 32 columns,
+    // for the smallest series, whose tiles are all resident at once (n = 2,500:
+    // 32 columns 0.105 ms, 64 0.127, 256 0.26).
+    const int64_t cols = nbands * (Tbase - g_lo) - span * (nbands * (nbands - 1) / 2);
+    int64_t L = std::max<int64_t>(cols / (5 * warps), 32);
+    L = (L + kFp64SplitUnit - 1) / kFp64SplitUnit * kFp64SplitUnit;
+    if (Tbase - g_lo <= L) return S;
+    S.L = L;
+    S.nseg = (Tbase - g_lo + L - 1) / L;
+    int64_t nb = 0;
+    fp32_tile_plan(Tbase, g_lo, g_hi, L, R, nb, S.seg_per_pair, S.ntiles);
+    return S;
+}
+
+size_t fp64_split_bytes(const Fp64Split& S, int64_t ndiag, int R) {
+    if (S.L == 0) return 0;
+    const size_t rows = (size_t)(S.ntiles * (S.L + 32 * R));
+    return align_up(8 * (size_t)((S.nseg - 1) * ndiag)) + align_up(8 * rows) + align_up(4 * rows);
+}
+
+void fp64_split_carve(Fp64Split& S, int64_t ndiag, int R, char* p) {
+    S.seeds = reinterpret_cast<double*>(p);
+    p += align_up(8 * (size_t)((S.nseg - 1) * ndiag));
+    S.seam_s = reinterpret_cast<double*>(p);
+    p += align_up(8 * (size_t)(S.ntiles * (S.L + 32 * R)));
+    S.seam_j = reinterpret_cast<int*>(p);
+}
+
+void launch_fp64_seeds(const Fp64BandParams& P, const double* Ah, int64_t nh, const double* Av,
+                       int64_t nv, int64_t m, cudaStream_t s) {
+    const int64_t nd = P.g_hi - P.g_lo;
+    const int64_t blocks1 = (nd + kSeedThreads - 1) / kSeedThreads;
+    if (blocks1 <= 2 * sm_count())
+        fp64_seed_kernel<1><<<(unsigned)blocks1, kSeedThreads, 0, s>>>(P, Ah, nh, Av, nv, m);
+    else
+        fp64_seed_kernel<4><<<(unsigned)((blocks1 + 3) / 4), kSeedThreads, 0, s>>>(P, Ah, nh, Av, nv, m);
+}
 
 template <int R>
 void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
@@ -509,15 +811,17 @@ void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
         resident[dev & 63].store(per_sm, std::memory_order_relaxed);
         configured.fetch_or(bit, std::memory_order_release);
     }
-    // one resident wave, fewer CTAs when there are fewer bands than warps
+    // one resident wave, fewer CTAs when there is less work than warps
     const int64_t wave = (int64_t)sm_count() * resident[dev & 63].load(std::memory_order_relaxed);
-    const int64_t want = (Q.nbands + kFp64WarpsPerBlock - 1) / kFp64WarpsPerBlock;
+    const int64_t count = Q.split.L > 0 ? Q.split.ntiles : Q.nbands;
+    const int64_t want = (count + kFp64WarpsPerBlock - 1) / kFp64WarpsPerBlock;
     const int64_t blocks = std::min<int64_t>(want, wave);
     if (blocks <= 0) return;
     Fp64BandParams P = Q;
     P.spread = (P.nbands + blocks * kFp64WarpsPerBlock - 1) / (blocks * kFp64WarpsPerBlock);
     cudaMemsetAsync(P.counter, 0, sizeof(unsigned), s);
     fp64_band_kernel<R><<<(unsigned)blocks, 32 * kFp64WarpsPerBlock, smem, s>>>(P);
+    if (P.split.L > 0) fp64_seam_kernel<R><<<(unsigned)P.split.ntiles, 128, 0, s>>>(P);
 }
 
 template void launch_fp64_band<1>(const Fp64BandParams&, cudaStream_t);

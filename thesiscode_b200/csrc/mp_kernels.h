@@ -40,6 +40,45 @@ __global__ void pack_fp32_kernel(const double* A, int64_t m, int64_t PL, int H, 
 // j < Tbase - g.  The reference's block geometry (blocks of B diagonals
 // starting at blk_origin, triangle length T = Tbase - block start) decides
 // per cell whether the fused or the separately rounded arithmetic applies.
+//
+// Bands cut into tiles of L columns (fp64_split_plan says when).  A tile starts
+// from its diagonals' running dot products at its first column, which
+// launch_fp64_seeds computes beforehand.  A row that several tiles of a band meet
+// keeps the whole band's choice: the tiles leave their best cells of it in
+// seam_s / seam_j, and fp64_seam_kernel merges the best of them.
+struct Fp64Split {
+    int64_t L;             // columns per tile, a multiple of kFp64SplitUnit; 0: whole bands
+    int64_t nseg;          // tiles of the longest band
+    int64_t seg_per_pair;  // tile numbering: see tile_of_pair
+    int64_t ntiles;
+    double* seeds;         // [nseg - 1][g_hi - g_lo]: dot product at column (s + 1) L
+    double* seam_s;        // [ntiles][L + 32R] best score of the tile's row t ...
+    int* seam_j;           // ... and its column, -1: none
+};
+constexpr int64_t kFp64SplitUnit = 16;
+// Number of a tile in a list of band pairs (k, nbands - 1 - k), whose lengths are
+// nearly complementary: pair p = lt / seg_per_pair holds the tiles of K columns of
+// band p, then those of band nbands - 1 - p.  False for the unused tail of a pair.
+// (Host-callable too, so the tile space can be checked without a GPU.)
+__host__ __device__ inline bool tile_of_pair(int64_t lt, int64_t PL, int64_t g_lo, int64_t K,
+                                             int64_t nbands, int64_t seg_per_pair, int64_t span,
+                                             int64_t& band, int64_t& seg) {
+    const int64_t p = lt / seg_per_pair;
+    int64_t s = lt % seg_per_pair;
+    const int64_t nseg0 = (PL - (g_lo + p * span) + K - 1) / K;
+    if (s < nseg0) {
+        band = p;
+        seg = s;
+        return true;
+    }
+    s -= nseg0;
+    const int64_t p2 = nbands - 1 - p;
+    if (p2 <= p) return false;
+    const int64_t nseg1 = (PL - (g_lo + p2 * span) + K - 1) / K;
+    band = p2;
+    seg = s;
+    return s < nseg1;
+}
 struct Fp64BandParams {
     const double4* colrec;  // colrec[j] = {A_hor[j], A_hor[j+m], s_hor[j], mu_hor[j]}
     const double4* rowrec;  // rowrec[r] = {A_vert[r], A_vert[r+m], s_vert[r], mu_vert[r]}
@@ -65,8 +104,9 @@ struct Fp64BandParams {
     double* thr;
     double thr_eps;   // relative margin, wider than the index key's resolution
     double thr_tiny;  // absolute margin near v = m - score = 0
-    unsigned* counter;  // ranks handed out beyond the first wave (zeroed by the launch)
+    unsigned* counter;  // work handed out beyond the first wave (zeroed by the launch)
     int64_t spread;     // set by the launch: every spread-th band is in the first wave
+    Fp64Split split;    // split.L > 0: bands cut into tiles of L columns
 };
 // Order of the bands: every spread-th band first (longest to shortest), then
 // the others, longest first.
@@ -94,6 +134,16 @@ inline double fp64_threshold_eps(int idx_bits) { return std::ldexp(1.0, idx_bits
 inline double fp64_threshold_tiny(double m) { return std::ldexp(m, -40); }
 template <int R>
 void launch_fp64_band(const Fp64BandParams& P, cudaStream_t s);
+// Split plan of a band join over diagonals [g_lo, g_hi) of Tbase columns (L = 0:
+// whole bands), the bytes its buffers need, and the buffers carved from `base`.
+Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R);
+size_t fp64_split_bytes(const Fp64Split& S, int64_t ndiag, int R);
+void fp64_split_carve(Fp64Split& S, int64_t ndiag, int R, char* base);
+// Running dot products at the tiles' first columns: Ah the series along columns,
+// Av along rows (nh and nv values; zero is read past them), P.qt0 the dot products
+// at column 0.
+void launch_fp64_seeds(const Fp64BandParams& P, const double* Ah, int64_t nh, const double* Av,
+                       int64_t nv, int64_t m, cudaStream_t s);
 
 // ---- FP32 re-anchored tile join (mp_join_fp32.cu) ---------------------------
 // One series of a (batched) join.  Its tiles are numbered
@@ -122,28 +172,10 @@ struct Fp32TileParams {
     const double* dg;
 };
 #ifdef __CUDACC__
-// Local tile lt of a series -> (band, column segment): band pair p = lt /
-// seg_per_pair holds bands p and nbands-1-p, whose lengths are nearly
-// complementary; the pair's tiles are its first band's segments, then the
-// second's.  False for the unused tail of a pair.  (Host-callable too, so the
-// tile space can be checked without a GPU.)
+// Local tile lt of a series -> (band, column segment), see tile_of_pair.
 __host__ __device__ __forceinline__ bool fp32_tile_of(const Fp32TileParams& P, int64_t lt, int64_t span,
                                              int64_t& band, int64_t& seg) {
-    const int64_t p = lt / P.seg_per_pair;
-    int64_t s = lt % P.seg_per_pair;
-    const int64_t nseg0 = (P.PL - (P.g_lo + p * span) + P.K - 1) / P.K;
-    if (s < nseg0) {
-        band = p;
-        seg = s;
-        return true;
-    }
-    s -= nseg0;
-    const int64_t p2 = P.nbands - 1 - p;
-    if (p2 <= p) return false;
-    const int64_t nseg1 = (P.PL - (P.g_lo + p2 * span) + P.K - 1) / P.K;
-    band = p2;
-    seg = s;
-    return s < nseg1;
+    return tile_of_pair(lt, P.PL, P.g_lo, P.K, P.nbands, P.seg_per_pair, span, band, seg);
 }
 // Guarded form: does the tile (band start gb, columns [j0, j1)) touch a
 // hazard window, as a column or as a row (rows j + g, g in [gb, gb + span))?
