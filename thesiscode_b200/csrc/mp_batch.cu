@@ -206,7 +206,8 @@ int enqueue_batch(mp_batch* b, cudaStream_t st) {
     batch_pack_kernel<<<grid, 256, 0, st>>>(b->d_series, b->d_A, b->d_mean, b->d_norm, b->d_row,
                                             b->d_col, b->d_key, b->d_ulim);
     cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), st);
-    launch_fp32_join<kR>(b->d_tiles, (int)b->count, b->total_tiles, b->d_counter, st);
+    launch_fp32_join<kR>(b->d_tiles, (int)b->count, b->total_tiles, b->d_counter, st,
+                         fp32_way_of(b->tiles.data(), b->tiles.size()));
     batch_finalize_kernel<<<grid, 256, 0, st>>>(b->d_series, b->d_key, b->d_d2, b->d_idx);
     b->launches = 6;
     const cudaError_t e = cudaGetLastError();

@@ -612,7 +612,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
                                      cudaMemcpyHostToDevice, st));
         MP_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
         // the guarded form's keys name candidate groups, resolved in FP64 below
-        launch_fp32_join<kFp32R>(desc, (int)Ps.size(), ntiles, counter, st, guarded);
+        launch_fp32_join<kFp32R>(desc, (int)Ps.size(), ntiles, counter, st, fp32_way_of(Ps.data(), Ps.size()), guarded);
         MP_LAUNCHED(ctx);
         if (guarded) {
             // the same tiles again: the FP64 pass evaluates those the FP32 pass skipped

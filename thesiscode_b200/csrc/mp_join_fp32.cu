@@ -11,19 +11,27 @@
 //             (the re-anchor; one per K recurrence steps);
 //  recurrence the centred update of SCAMP (Zimmerman et al., SoCC 2019),
 //               cov(j+1, r+1) = cov(j, r) + df[j]*dg[r] + df[r]*dg[j],
-//             in FP32 on the Blackwell f32x2 datapath: diagonals a and a+R/2
-//             share one 64-bit register pair, so every fma/mul instruction
-//             advances two cells;
+//             in FP32 with fused multiply-adds;
 //  distance   u = 1 - cov*nn[j]*nn[r] (= d^2 / 2m) as a single fused op;
 //  min/argmin the low 8 bits of u's bit pattern are replaced by the cell's
 //             position in the band (lane<<3 | a), so one float min tracks
 //             value and origin at once (2^-15 relative resolution, far
-//             inside the 1e-4 target).  Rows accumulate in registers for R
-//             steps (columns go in pairs, so one 3-input min takes a cell
-//             of each column) and then in a per-warp shared-memory ring; a column's
-//             warp minimum is one REDUX instruction.  Finished rows/columns
-//             are merged into the profile with a 64-bit atomicMin on
-//             (ordered u, neighbour).
+//             inside the 1e-4 target).  A row's best tagged distance sits in
+//             the warp's shared memory until the warp's lowest lane has met
+//             the row; a column's warp minimum is one REDUX instruction.
+//             Finished rows/columns are merged into the profile with a 64-bit
+//             atomicMin on (ordered u, neighbour).
+//  gate       almost no cell can lower either minimum, so a pass of 16 columns
+//             first runs the recurrence with one more fused operation per cell,
+//             whose sign says whether the distance is at or below the loosest
+//             bound that the lane meets in the pass: its rows' best distances,
+//             which start just above the rows' keys as they stand in global
+//             memory (a stale key is only a looser start), and the columns'
+//             keys.  A cell that passes neither can change neither key.  When
+//             some lane has a cell that may, the pass is evaluated again with
+//             the selection (dense_pass); a pass that lowered something is
+//             followed by one with the selection straight away, so data that
+//             selects everywhere costs little more than the selection itself.
 //  group keys (the guarded form) a lane takes plain float minima over its
 //             own cells, and only the lane's results carry the lane number
 //             in their low 8 bits (one tag per row or column, not per cell);
@@ -31,6 +39,16 @@
 //             neighbours, among which the finalisation picks with FP64 dot
 //             products (fp32_pick_neighbour) -- which also removes FP32
 //             ranking noise between adjacent diagonals.
+//
+// What bounds it: instruction issue and register reads.  Behind the gate a column of
+// a lane's 8 cells takes 24 fused multiply-adds, 5 others for the test and 3
+// shared-memory reads (12 bytes a lane), 53 cycles of a scheduler; a fused operation
+// with three different operands takes the register file 1.5 cycles (measured;
+// packed f32x2 pairs cost the same words, their pair records twice the
+// shared-memory bandwidth, and minima in place of sign bits three cycles each).
+// n = 1,048,576, m = 256, K = 1024: 128 ms (100 the columns, 10 the passes' ends, 8
+// passes evaluated again, the rest anchors), 178 ms with every pass selecting,
+// which stays the better way for short windows and short series (fp32_gate_pays).
 //
 // Reference semantics kept: strict improvement over the initial score -1
 // (u < 1 + 1/m), NaN never wins (a zero-variance window has nn = NaN).
@@ -44,41 +62,23 @@ namespace mpgpu {
 
 namespace {
 
-// A row record in memory (global and the shared-memory ring): 32 bytes.
-struct RowRec {
-    float4 dfdg;  // (df[j], df[j+H], dg[j], dg[j+H])
-    float4 nn1;   // (nn[j], nn[j+H], 1, 1)
-};
-// The part of a row record a lane keeps in registers (the constant pair stays
-// behind: one shared (1, 1) operand serves every fused distance).
-struct RowWin {
-    float4 dfdg;
-    float2 nn;
-};
-__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
-static_assert(sizeof(RowRec) == 32, "row record is 32 bytes");
+// A row or column record in global memory: (x[j], x[j+4]) pairs of df, dg, nn for
+// rows, (-df, -df, -dg, -dg, nn, nn, 1/nn, 1/nn) for columns.
+constexpr int kRecFloats = 8;
+constexpr int kR = 8;  // diagonals per lane: 8 row terms per column, tags of 3 + 5 bits
 
 constexpr unsigned kTagMask = 0xffu;
 constexpr float kInf = __builtin_huge_valf();
 
-// Row-partial ring: 34 chunks of 8 rows, 12 floats apart (48 bytes), so that
-// the 8 lanes of a quarter-warp merging their chunks with 16-byte accesses
-// hit 8 distinct groups of 4 banks (a 32-byte stride would pair them up).
-constexpr int kRowChunks = 34;
+// Floats between the ring's groups of 8 rows (48 bytes), so that the 8 lanes of a
+// quarter-warp taking a group each with 16-byte accesses hit 8 distinct groups of
+// 4 banks (a 32-byte stride would pair them up).
 constexpr int kRowStride = 12;
 
-// Terms of the FP64 anchor staged per pass: the column's chunk plus the warp's
-// 32*8 + chunk rows (skewed by 1/8) must fit the record ring.
-constexpr int kAnchorChunk = 512;
-static_assert(8 * (kAnchorChunk + (32 * 8 + kAnchorChunk) * 9 / 8) <= kRecRingBytes,
-              "anchor staging fits the record ring");
-
-// 16-byte copy global -> shared that completes asynchronously (cp.async.cg:
-// cached in L2 only); both addresses 16-byte aligned.
-__device__ __forceinline__ void cp_async16(char* dst_smem, const void* src) {
+// 4-byte copy global -> shared that completes asynchronously.
+__device__ __forceinline__ void cp_async4(float* dst_smem, const float* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ float tag_key(float u, unsigned tag) {
@@ -106,43 +106,160 @@ __device__ __forceinline__ void merge_group(unsigned long long* key, float u, in
         atomicMin(key, ((unsigned long long)hi << 32) | kFp32GroupBit | (unsigned long long)base);
 }
 // Row r's minimum over the band, tagged with its lane L: the cells of lane L
-// in row r are (j = r - g, g = gL + a) for a < R with g < g_hi and j >= 0,
-// gL = gb + L*R, i.e. the columns [r - gL - amax, r - gL].  WHOLE: the tile
-// guarantees amax = R - 1 for every lane (see tile_fp32).
-template <int R, bool WHOLE>
+// in row r are (j = r - g, g = gL + a) for a < kR with g < g_hi and j >= 0,
+// gL = gb + L*kR, i.e. the columns [r - gL - amax, r - gL].
 __device__ __forceinline__ void flush_row_group(const Fp32TileParams& P, float v, int64_t r,
                                                 int64_t gb, unsigned ulim_ord) {
     const unsigned bits = __float_as_uint(v);
     const float u = untag_value(bits);
     if (!(u < kInf)) return;  // no cell (kInf or a NaN pattern)
-    const int64_t gL = gb + (int64_t)(bits & kTagMask) * R;
-    const int64_t amax = WHOLE ? (int64_t)R - 1 : min(min((int64_t)R - 1, P.g_hi - 1 - gL), r - gL);
+    const int64_t gL = gb + (int64_t)(bits & kTagMask) * kR;
+    const int64_t amax = min(min((int64_t)kR - 1, P.g_hi - 1 - gL), r - gL);
     merge_group(P.key + r, u, r - gL - amax, (int)amax + 1, ulim_ord);
 }
 // Column j's minimum over the band, tagged with its lane L: the candidates
-// are rows j + gL + a, a < R, on diagonals < g_hi and rows < PL.  WHOLE: the
-// tile guarantees all R of them for every lane.
-template <int R, bool WHOLE>
+// are rows j + gL + a, a < kR, on diagonals < g_hi and rows < PL.
 __device__ __forceinline__ void flush_col_group(const Fp32TileParams& P, unsigned bits, int64_t j,
                                                 int64_t gb, unsigned ulim_ord) {
     const float u = untag_value(bits);
     if (!(u < kInf)) return;
-    const int64_t gL = gb + (int64_t)(bits & kTagMask) * R;
-    const int64_t cnt = WHOLE ? (int64_t)R : min(min((int64_t)R, P.g_hi - gL), P.PL - j - gL);
+    const int64_t gL = gb + (int64_t)(bits & kTagMask) * kR;
+    const int64_t cnt = min(min((int64_t)kR, P.g_hi - gL), P.PL - j - gL);
     merge_group(P.key + j, u, j + gL, (int)cnt, ulim_ord);
 }
 
-template <int R>
 __device__ __forceinline__ void flush_row(const Fp32TileParams& P, float v, int64_t r,
                                           int64_t gb, float ulim) {
     const unsigned bits = __float_as_uint(v);
     const float u = untag_value(bits);
     if (u < ulim) {
         const unsigned t = bits & kTagMask;
-        const int64_t dw = (int64_t)(t >> 3) * R + (t & 7u);
-        const int64_t j = r - (gb + dw);
+        const int64_t j = r - (gb + t);  // lane << 3 | a is the diagonal's place in the band
         atomicMin(P.key + r, ((unsigned long long)ord_f32(u) << 32) | (unsigned long long)j);
     }
+}
+
+// FP64 re-anchor of a tile: minus the covariance at its first column j0 of the
+// lane's diagonals.  The series terms are staged in
+// a (not yet used) shared-memory area with coalesced loads, CHUNK terms at a
+// time: the column's A[j0 + k] and the warp's rows A[j0 + gb + i], i < 32R + chunk,
+// skewed by one double per 8 so that lanes reading rows 8 apart hit distinct
+// banks.  Each lane then sums its R products in k order from shared memory.
+template <int CHUNK>
+__device__ __forceinline__ void anchor_fp32(const Fp32TileParams& P, int64_t j0, int64_t gb, int64_t g0,
+                                            int lane, char* rring, float (&nc)[kR]) {
+    constexpr int R = kR;
+    double mu0 = (double)P.m * __ldg(P.mean + j0);
+    double mr[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) mr[a] = __ldg(P.mean + j0 + g0 + a);
+    double q[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) q[a] = 0.0;
+    {
+        static_assert(R % 8 == 0, "anchor row skew assumes lanes start on multiples of 8 rows");
+        double* scol = reinterpret_cast<double*>(rring);
+        double* srow = scol + CHUNK;
+        const double* Ac = P.A + j0;
+        const double* Ar = P.A + j0 + gb;
+        // lane's rows i = lane*R + t sit at srow[lane*(R + R/8) + t + t/8]
+        const double* wl = srow + lane * (R + R / 8);
+        for (int64_t kb0 = 0; kb0 < P.m; kb0 += CHUNK) {
+            const int kc = (int)min((int64_t)CHUNK, P.m - kb0);
+            __syncwarp();
+#pragma unroll 4
+            for (int i = lane; i < kc; i += 32) scol[i] = __ldg(Ac + kb0 + i);
+#pragma unroll 4
+            for (int i = lane; i < 32 * R + kc; i += 32) srow[i + (i >> 3)] = __ldg(Ar + kb0 + i);
+            __syncwarp();
+            double w[R];
+#pragma unroll
+            for (int a = 0; a < R - 1; ++a) w[a] = wl[a];
+            int k = 0;
+            for (; k + R <= kc; k += R) {
+                const double* wk = wl + (k / 8) * 9;  // row lane*R + k, k % 8 == 0
+#pragma unroll
+                for (int kk = 0; kk < R; ++kk) {
+                    const int t = kk + R - 1;
+                    w[(kk + R - 1) % R] = wk[t + (t >> 3)];
+                    const double x = scol[k + kk];
+#pragma unroll
+                    for (int a = 0; a < R; ++a) q[a] = __fma_rn(x, w[(kk + a) % R], q[a]);
+                }
+            }
+            for (; k < kc; ++k) {
+                const double x = scol[k];
+#pragma unroll
+                for (int a = 0; a < R; ++a) {
+                    const int t = k + a;
+                    q[a] = __fma_rn(x, wl[t + (t >> 3)], q[a]);
+                }
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int a = 0; a < R; ++a) nc[a] = (float)__fma_rn(mu0, mr[a], -q[a]);
+}
+
+// Persistent warps: each takes the next tile number from one global counter until
+// the tile space is exhausted (no waiting on anything).
+template <class F>
+__device__ __forceinline__ void for_each_tile(const Fp32TileParams* series, int nseries, int64_t total,
+                                              unsigned long long* counter, int lane, F tile) {
+    for (;;) {
+        unsigned long long t0 = 0;
+        if (lane == 0) t0 = atomicAdd(counter, 1ull);
+        const int64_t tt = (int64_t)__shfl_sync(kFullMask, t0, 0);
+        if (tt >= total) break;
+        // the series owning tile tt: last descriptor with tile_begin <= tt
+        int lo = 0, hi = nseries - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (series[mid].tile_begin <= tt) lo = mid;
+            else hi = mid - 1;
+        }
+        const Fp32TileParams P = series[lo];
+        // local tile -> band and column segment (band pairs of nearly equal
+        // tile counts); consecutive tiles are consecutive column segments of
+        // one band, so tiles running together touch disjoint columns and rows
+        int64_t band, seg;
+        if (fp32_tile_of(P, tt - P.tile_begin + P.tile_skip, 32 * 8, band, seg))
+            tile(P, band, seg);
+    }
+}
+
+// Terms of the FP64 anchor staged per pass.
+constexpr int kAnchorChunk = 320;
+constexpr int kAnchorBytes = 8 * (kAnchorChunk + (32 * 8 + kAnchorChunk) * 9 / 8);
+static_assert(kAnchorBytes <= kRecRingBytes, "anchor staging fits the record ring");
+
+// ---- every pass with the selection (see fp32_gate_pays) ----------------------
+// A row record in memory: 32 bytes.
+struct RowRec {
+    float4 dfdg;  // (df[j], df[j+4], dg[j], dg[j+4])
+    float4 nn1;   // (nn[j], nn[j+4], 1, 1)
+};
+// The part of a row record a lane keeps in registers (the constant pair stays
+// behind: one shared (1, 1) operand serves every fused distance).
+struct DenseWin {
+    float4 dfdg;
+    float2 nn;
+};
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+static_assert(sizeof(RowRec) == 4 * kRecFloats, "row record is 32 bytes");
+
+// Row-partial ring: 34 chunks of 8 rows, 12 floats apart (48 bytes), so that
+// the 8 lanes of a quarter-warp merging their chunks with 16-byte accesses
+// hit 8 distinct groups of 4 banks (a 32-byte stride would pair them up).
+constexpr int kRowChunks = 34;
+
+// 16-byte copy global -> shared that completes asynchronously (cp.async.cg:
+// cached in L2 only); both addresses 16-byte aligned.
+__device__ __forceinline__ void cp_async16(char* dst_smem, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 
 // One chunk = R consecutive columns.  Per column: R cells per lane, the
@@ -156,7 +273,7 @@ __device__ __forceinline__ void flush_row(const Fp32TileParams& P, float v, int6
 // jr + b < min(lim0 - d, ncols).
 template <int R, bool FAST, int OFF, bool GROUP>
 __device__ __forceinline__ void chunk_fp32(const char* rbase, const char* cbuf,
-                                           RowWin (&win)[R / 2], float2 (&nc2)[R / 2],
+                                           DenseWin (&win)[R / 2], float2 (&nc2)[R / 2],
                                            float (&acc)[2 * R], const unsigned (&tag)[R],
                                            int lim0, int ncols, int ghi_rel, int jr, int lane,
                                            int& colkey) {
@@ -181,7 +298,7 @@ __device__ __forceinline__ void chunk_fp32(const char* rbase, const char* cbuf,
             float cmin;
 #pragma unroll
             for (int a = 0; a < H; ++a) {
-                const RowWin& rv = win[(b + a) % H];
+                const DenseWin& rv = win[(b + a) % H];
                 const float2 nn2 = __fmul2_rn(cnn, rv.nn);
                 const float2 u2 = __ffma2_rn(nc2[a], nn2, one2);
                 nc2[a] = __ffma2_rn(lo2(cv), hi2(rv.dfdg), nc2[a]);
@@ -213,7 +330,7 @@ __device__ __forceinline__ void chunk_fp32(const char* rbase, const char* cbuf,
             float cmin;
 #pragma unroll
             for (int a = 0; a < H; ++a) {
-                const RowWin& rv = win[(c + a) % H];
+                const DenseWin& rv = win[(c + a) % H];
                 const float2 nn2 = __fmul2_rn(cnn, rv.nn);
                 const float2 u2 = __ffma2_rn(nc2[a], nn2, one2);
                 nc2[a] = __ffma2_rn(lo2(cv), hi2(rv.dfdg), nc2[a]);
@@ -248,7 +365,7 @@ __device__ __forceinline__ void chunk_fp32(const char* rbase, const char* cbuf,
 }
 
 template <int R, bool GROUP>
-__device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, int lane, float* ring,
+__device__ void tile_dense(const Fp32TileParams& P, int64_t band, int64_t seg, int lane, float* ring,
                           char* rring, char* cring) {
     constexpr int H = R / 2;
     constexpr int RING = 32 * R;
@@ -262,11 +379,6 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
     if (P.hazard && fp32_tile_hazardous(P, gb, j0, j1, 32 * R)) return;
     const float ulim = (float)(1.0 + 1.0 / (double)P.m);
     const unsigned ulim_ord = ord_f32(ulim);
-    // group keys: every lane's candidate groups hold all R candidates (its
-    // diagonals lie below g_hi, rows below PL, and columns, j0 >= R - 1, at or
-    // above 0)
-    const bool whole = j0 >= R - 1 && gb + 32 * R <= P.g_hi && j1 + gb + 32 * R <= P.PL;
-
     // cell (column j, diagonal g0 + d) is evaluated iff d < ghi_rel and
     // j - j0 < min(lim0 - d, ncols); every cell of a chunk ending at or
     // before minlim exists
@@ -279,69 +391,11 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
 #pragma unroll
     for (int a = 0; a < R; ++a) tag[a] = ((unsigned)lane << 3) | (unsigned)a;
 
-    // ---- FP64 re-anchor: cov(j0, j0+g) for the lane's R diagonals ----------
-    // The series terms are staged in the (not yet used) record ring with
-    // coalesced loads, kAnchorChunk terms at a time: the column's A[j0 + k]
-    // and the warp's rows A[j0 + gb + i], i < 32R + chunk, skewed by one double
-    // per 8 so that lanes reading rows 8 apart hit distinct banks.  Each lane
-    // then sums its R products in k order from shared memory.
-    double mu0 = (double)P.m * __ldg(P.mean + j0);
-    double mr[R];
-#pragma unroll
-    for (int a = 0; a < R; ++a) mr[a] = __ldg(P.mean + j0 + g0 + a);
-    double q[R];
-#pragma unroll
-    for (int a = 0; a < R; ++a) q[a] = 0.0;
-    {
-        static_assert(R % 8 == 0, "anchor row skew assumes lanes start on multiples of 8 rows");
-        double* scol = reinterpret_cast<double*>(rring);
-        double* srow = scol + kAnchorChunk;
-        const double* Ac = P.A + j0;
-        const double* Ar = P.A + j0 + gb;
-        // lane's rows i = lane*R + t sit at srow[lane*(R + R/8) + t + t/8]
-        const double* wl = srow + lane * (R + R / 8);
-        for (int64_t kb0 = 0; kb0 < P.m; kb0 += kAnchorChunk) {
-            const int kc = (int)min((int64_t)kAnchorChunk, P.m - kb0);
-            __syncwarp();
-#pragma unroll 4
-            for (int i = lane; i < kc; i += 32) scol[i] = __ldg(Ac + kb0 + i);
-#pragma unroll 4
-            for (int i = lane; i < 32 * R + kc; i += 32) srow[i + (i >> 3)] = __ldg(Ar + kb0 + i);
-            __syncwarp();
-            double w[R];
-#pragma unroll
-            for (int a = 0; a < R - 1; ++a) w[a] = wl[a];
-            int k = 0;
-            for (; k + R <= kc; k += R) {
-                const double* wk = wl + (k / 8) * 9;  // row lane*R + k, k % 8 == 0
-#pragma unroll
-                for (int kk = 0; kk < R; ++kk) {
-                    const int t = kk + R - 1;
-                    w[(kk + R - 1) % R] = wk[t + (t >> 3)];
-                    const double x = scol[k + kk];
-#pragma unroll
-                    for (int a = 0; a < R; ++a) q[a] = __fma_rn(x, w[(kk + a) % R], q[a]);
-                }
-            }
-            for (; k < kc; ++k) {
-                const double x = scol[k];
-#pragma unroll
-                for (int a = 0; a < R; ++a) {
-                    const int t = k + a;
-                    q[a] = __fma_rn(x, wl[t + (t >> 3)], q[a]);
-                }
-            }
-        }
-        __syncwarp();
-    }
+    float nc[R];
+    anchor_fp32<kAnchorChunk>(P, j0, gb, g0, lane, rring, nc);
     float2 nc2[H];
-    {
-        float nc[R];
 #pragma unroll
-        for (int a = 0; a < R; ++a) nc[a] = (float)__fma_rn(mu0, mr[a], -q[a]);
-#pragma unroll
-        for (int a = 0; a < H; ++a) nc2[a] = make_float2(nc[a], nc[a + H]);
-    }
+    for (int a = 0; a < H; ++a) nc2[a] = make_float2(nc[a], nc[a + H]);
 
     // ---- ring of row partials for this tile -----------------------------------
     for (int k = lane; k < kRowChunks * kRowStride; k += 32) ring[k] = kInf;
@@ -363,7 +417,7 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
         reinterpret_cast<const RowRec*>(P.colrec) + j0);
     *reinterpret_cast<uint4*>(cring + 16 * lane) = __ldg(csrc + lane);
     __syncwarp();
-    RowWin win[H];
+    DenseWin win[H];
 #pragma unroll
     for (int k = 0; k < H - 1; ++k) {
         const char* p = rring + rec_off(rec_slot(lane * R + k));
@@ -444,13 +498,8 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
                 const float v = ring[e];
                 ring[e] = kInf;
                 const int64_t j = j0 + jr + lane, r = j0 + gb + jr + lane;
-                if (whole) {
-                    flush_col_group<R, true>(P, (unsigned)colkey, j, gb, ulim_ord);
-                    flush_row_group<R, true>(P, v, r, gb, ulim_ord);
-                } else {
-                    flush_col_group<R, false>(P, (unsigned)colkey, j, gb, ulim_ord);
-                    flush_row_group<R, false>(P, v, r, gb, ulim_ord);
-                }
+                flush_col_group(P, (unsigned)colkey, j, gb, ulim_ord);
+                flush_row_group(P, v, r, gb, ulim_ord);
             } else {
                 const unsigned bits = (unsigned)colkey;
                 const float u = untag_value(bits);
@@ -465,7 +514,7 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
                 const int e = (c % RK_CHUNKS) * kRowStride + (lane & (R - 1));
                 const float v = ring[e];
                 ring[e] = kInf;
-                flush_row<R>(P, v, j0 + gb + jr + lane, gb, ulim);
+                flush_row(P, v, j0 + gb + jr + lane, gb, ulim);
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -487,67 +536,418 @@ __device__ void tile_fp32(const Fp32TileParams& P, int64_t band, int64_t seg, in
         const int rel = (cs - cend % RK_CHUNKS + RK_CHUNKS) % RK_CHUNKS;
         const int64_t r = j0 + gb + (int64_t)(cend + rel) * R + (e % R);
         if constexpr (GROUP)
-            flush_row_group<R, false>(P, ring[cs * kRowStride + e % R], r, gb, ulim_ord);
+            flush_row_group(P, ring[cs * kRowStride + e % R], r, gb, ulim_ord);
         else
-            flush_row<R>(P, ring[cs * kRowStride + e % R], r, gb, ulim);
+            flush_row(P, ring[cs * kRowStride + e % R], r, gb, ulim);
+    }
+    __syncwarp();
+}
+
+constexpr int kDenseSmem = kRecRingBytes + kRowChunks * kRowStride * (int)sizeof(float) + 4 * 32 * kR;
+static_assert(kDenseSmem % 16 == 0, "warps' areas stay 16-byte aligned");
+
+// ---- passes behind the gate ---------------------------------------------------
+constexpr int kPassCols = 16;    // columns per pass
+constexpr int kGroups = 40;  // ring: groups of 8 rows; a pass reads 34, 2 more arrive
+constexpr int kPad = 9;      // elements between groups: lanes 8 rows apart hit distinct banks
+// The gate asks for nc * nn_r < -sn / nn_j with sn = 1 - bound - kGateSlack, where u
+// = fl(1 + nc * fl(nn_j nn_r)) <= bound is meant: roundings of four values below
+// 1.01 in size near a bound, 2.5e-7 together (5e-7 where nn_j nn_r is subnormal).
+constexpr float kGateSlack = 2e-6f;
+constexpr int kTileSmem = kGroups * kPad * 12 + 2 * kPassCols * 16 +
+                          2 * kGroups * kRowStride * 4 + 2 * kPassCols * 4 + kGroups * 4;
+static_assert(kTileSmem % 16 == 0, "warps' areas stay 16-byte aligned");
+static_assert(kAnchorBytes <= kTileSmem, "anchor staging fits");
+__device__ __forceinline__ int wrap_group(int s) { return s < kGroups ? s : s - kGroups; }
+
+// High word of a key as it stands (merged meanwhile by other warps).
+__device__ __forceinline__ unsigned ld_key_hi(const unsigned long long* key) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
+                 : "=r"(v)
+                 : "l"(reinterpret_cast<const unsigned*>(key) + 1));
+    return v;
+}
+// Where a row starts: just above every tagged distance that could tie the key
+// (2^-15 steps), 0 for a key below 0 (every negative distance goes on).
+__device__ __forceinline__ unsigned key_bound(unsigned hi) {
+    return (hi & 0x80000000u) ? (hi & 0x7fffff00u) + 0x100u : 0u;
+}
+
+// The warp's shared memory for a tile.
+struct TileSmem {
+    float2* dd;      // row terms df, dg, kPad per group
+    float* nn;       // ... and nn
+    float4* col;     // column terms -df, -dg, nn, 1 / nn, two buffers of kPassCols
+    float* best;     // best tagged distance per row, kRowStride per group
+    float* start;    // what it started from
+    unsigned* cthr;  // column bounds (bit patterns), two buffers of kPassCols
+    unsigned* gate;  // per group: the loosest of its rows' bests (bit pattern)
+    __device__ __forceinline__ explicit TileSmem(char* p) {
+        col = reinterpret_cast<float4*>(p);
+        best = reinterpret_cast<float*>(col + 2 * kPassCols);
+        start = best + kGroups * kRowStride;
+        dd = reinterpret_cast<float2*>(start + kGroups * kRowStride);
+        nn = reinterpret_cast<float*>(dd + kGroups * kPad);
+        cthr = reinterpret_cast<unsigned*>(nn + kGroups * kPad);
+        gate = cthr + 2 * kPassCols;
+    }
+    // Copies the terms of 16 rows (two groups from slot s) from pair records.
+    __device__ __forceinline__ void stage_rows(int s, const float* src, int lane) const {
+        const int e = (s + ((lane & 15) >> 3)) * kPad + (lane & 7);
+        const float* r = src + kRecFloats * (lane & 15);
+        cp_async4(reinterpret_cast<float*>(dd + e) + (lane >> 4), r + 2 * (lane >> 4));
+        if (lane < 16) cp_async4(nn + e, r + 4);
+    }
+    // ... and of kPassCols columns into buffer b
+    __device__ __forceinline__ void stage_cols(int b, const float* src, int lane) const {
+        float* d = reinterpret_cast<float*>(col + b * kPassCols);
+        const float* r = src + kRecFloats * (lane >> 1) + 4 * (lane & 1);
+        cp_async4(d + 4 * (lane >> 1) + 2 * (lane & 1), r);
+        cp_async4(d + 4 * (lane >> 1) + 2 * (lane & 1) + 1, r + 2);
+    }
+    __device__ __forceinline__ unsigned group_gate(int s) const {
+        const float4 a = *reinterpret_cast<const float4*>(best + s * kRowStride);
+        const float4 b = *reinterpret_cast<const float4*>(best + s * kRowStride + 4);
+        const float m = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)),
+                              fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+        return __float_as_uint(fmaxf(m, 0.f));
+    }
+};
+
+// A lane's window of 8 rows.
+struct RowWin {
+    float df[8], dg[8], nn[8];
+    __device__ __forceinline__ void load(const TileSmem& sm, int s) {
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            const float2 x = sm.dd[s * kPad + a];
+            df[a] = x.x;
+            dg[a] = x.y;
+            nn[a] = sm.nn[s * kPad + a];
+        }
+    }
+};
+
+__device__ __forceinline__ unsigned gate_pass(const TileSmem& sm, int s1, int s2, const float4* col,
+                                           float sn, RowWin& win, float (&nc)[8]) {
+    const float2 *d1 = sm.dd + s1 * kPad, *d2 = sm.dd + s2 * kPad;
+    const float *n1 = sm.nn + s1 * kPad, *n2 = sm.nn + s2 * kPad;
+    unsigned t = 0;
+#pragma unroll
+    for (int b = 0; b < kPassCols; ++b) {
+        const float4 cv = col[b];
+        const float c = sn * cv.w;
+        float v[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) v[a] = __fmaf_rn(nc[a], win.nn[(b + a) % 8], c);
+#pragma unroll
+        for (int a = 0; a < 8; ++a) nc[a] = __fmaf_rn(cv.x, win.dg[(b + a) % 8], nc[a]);
+#pragma unroll
+        for (int a = 0; a < 8; ++a) nc[a] = __fmaf_rn(cv.y, win.df[(b + a) % 8], nc[a]);
+        {  // row b gives way to row b + 8
+            const float2 x = b < 8 ? d1[b] : d2[b - 8];
+            win.df[b % 8] = x.x;
+            win.dg[b % 8] = x.y;
+            win.nn[b % 8] = b < 8 ? n1[b] : n2[b - 8];
+        }
+#pragma unroll
+        for (int a = 0; a < 8; a += 2) t |= __float_as_uint(v[a]) | __float_as_uint(v[a + 1]);
+    }
+    return t;
+}
+
+// One pass with the selection.  Columns go in pairs: row element e takes cell
+// e - b of column b and cell e - b - 1 of column b + 1, so one 3-input minimum per
+// element serves both; a column's minimum over the warp is one REDUX, kept by lane
+// b in colkey.  Elements 8g .. 8g + 7 go to the lane's group g as soon as they are
+// complete.  EDGE: cell (column jr + b, diagonal g0 + d) exists iff d < ghi_rel and
+// jr + b < min(lim0 - d, ncols).  Window as in gate_pass.  Returns whether a row's
+// best fell.
+template <bool EDGE, bool GROUP>
+__device__ __forceinline__ bool dense_pass(const TileSmem& sm, int s0, int s1, int s2,
+                                           const float4* col, RowWin& win, float (&nc)[8], int lim0,
+                                           int ncols, int ghi_rel, int jr, int lane, int& colkey) {
+    const float2 *d1 = sm.dd + s1 * kPad, *d2 = sm.dd + s2 * kPad;
+    const float *n1 = sm.nn + s1 * kPad, *n2 = sm.nn + s2 * kPad;
+    float acc[8 + kPassCols];
+    unsigned fell = 0;
+    auto merge = [&](int g) {  // elements 8g .. 8g + 7
+        __syncwarp();  // lane l's group g + 1 is lane l + 1's group g
+        float4* e = reinterpret_cast<float4*>(sm.best + (g == 0 ? s0 : g == 1 ? s1 : s2) * kRowStride);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 o = e[h];
+            float4 v;
+            const float* k = acc + 8 * g + 4 * h;
+            v.x = fminf(o.x, lane_min<GROUP>(k[0], lane));
+            v.y = fminf(o.y, lane_min<GROUP>(k[1], lane));
+            v.z = fminf(o.z, lane_min<GROUP>(k[2], lane));
+            v.w = fminf(o.w, lane_min<GROUP>(k[3], lane));
+            e[h] = v;
+            fell |= __float_as_uint(v.x) ^ __float_as_uint(o.x);
+            fell |= __float_as_uint(v.y) ^ __float_as_uint(o.y);
+            fell |= __float_as_uint(v.z) ^ __float_as_uint(o.z);
+            fell |= __float_as_uint(v.w) ^ __float_as_uint(o.w);
+        }
+    };
+#pragma unroll
+    for (int b = 0; b < kPassCols; b += 2) {
+        float kb[8];  // column b's cells
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = b + h;
+            const float4 cv = col[c];
+            float kc[8], cmin = kInf;
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                const int w = (c + d) % 8;
+                const float u = __fmaf_rn(nc[d], __fmul_rn(cv.z, win.nn[w]), 1.f);
+                nc[d] = __fmaf_rn(cv.x, win.dg[w], nc[d]);
+                nc[d] = __fmaf_rn(win.df[w], cv.y, nc[d]);
+                kc[d] = GROUP ? u : tag_key(u, ((unsigned)lane << 3) | (unsigned)d);
+                if (EDGE) {
+                    const int l = d < ghi_rel ? min(lim0 - d, ncols) : 0;
+                    if (jr + c >= l) kc[d] = kInf;
+                }
+                if (d % 2) cmin = d == 1 ? fminf(kc[0], kc[1]) : fmin3(cmin, kc[d - 1], kc[d]);
+            }
+            {  // row c gives way to row c + 8
+                const float2 x = c < 8 ? d1[c] : d2[c - 8];
+                win.df[c % 8] = x.x;
+                win.dg[c % 8] = x.y;
+                win.nn[c % 8] = c < 8 ? n1[c] : n2[c - 8];
+            }
+            const int kmin =
+                __reduce_min_sync(kFullMask, __float_as_int(GROUP ? tag_lane(cmin, lane) : cmin));
+            colkey = lane == c ? kmin : colkey;
+            if (h == 0) {
+#pragma unroll
+                for (int d = 0; d < 8; ++d) kb[d] = kc[d];
+                continue;
+            }
+            acc[b] = b == 0 ? kb[0] : fminf(acc[b], kb[0]);
+#pragma unroll
+            for (int d = 0; d < 7; ++d) {
+                const int e = b + 1 + d;  // first met by column b when b == 0 or d == 6
+                acc[e] = b == 0 || d == 6 ? fminf(kb[d + 1], kc[d]) : fmin3(acc[e], kb[d + 1], kc[d]);
+            }
+            acc[b + 8] = kc[7];
+        }
+        if (b == 6) merge(0);
+        if (b == 14) merge(1);
+    }
+    acc[8 + kPassCols - 1] = kInf;  // no cell
+    merge(2);
+    return __any_sync(kFullMask, fell != 0);
+}
+
+template <bool GROUP>
+__device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, int lane,
+                          const TileSmem& sm) {
+    constexpr int R = kR;
+    const int64_t gb = P.g_lo + band * (int64_t)(32 * R);
+    const int64_t g0 = gb + (int64_t)lane * R;
+    const int64_t jmax = P.PL - gb;
+    const int64_t j0 = seg * P.K;
+    const int64_t j1 = min(j0 + P.K, jmax);
+    if (j0 >= j1) return;
+    // guarded form: tiles touching a hazard window are evaluated in FP64
+    if (P.hazard && fp32_tile_hazardous(P, gb, j0, j1, 32 * R)) return;
+    const float ulim = (float)(1.0 + 1.0 / (double)P.m);
+    const unsigned ulim_ord = ord_f32(ulim);
+    // extents of the tile's cells, as in tile_fp32
+    const int ncols = (int)(j1 - j0);
+    const int lim0 = (int)min(P.PL - g0 - j0, (int64_t)ncols + R);
+    const int ghi_rel = (int)max(min(P.g_hi - g0, (int64_t)R), (int64_t)0);
+    const int minlim = __reduce_min_sync(kFullMask, ghi_rel < R ? 0 : min(lim0 - (R - 1), ncols));
+
+    float nc[R];
+    anchor_fp32<kAnchorChunk>(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), nc);
+
+    // groups 0 .. 33 and the first pass's columns; from here on lanes 0 - 15 look
+    // after rows, lanes 16 - 31 after columns
+    const int64_t rb = j0 + gb;  // row of element 0 of group 0
+    const float* nrow = reinterpret_cast<const float*>(P.rowrec) + rb * kRecFloats;
+    const float* ncol = reinterpret_cast<const float*>(P.colrec) + j0 * kRecFloats;
+    for (int i = 0; i < 17; ++i) sm.stage_rows(2 * i, nrow + 16 * kRecFloats * i, lane);
+    sm.stage_cols(0, ncol, lane);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int i = lane; i < 34 * R; i += 32) {
+        const unsigned f = rb + i < P.PL ? key_bound(ld_key_hi(P.key + rb + i)) : 0u;
+        const int e = (i / R) * kRowStride + i % R;
+        sm.best[e] = __uint_as_float(f);
+        sm.start[e] = __uint_as_float(f);
+    }
+    unsigned cgate = 0;
+    if (lane < kPassCols) {
+        cgate = j0 + lane < P.PL ? key_bound(ld_key_hi(P.key + j0 + lane)) : 0u;
+        sm.cthr[lane] = cgate | kTagMask;
+    }
+    cgate = __reduce_max_sync(kFullMask, cgate);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+    sm.gate[lane] = sm.group_gate(lane);
+    if (lane < 2) sm.gate[32 + lane] = sm.group_gate(32 + lane);
+    __syncwarp();
+    RowWin win;
+    win.load(sm, lane);
+
+    const int64_t inc0 = lane < 16 ? rb + 34 * R + lane : j0 + lane;  // - 16 + kPassCols
+    int s0 = lane;  // slot of the lane's first group
+    int sf = 0;     // slot of the first group that the pass finishes
+    int cb = 0;
+    bool sel = false;
+    int skip = 0, streak = 0;
+    int jr = 0;
+    for (; jr < ncols; jr += kPassCols) {
+        // what the next pass appends: 16 rows, 16 columns and their keys
+        const int sn = wrap_group(sf + 34);
+        sm.stage_rows(sn, nrow + (34 * R + jr) * kRecFloats, lane);
+        sm.stage_cols(cb ^ 1, ncol + (jr + kPassCols) * kRecFloats, lane);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const int64_t inc = inc0 + jr;
+        unsigned f = 0;
+        if (inc < P.PL) f = ld_key_hi(P.key + inc);
+
+        const int s1 = wrap_group(s0 + 1), s2 = wrap_group(s0 + 2);
+        const float bound =
+            __uint_as_float(max(max(sm.gate[s0], sm.gate[s1]), max(sm.gate[s2], cgate)) | kTagMask);
+        const float4* col = sm.col + cb * kPassCols;
+        const unsigned* cthr = sm.cthr + cb * kPassCols;
+        const bool inside = jr + kPassCols <= minlim;
+        // A pass after one that lowered something goes straight on; so do the next
+        // 1, 2, 4 .. 16 passes after gates that opened in a row, where a gate in
+        // every pass would only add to the selection.
+        bool open = !inside || sel || skip > 0;
+        skip -= skip > 0;
+        const bool again = !open;
+        if (!open) {
+            float q0[8];
+#pragma unroll
+            for (int a = 0; a < 8; ++a) q0[a] = nc[a];
+            const float sn = (1.f - bound) - kGateSlack;
+            const unsigned t = gate_pass(sm, s1, s2, col, sn, win, nc);
+            open = __any_sync(kFullMask, (int)t < 0 || sn <= 0.f);
+            streak = open ? min(max(2 * streak, 1), 16) : 0;
+            skip = streak;
+            if (open) {
+#pragma unroll
+                for (int a = 0; a < 8; ++a) nc[a] = q0[a];
+            }
+        }
+        sel = false;
+        if (open) {
+            if (again) win.load(sm, s0);
+            int colkey = 0x7fffffff;
+            sel = inside ? dense_pass<false, GROUP>(sm, s0, s1, s2, col, win, nc, lim0, ncols, ghi_rel, jr,
+                                                    lane, colkey)
+                         : dense_pass<true, GROUP>(sm, s0, s1, s2, col, win, nc, lim0, ncols, ghi_rel, jr,
+                                                   lane, colkey);
+            // columns jr + lane at or below their keys
+            bool low = false;
+            if (lane < kPassCols) {
+                const float v = untag_value((unsigned)colkey);
+                low = v <= __uint_as_float(cthr[lane]);
+                const int64_t j = j0 + jr + lane;
+                if (low) {
+                    if constexpr (GROUP) {
+                        flush_col_group(P, (unsigned)colkey, j, gb, ulim_ord);
+                    } else if (v < ulim) {
+                        atomicMin(P.key + j, ((unsigned long long)ord_f32(v) << 32) |
+                                                 (unsigned long long)(j + gb + ((unsigned)colkey & kTagMask)));
+                    }
+                }
+            }
+            sel |= __any_sync(kFullMask, low);
+        }
+        __syncwarp();
+        // the pass's first two groups have met every lane: merge the rows that fell
+        f = inc < P.PL ? key_bound(f) : 0u;
+        if (lane < 16) {
+            const int e = (sf + (lane >> 3)) * kRowStride + (lane & 7);
+            const float v = sm.best[e];
+            if (v < sm.start[e]) {
+                if constexpr (GROUP)
+                    flush_row_group(P, v, rb + jr + lane, gb, ulim_ord);
+                else
+                    flush_row(P, v, rb + jr + lane, gb, ulim);
+            }
+            const int en = (sn + (lane >> 3)) * kRowStride + (lane & 7);
+            sm.best[en] = __uint_as_float(f);
+            sm.start[en] = __uint_as_float(f);
+        } else {
+            sm.cthr[(cb ^ 1) * kPassCols + lane - 16] = f | kTagMask;
+        }
+        const unsigned g0v = __reduce_max_sync(kFullMask, lane < 8 ? f : 0u);
+        const unsigned g1v = __reduce_max_sync(kFullMask, (lane & 24) == 8 ? f : 0u);
+        cgate = __reduce_max_sync(kFullMask, lane >= 16 ? f : 0u);
+        if (lane == 0) {
+            sm.gate[sn] = g0v;
+            sm.gate[sn + 1] = g1v;
+        }
+        s0 = s2;
+        if (sel) sm.gate[s0] = sm.group_gate(s0);  // bests of the groups still alive fell
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncwarp();
+        sf = wrap_group(sf + 2);
+        cb ^= 1;
+    }
+
+    // drain: rows of the next 32 groups
+    for (int i = lane; i < 32 * R; i += 32) {
+        const int e = wrap_group(sf + i / R) * kRowStride + i % R;
+        const float v = sm.best[e];
+        if (v < sm.start[e]) {
+            if constexpr (GROUP)
+                flush_row_group(P, v, rb + jr + i, gb, ulim_ord);
+            else
+                flush_row(P, v, rb + jr + i, gb, ulim);
+        }
     }
     __syncwarp();
 }
 
 constexpr int kFp32WarpsPerBlock = 4;
-
-constexpr int kRowKeySlots = kRowChunks * kRowStride;
-template <int R>
-constexpr int fp32_smem_bytes() {
-    return kFp32WarpsPerBlock * (kRecRingBytes + kRowKeySlots * (int)sizeof(float) + 4 * 32 * R);
-}
-
-#ifndef MPGPU_FP32_MIN_BLOCKS
-#define MPGPU_FP32_MIN_BLOCKS 3  // 3 x 4 warps per SM (measured best of 2, 3, 4)
-#endif
-
-// CTAs per SM: group keys need fewer registers (no per-cell tags), and at 4
-// CTAs (128 registers) that instantiation ran faster than at 3 (c2 guarded
-// join 175 ms against 178); the tagged one spills more there and ran slower.
-template <bool GROUP>
+// CTAs per SM: the gate's registers allow 4 (n = 1,048,576: 127 ms against 134 at
+// 3), the dense way's 3 (178 ms against 185), except with group keys, which need
+// no per-cell tags.
+template <Fp32Way WAY, bool GROUP>
 constexpr int fp32_blocks_per_sm() {
-    return GROUP ? 4 : MPGPU_FP32_MIN_BLOCKS;
+    return WAY == kFp32Gate || (WAY == kFp32Dense && GROUP) ? 4 : 3;
 }
+template <Fp32Way WAY>
+struct Fp32Smem {
+    static constexpr int kPerWarp =
+        WAY == kFp32Gate ? kTileSmem : (kDenseSmem > kTileSmem ? kDenseSmem : kTileSmem);
+    static constexpr int kPerBlock = kFp32WarpsPerBlock * kPerWarp;
+};
 
-template <int R, bool GROUP>
-__global__ void __launch_bounds__(32 * kFp32WarpsPerBlock, fp32_blocks_per_sm<GROUP>())
+template <Fp32Way WAY, bool GROUP>
+__global__ void __launch_bounds__(32 * kFp32WarpsPerBlock, fp32_blocks_per_sm<WAY, GROUP>())
     fp32_join_kernel(const Fp32TileParams* __restrict__ series, int nseries, int64_t total,
                      unsigned long long* __restrict__ counter) {
     extern __shared__ __align__(128) char smem_fp32[];
     const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    char* rring = smem_fp32 + w * kRecRingBytes;
-    float* ring = reinterpret_cast<float*>(smem_fp32 + kFp32WarpsPerBlock * kRecRingBytes) +
-                  w * kRowKeySlots;
-    char* cring = smem_fp32 + kFp32WarpsPerBlock * (kRecRingBytes + kRowKeySlots * (int)sizeof(float)) +
-                  w * 4 * 32 * R;
-    // Persistent warps: each takes the next tile number from one global
-    // counter until the tile space is exhausted (no waiting on anything).
-    for (;;) {
-        unsigned long long t0 = 0;
-        if (lane == 0) t0 = atomicAdd(counter, 1ull);
-        const int64_t tt = (int64_t)__shfl_sync(kFullMask, t0, 0);
-        if (tt >= total) break;
-        // the series owning tile tt: last descriptor with tile_begin <= tt
-        int lo = 0, hi = nseries - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (series[mid].tile_begin <= tt) lo = mid;
-            else hi = mid - 1;
-        }
-        const Fp32TileParams P = series[lo];
-        // local tile -> band and column segment (band pairs of nearly equal
-        // tile counts); consecutive tiles are consecutive column segments of
-        // one band, so tiles running together touch disjoint columns and rows
-        int64_t band, seg;
-        if (fp32_tile_of(P, tt - P.tile_begin + P.tile_skip, 32 * R, band, seg))
-            tile_fp32<R, GROUP>(P, band, seg, lane, ring, rring, cring);
-    }
+    char* mine = smem_fp32 + (threadIdx.x >> 5) * Fp32Smem<WAY>::kPerWarp;
+    for_each_tile(series, nseries, total, counter, lane,
+                  [&](const Fp32TileParams& P, int64_t band, int64_t seg) {
+                      if (WAY == kFp32Gate || (WAY == kFp32Mixed && fp32_gate_pays(P.m, P.PL)))
+                          tile_gate<GROUP>(P, band, seg, lane, TileSmem(mine));
+                      else
+                          tile_dense<kR, GROUP>(P, band, seg, lane, reinterpret_cast<float*>(mine + kRecRingBytes),
+                                                mine, mine + kRecRingBytes + kRowChunks * kRowStride * 4);
+                  });
+}
+
+template <Fp32Way WAY, bool GROUP>
+void launch_way(const Fp32TileParams* series, int nseries, int64_t total, unsigned long long* counter,
+                cudaStream_t s) {
+    const int64_t want = (total + kFp32WarpsPerBlock - 1) / kFp32WarpsPerBlock;
+    const int64_t blocks = std::min<int64_t>(want, (int64_t)sm_count() * fp32_blocks_per_sm<WAY, GROUP>());
+    if (blocks > 0)
+        fp32_join_kernel<WAY, GROUP><<<(unsigned)blocks, 32 * kFp32WarpsPerBlock, Fp32Smem<WAY>::kPerBlock, s>>>(
+            series, nseries, total, counter);
 }
 
 }  // namespace
@@ -571,15 +971,18 @@ void fp32_tile_plan(int64_t PL, int64_t g_lo, int64_t g_hi, int64_t K, int R, in
 
 template <int R>
 void configure_fp32_join() {
-    cudaFuncSetAttribute(fp32_join_kernel<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         fp32_smem_bytes<R>());
-    cudaFuncSetAttribute(fp32_join_kernel<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         fp32_smem_bytes<R>());
+    static_assert(R == kR, "the tile kernel is laid out for 8 diagonals per lane");
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaFuncSetAttribute(fp32_join_kernel<kFp32Dense, false>, attr, Fp32Smem<kFp32Dense>::kPerBlock);
+    cudaFuncSetAttribute(fp32_join_kernel<kFp32Dense, true>, attr, Fp32Smem<kFp32Dense>::kPerBlock);
+    cudaFuncSetAttribute(fp32_join_kernel<kFp32Gate, false>, attr, Fp32Smem<kFp32Gate>::kPerBlock);
+    cudaFuncSetAttribute(fp32_join_kernel<kFp32Gate, true>, attr, Fp32Smem<kFp32Gate>::kPerBlock);
+    cudaFuncSetAttribute(fp32_join_kernel<kFp32Mixed, false>, attr, Fp32Smem<kFp32Mixed>::kPerBlock);
 }
 
 template <int R>
 void launch_fp32_join(const Fp32TileParams* series_dev, int nseries, int64_t total,
-                      unsigned long long* counter, cudaStream_t s, bool group) {
+                      unsigned long long* counter, cudaStream_t s, Fp32Way way, bool group) {
     // the shared-memory limit is a per-device attribute; setting it is
     // idempotent, so concurrent first launches (server threads) are harmless
     static std::atomic<unsigned long long> configured{0};
@@ -590,19 +993,18 @@ void launch_fp32_join(const Fp32TileParams* series_dev, int nseries, int64_t tot
         configure_fp32_join<R>();
         configured.fetch_or(bit, std::memory_order_release);
     }
-    const int64_t want = (total + kFp32WarpsPerBlock - 1) / kFp32WarpsPerBlock;
-    const int64_t blocks = std::min<int64_t>(
-        want, (int64_t)sm_count() * (group ? fp32_blocks_per_sm<true>() : fp32_blocks_per_sm<false>()));
-    if (blocks > 0 && group)
-        fp32_join_kernel<R, true><<<(unsigned)blocks, 32 * kFp32WarpsPerBlock, fp32_smem_bytes<R>(), s>>>(
-            series_dev, nseries, total, counter);
-    else if (blocks > 0)
-        fp32_join_kernel<R, false><<<(unsigned)blocks, 32 * kFp32WarpsPerBlock, fp32_smem_bytes<R>(),
-                                     s>>>(series_dev, nseries, total, counter);
+    if (way == kFp32Mixed)
+        launch_way<kFp32Mixed, false>(series_dev, nseries, total, counter, s);
+    else if (way == kFp32Gate)
+        group ? launch_way<kFp32Gate, true>(series_dev, nseries, total, counter, s)
+              : launch_way<kFp32Gate, false>(series_dev, nseries, total, counter, s);
+    else
+        group ? launch_way<kFp32Dense, true>(series_dev, nseries, total, counter, s)
+              : launch_way<kFp32Dense, false>(series_dev, nseries, total, counter, s);
 }
 
 template void launch_fp32_join<8>(const Fp32TileParams*, int, int64_t, unsigned long long*,
-                                  cudaStream_t, bool);
+                                  cudaStream_t, Fp32Way, bool);
 template void configure_fp32_join<8>();
 
 }  // namespace mpgpu

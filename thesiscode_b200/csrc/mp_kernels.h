@@ -266,10 +266,31 @@ __host__ __device__ inline int64_t fp32_pick_neighbour(const double* A, const do
 // Persistent launch over `nseries` descriptors (device array) holding `total`
 // tiles; warps take tiles from *counter (zeroed by the caller beforehand).
 // group: the keys name candidate groups (see kFp32GroupBit) instead of
-// neighbours, which the finalisation resolves in FP64.
+// neighbours, which the finalisation resolves in FP64 (not with kFp32Mixed).
+enum Fp32Way { kFp32Dense, kFp32Gate, kFp32Mixed };
 template <int R>
 void launch_fp32_join(const Fp32TileParams* series_dev, int nseries, int64_t total,
-                      unsigned long long* counter, cudaStream_t s, bool group = false);
+                      unsigned long long* counter, cudaStream_t s, Fp32Way way, bool group = false);
+// Whether a join's passes go behind the gate (mp_join_fp32.cu) or all select.  A
+// row's minimum falls about as often as a record in a random sequence, log of the
+// candidates, each time over a run of lags that grows shorter with the window; the
+// gate opens for the loosest of 24 rows and 16 columns, which lie further apart
+// with short windows.  Random walks, K = 1024, gate / every pass selecting (ms):
+//   m = 64    n = 500,000 50.2 / 39.0
+//   m = 128   262,144 11.1 / 10.9     500,000 37.8 / 39.5
+//   m = 192   65,536 0.81 / 0.75      131,072 2.71 / 2.83     500,000 32.5 / 40.1
+//   m = 256   65,536 0.77 / 0.76      131,072 2.53 / 2.86     500,000 30.8 / 40.5
+//   m = 400   32,768 0.28 / 0.28      65,536 0.75 / 0.79      500,000 31.0 / 41.9
+//   m = 1024  16,384 0.16 / 0.12      32,768 0.27 / 0.30      500,000 35.8 / 47.4
+__host__ __device__ inline bool fp32_gate_pays(int64_t m, int64_t PL) {
+    return (m >= 160 && m * PL >= 25000000) || (m >= 128 && PL >= 400000);
+}
+// The way of a launch over these series.
+inline Fp32Way fp32_way_of(const Fp32TileParams* P, size_t n) {
+    size_t gate = 0;
+    for (size_t i = 0; i < n; ++i) gate += fp32_gate_pays(P[i].m, P[i].PL);
+    return gate == 0 ? kFp32Dense : gate == n ? kFp32Gate : kFp32Mixed;
+}
 template <int R>
 void configure_fp32_join();
 // Guarded form (mp_guard.cu): hazard windows and the FP64 pass over their tiles.

@@ -205,7 +205,7 @@ extern "C" int mp_selfjoin_fp32_noalloc(const double* A_dev, int64_t n, int64_t 
         P.key = key;
         noalloc_desc_kernel<<<1, 1, 0, st>>>(desc, P);
         cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
-        launch_fp32_join<kR>(desc, 1, ntiles, counter, st);
+        launch_fp32_join<kR>(desc, 1, ntiles, counter, st, fp32_way_of(&P, 1));
     }
     finalize_fp32_kernel<<<grid_for(PL), kThreads, 0, st>>>(key, PL, (double)m, Apad, mean, norm, 0,
                                                             dist2_dev, idx_dev);

@@ -77,7 +77,8 @@ __device__ __forceinline__ void pack_fp32_record(const double* A, int64_t m, int
     rowrec[2 * j] = make_float4(df0, df1, dg0, dg1);
     rowrec[2 * j + 1] = make_float4(nn0, nn1, 1.f, 1.f);
     colrec[2 * j] = make_float4(-df0, -df0, -dg0, -dg0);
-    colrec[2 * j + 1] = make_float4(nn0, nn0, 0.f, 0.f);
+    const float inv = 1.f / nn0;
+    colrec[2 * j + 1] = make_float4(nn0, nn0, inv, inv);
 }
 
 }  // namespace mpgpu

@@ -153,7 +153,7 @@ int64_t serve_launch_epoch(ServeEpochBuffers& b, int ring_slot, const std::vecto
         cudaMemsetAsync(b.counter, 0, sizeof(unsigned long long), st) != cudaSuccess)
         return -1;
     launch_fp32_join<kR>(static_cast<const Fp32TileParams*>(b.desc_dev[ring_slot]),
-                         (int)slices.size(), total, b.counter, st);
+                         (int)slices.size(), total, b.counter, st, fp32_way_of(h, slices.size()));
     return cudaGetLastError() == cudaSuccess ? total : -1;
 }
 
