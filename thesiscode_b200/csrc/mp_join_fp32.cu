@@ -57,6 +57,7 @@
 
 #include "mp_common.cuh"
 #include "mp_kernels.h"
+#include "mp_tile.cuh"
 
 namespace mpgpu {
 
@@ -65,7 +66,7 @@ namespace {
 // A row or column record in global memory: (x[j], x[j+4]) pairs of df, dg, nn for
 // rows, (-df, -df, -dg, -dg, nn, nn, 1/nn, 1/nn) for columns.
 constexpr int kRecFloats = 8;
-constexpr int kR = 8;  // diagonals per lane: 8 row terms per column, tags of 3 + 5 bits
+constexpr int kR = kTileR;  // 8: tags of 3 + 5 bits
 
 constexpr unsigned kTagMask = 0xffu;
 constexpr float kInf = __builtin_huge_valf();
@@ -136,96 +137,6 @@ __device__ __forceinline__ void flush_row(const Fp32TileParams& P, float v, int6
         const unsigned t = bits & kTagMask;
         const int64_t j = r - (gb + t);  // lane << 3 | a is the diagonal's place in the band
         atomicMin(P.key + r, ((unsigned long long)ord_f32(u) << 32) | (unsigned long long)j);
-    }
-}
-
-// FP64 re-anchor of a tile: minus the covariance at its first column j0 of the
-// lane's diagonals.  The series terms are staged in
-// a (not yet used) shared-memory area with coalesced loads, CHUNK terms at a
-// time: the column's A[j0 + k] and the warp's rows A[j0 + gb + i], i < 32R + chunk,
-// skewed by one double per 8 so that lanes reading rows 8 apart hit distinct
-// banks.  Each lane then sums its R products in k order from shared memory.
-template <int CHUNK>
-__device__ __forceinline__ void anchor_fp32(const Fp32TileParams& P, int64_t j0, int64_t gb, int64_t g0,
-                                            int lane, char* rring, float (&nc)[kR]) {
-    constexpr int R = kR;
-    double mu0 = (double)P.m * __ldg(P.mean + j0);
-    double mr[R];
-#pragma unroll
-    for (int a = 0; a < R; ++a) mr[a] = __ldg(P.mean + j0 + g0 + a);
-    double q[R];
-#pragma unroll
-    for (int a = 0; a < R; ++a) q[a] = 0.0;
-    {
-        static_assert(R % 8 == 0, "anchor row skew assumes lanes start on multiples of 8 rows");
-        double* scol = reinterpret_cast<double*>(rring);
-        double* srow = scol + CHUNK;
-        const double* Ac = P.A + j0;
-        const double* Ar = P.A + j0 + gb;
-        // lane's rows i = lane*R + t sit at srow[lane*(R + R/8) + t + t/8]
-        const double* wl = srow + lane * (R + R / 8);
-        for (int64_t kb0 = 0; kb0 < P.m; kb0 += CHUNK) {
-            const int kc = (int)min((int64_t)CHUNK, P.m - kb0);
-            __syncwarp();
-#pragma unroll 4
-            for (int i = lane; i < kc; i += 32) scol[i] = __ldg(Ac + kb0 + i);
-#pragma unroll 4
-            for (int i = lane; i < 32 * R + kc; i += 32) srow[i + (i >> 3)] = __ldg(Ar + kb0 + i);
-            __syncwarp();
-            double w[R];
-#pragma unroll
-            for (int a = 0; a < R - 1; ++a) w[a] = wl[a];
-            int k = 0;
-            for (; k + R <= kc; k += R) {
-                const double* wk = wl + (k / 8) * 9;  // row lane*R + k, k % 8 == 0
-#pragma unroll
-                for (int kk = 0; kk < R; ++kk) {
-                    const int t = kk + R - 1;
-                    w[(kk + R - 1) % R] = wk[t + (t >> 3)];
-                    const double x = scol[k + kk];
-#pragma unroll
-                    for (int a = 0; a < R; ++a) q[a] = __fma_rn(x, w[(kk + a) % R], q[a]);
-                }
-            }
-            for (; k < kc; ++k) {
-                const double x = scol[k];
-#pragma unroll
-                for (int a = 0; a < R; ++a) {
-                    const int t = k + a;
-                    q[a] = __fma_rn(x, wl[t + (t >> 3)], q[a]);
-                }
-            }
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int a = 0; a < R; ++a) nc[a] = (float)__fma_rn(mu0, mr[a], -q[a]);
-}
-
-// Persistent warps: each takes the next tile number from one global counter until
-// the tile space is exhausted (no waiting on anything).
-template <class F>
-__device__ __forceinline__ void for_each_tile(const Fp32TileParams* series, int nseries, int64_t total,
-                                              unsigned long long* counter, int lane, F tile) {
-    for (;;) {
-        unsigned long long t0 = 0;
-        if (lane == 0) t0 = atomicAdd(counter, 1ull);
-        const int64_t tt = (int64_t)__shfl_sync(kFullMask, t0, 0);
-        if (tt >= total) break;
-        // the series owning tile tt: last descriptor with tile_begin <= tt
-        int lo = 0, hi = nseries - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (series[mid].tile_begin <= tt) lo = mid;
-            else hi = mid - 1;
-        }
-        const Fp32TileParams P = series[lo];
-        // local tile -> band and column segment (band pairs of nearly equal
-        // tile counts); consecutive tiles are consecutive column segments of
-        // one band, so tiles running together touch disjoint columns and rows
-        int64_t band, seg;
-        if (fp32_tile_of(P, tt - P.tile_begin + P.tile_skip, 32 * 8, band, seg))
-            tile(P, band, seg);
     }
 }
 
@@ -391,8 +302,11 @@ __device__ void tile_dense(const Fp32TileParams& P, int64_t band, int64_t seg, i
 #pragma unroll
     for (int a = 0; a < R; ++a) tag[a] = ((unsigned)lane << 3) | (unsigned)a;
 
+    double anchor[R];
+    tile_anchor<kAnchorChunk>(P, j0, gb, g0, lane, rring, anchor);
     float nc[R];
-    anchor_fp32<kAnchorChunk>(P, j0, gb, g0, lane, rring, nc);
+#pragma unroll
+    for (int a = 0; a < R; ++a) nc[a] = (float)anchor[a];
     float2 nc2[H];
 #pragma unroll
     for (int a = 0; a < H; ++a) nc2[a] = make_float2(nc[a], nc[a + H]);
@@ -762,8 +676,11 @@ __device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, in
     const int ghi_rel = (int)max(min(P.g_hi - g0, (int64_t)R), (int64_t)0);
     const int minlim = __reduce_min_sync(kFullMask, ghi_rel < R ? 0 : min(lim0 - (R - 1), ncols));
 
+    double anchor[R];
+    tile_anchor<kAnchorChunk>(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), anchor);
     float nc[R];
-    anchor_fp32<kAnchorChunk>(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), nc);
+#pragma unroll
+    for (int a = 0; a < R; ++a) nc[a] = (float)anchor[a];
 
     // groups 0 .. 33 and the first pass's columns; from here on lanes 0 - 15 look
     // after rows, lanes 16 - 31 after columns
