@@ -38,12 +38,9 @@ int main(int argc, char** argv) {
     cudaMalloc(&desc, sizeof(Fp32TileParams));
     cudaMemset(A, 0, 8 * (n + pad)); cudaMemset(mean, 0, 8 * (PL + pad)); cudaMemset(norm, 0, 8 * (PL + pad));
     cudaMemcpy(A, x.data(), 8 * n, cudaMemcpyHostToDevice);
-    change_flags_kernel<<<grid_for(n), 256>>>(A, n, chg);
-    scan_blocks_kernel<<<(unsigned)blk, 256>>>(chg, n, tot);
-    scan_totals_kernel<<<1, 1>>>(tot, blk);
-    scan_add_kernel<<<(unsigned)blk, 256>>>(chg, n, tot);
-    welford_kernel<<<grid_for((PL + 255) / 256), 256>>>(A, m, PL, 256, chg, mean, norm);
-    pack_fp32_kernel<<<grid_for(PL + pad), 256>>>(A, m, PL, 4, PL + pad, mean, norm, row, col);
+    launch_fp32_stats(A, m, PL, pad, chg, tot, mean, norm, 0);
+    pack_fp32_kernel<<<grid_for(PL + pad), 256>>>(A, m, PL, 4, PL + pad, mean, norm, row, col, key, 0ull,
+                                                  Fp32TileParams{}, nullptr, nullptr);
     Fp32TileParams P{};
     P.rowrec = row; P.colrec = col; P.A = A; P.mean = mean; P.m = m; P.PL = PL;
     P.g_lo = lo; P.g_hi = hi < PL ? hi : PL; P.K = reanchor_interval(K, 8); P.key = key;

@@ -42,11 +42,7 @@ int main(int argc, char** argv) {
     cudaMemset(counter, 0, 8);
     cudaMemcpy(A, x.data(), 8 * n, cudaMemcpyHostToDevice);
     cudaMemcpy(hazard, hz.data(), 4 * (PL + 1), cudaMemcpyHostToDevice);
-    change_flags_kernel<<<grid_for(n), 256>>>(A, n, chg);
-    scan_blocks_kernel<<<(unsigned)blk, 256>>>(chg, n, tot);
-    scan_totals_kernel<<<1, 1>>>(tot, blk);
-    scan_add_kernel<<<(unsigned)blk, 256>>>(chg, n, tot);
-    welford_kernel<<<grid_for((PL + 255) / 256), 256>>>(A, m, PL, 256, chg, mean, norm);
+    launch_fp32_stats(A, m, PL, pad, chg, tot, mean, norm, 0);
     guard_terms_kernel<<<grid_for(PL), 256>>>(A, m, PL, mean, df, dg);
     const float ulim = (float)(1.0 + 1.0 / (double)m);
     init_keys_kernel<<<grid_for(PL), 256>>>(key, PL, (unsigned long long)host_ord_f32(ulim) << 32);

@@ -47,13 +47,32 @@ __global__ void batch_convert_kernel(const BatchSeries* __restrict__ S, const vo
     }
 }
 
-// Per-series inclusive count of value changes (one block per series; the
-// block walks the series in blockDim-sized pieces carrying the running sum).
-__global__ void batch_change_count_kernel(const BatchSeries* __restrict__ S,
-                                          const double* __restrict__ A, int* __restrict__ nchg) {
+// Window statistics, a block per 32 chunks of a series (see stat_block), and the
+// zeros behind them.
+__global__ void __launch_bounds__(kStatThreads)
+    batch_stat_kernel(const BatchSeries* __restrict__ S, const double* __restrict__ A,
+                      double* __restrict__ mean, double* __restrict__ norm) {
+    extern __shared__ __align__(16) char smem_stat[];
+    const BatchSeries s = S[blockIdx.y];
+    FOR_SERIES_ELEMS(kPad) {
+        mean[s.w_off + s.PL + i] = 0.0;
+        norm[s.w_off + s.PL + i] = 0.0;
+    }
+    if (s.m > kStatMaxM) return;  // batch_long_stat_kernel
+    for (int64_t base = blockIdx.x * (int64_t)kStatSpan; base < s.PL; base += (int64_t)gridDim.x * kStatSpan)
+        stat_block(A + s.a_off, s.m, s.PL, base, mean + s.w_off, norm + s.w_off, smem_stat);
+}
+
+// Series whose windows are too long for that: one block counts the value changes
+// (walking the series in pieces and carrying the running sum), then walks the
+// chunks, one per thread.
+__global__ void batch_long_stat_kernel(const BatchSeries* __restrict__ S, const double* __restrict__ A,
+                                       int* __restrict__ nchg, double* __restrict__ mean,
+                                       double* __restrict__ norm) {
     __shared__ int wsum[32];
     __shared__ int carry;
     const BatchSeries s = S[blockIdx.x];
+    if (s.m <= kStatMaxM) return;
     const double* a = A + s.a_off;
     int* out = nchg + s.a_off;
     if (threadIdx.x == 0) carry = 0;
@@ -86,21 +105,9 @@ __global__ void batch_change_count_kernel(const BatchSeries* __restrict__ S,
         if (threadIdx.x == blockDim.x - 1) carry = v;
         __syncthreads();
     }
-}
-
-__global__ void batch_welford_kernel(const BatchSeries* __restrict__ S, const double* __restrict__ A,
-                                     const int* __restrict__ nchg, int64_t chunk,
-                                     double* __restrict__ mean, double* __restrict__ norm) {
-    const BatchSeries s = S[blockIdx.y];
-    const int64_t nchunks = (s.PL + chunk - 1) / chunk;
-    FOR_SERIES_ELEMS(nchunks) {
-        welford_chunk(A + s.a_off, s.m, s.PL, chunk, i, nchg + s.a_off, mean + s.w_off,
-                      norm + s.w_off);
-    }
-    FOR_SERIES_ELEMS(kPad) {
-        mean[s.w_off + s.PL + i] = 0.0;
-        norm[s.w_off + s.PL + i] = 0.0;
-    }
+    const int64_t nchunks = (s.PL + kStatChunk - 1) / kStatChunk;
+    for (int64_t c = threadIdx.x; c < nchunks; c += blockDim.x)
+        welford_chunk(a, s.m, s.PL, kStatChunk, c, out, mean + s.w_off, norm + s.w_off);
 }
 
 __global__ void batch_pack_kernel(const BatchSeries* __restrict__ S, const double* __restrict__ A,
@@ -200,9 +207,15 @@ int enqueue_batch(mp_batch* b, cudaStream_t st) {
     if (b->count > 65535) return MP_ERR_NOT_SUPPORTED;
     const dim3 grid(64, maxy);
     batch_convert_kernel<<<grid, 256, 0, st>>>(b->d_series, b->d_in, b->input_f32, b->d_A);
-    batch_change_count_kernel<<<(unsigned)b->count, 256, 0, st>>>(b->d_series, b->d_A, b->d_nchg);
-    batch_welford_kernel<<<grid, 256, 0, st>>>(b->d_series, b->d_A, b->d_nchg, 256, b->d_mean,
-                                               b->d_norm);
+    int64_t m = 2, PL = 1;  // longest window of one block's statistics, longest profile
+    for (const BatchSeries& s : b->series) {
+        if (s.m <= kStatMaxM) m = std::max(m, s.m);
+        PL = std::max(PL, s.PL);
+    }
+    const dim3 sgrid((unsigned)std::min<int64_t>((PL + kStatSpan - 1) / kStatSpan, 128), maxy);
+    batch_stat_kernel<<<sgrid, kStatThreads, stat_smem_bytes(m), st>>>(b->d_series, b->d_A, b->d_mean, b->d_norm);
+    batch_long_stat_kernel<<<(unsigned)b->count, 256, 0, st>>>(b->d_series, b->d_A, b->d_nchg, b->d_mean,
+                                                               b->d_norm);
     batch_pack_kernel<<<grid, 256, 0, st>>>(b->d_series, b->d_A, b->d_mean, b->d_norm, b->d_row,
                                             b->d_col, b->d_key, b->d_ulim);
     cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), st);
@@ -337,6 +350,8 @@ int mp_batch_create(mp_context* ctx, int64_t count, const int64_t* lengths, cons
         return MP_ERR_CUDA;
     }
     configure_fp32_join<kR>();
+    cudaFuncSetAttribute(batch_stat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)stat_smem_bytes(kStatMaxM));
     *out = b;
     return MP_OK;
 }

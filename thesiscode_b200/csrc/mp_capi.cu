@@ -533,61 +533,55 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
     MP_CUDA(ctx, cudaMemcpyAsync(Apad, A, 8 * n, a_dev ? cudaMemcpyDeviceToDevice
                                                        : cudaMemcpyHostToDevice, st));
     mark(ctx, 0, st);
-    MP_CUDA(ctx, cudaMemsetAsync(Apad + n, 0, 8 * kFp32Pad, st));
-    change_flags_kernel<<<grid_for(n), kThreads, 0, st>>>(Apad, n, nchg);
-    MP_LAUNCHED(ctx);
-    scan_blocks_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    MP_LAUNCHED(ctx);
-    scan_totals_kernel<<<1, 1, 0, st>>>(tot, nblk);
-    MP_LAUNCHED(ctx);
-    scan_add_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    MP_LAUNCHED(ctx);
-    MP_CUDA(ctx, cudaMemsetAsync(mean + PL, 0, 8 * kFp32Pad, st));
-    MP_CUDA(ctx, cudaMemsetAsync(norm + PL, 0, 8 * kFp32Pad, st));
-    const int64_t chunk = 256;
-    welford_kernel<<<grid_for((PL + chunk - 1) / chunk), kThreads, 0, st>>>(Apad, m, PL, chunk, nchg,
-                                                                           mean, norm);
-    MP_LAUNCHED(ctx);
-    pack_fp32_kernel<<<grid_for(PL + kFp32Pad), kThreads, 0, st>>>(
-        Apad, m, PL, kFp32R / 2, PL + kFp32Pad, mean, norm, rowrec, colrec);
-    MP_LAUNCHED(ctx);
+    ctx->launches += launch_fp32_stats(Apad, m, PL, kFp32Pad, nchg, tot, mean, norm, st);
+    // one descriptor per diagonal range, all merging into the same keys
+    std::vector<Fp32TileParams> Ps;
+    int64_t ntiles = 0;
+    for (const DiagRange& r : ranges) {
+        Fp32TileParams Q{};
+        Q.rowrec = rowrec;
+        Q.colrec = colrec;
+        Q.A = Apad;
+        Q.mean = mean;
+        Q.m = m;
+        Q.PL = PL;
+        Q.g_lo = r.lo;
+        Q.g_hi = r.hi;
+        Q.K = K;
+        int64_t nt = 0;
+        fp32_tile_plan(PL, r.lo, r.hi, K, kFp32R, Q.nbands, Q.seg_per_pair, nt);
+        Q.tile_begin = ntiles;
+        ntiles += nt;
+        Q.key = key;
+        Ps.push_back(Q);
+    }
+    int *hz = nullptr, *htot = nullptr;
+    double *pre = nullptr, *suf = nullptr, *gdf = nullptr, *gdg = nullptr;
+    if (guarded && ndiag > 0) {  // exactly one range
+        hz = cv.take<int>(PL + 1);
+        htot = cv.take<int>((PL + 1 + kThreads - 1) / kThreads + 1);
+        pre = cv.take<double>(PL);
+        suf = cv.take<double>(PL);
+        gdf = cv.take<double>(PL);
+        gdg = cv.take<double>(PL);
+        Ps[0].hazard = hz;
+        Ps[0].norm = norm;
+        Ps[0].df = gdf;
+        Ps[0].dg = gdg;
+    }
     const float ulim = (float)(1.0 + 1.0 / (double)m);
-    init_keys_kernel<<<grid_for(PL), kThreads, 0, st>>>(
-        key, PL, (unsigned long long)host_ord_f32(ulim) << 32);
+    const bool single = Ps.size() == 1;  // then the descriptor travels as a kernel argument
+    pack_fp32_kernel<<<grid_for(PL + kFp32Pad), kThreads, 0, st>>>(
+        Apad, m, PL, kFp32R / 2, PL + kFp32Pad, mean, norm, rowrec, colrec, key,
+        (unsigned long long)host_ord_f32(ulim) << 32, single ? Ps[0] : Fp32TileParams{},
+        single ? desc : nullptr, counter);
     MP_LAUNCHED(ctx);
     mark(ctx, 1, st);
     if (ndiag > 0) {
-        // one descriptor per diagonal range, all merging into the same keys
-        std::vector<Fp32TileParams> Ps;
-        int64_t ntiles = 0;
-        for (const DiagRange& r : ranges) {
-            Fp32TileParams Q{};
-            Q.rowrec = rowrec;
-            Q.colrec = colrec;
-            Q.A = Apad;
-            Q.mean = mean;
-            Q.m = m;
-            Q.PL = PL;
-            Q.g_lo = r.lo;
-            Q.g_hi = r.hi;
-            Q.K = K;
-            int64_t nt = 0;
-            fp32_tile_plan(PL, r.lo, r.hi, K, kFp32R, Q.nbands, Q.seg_per_pair, nt);
-            Q.tile_begin = ntiles;
-            ntiles += nt;
-            Q.key = key;
-            Ps.push_back(Q);
-        }
-        Fp32TileParams& P = Ps[0];  // the guarded form has exactly one range
+        const Fp32TileParams& P = Ps[0];
         if (guarded) {
             // hazard windows (prefix counts over PL + 1 entries) and FP64 terms
-            int* hz = cv.take<int>(PL + 1);
             const int64_t hblk = (PL + 1 + kThreads - 1) / kThreads;
-            int* htot = cv.take<int>(hblk + 1);
-            double* pre = cv.take<double>(PL);
-            double* suf = cv.take<double>(PL);
-            double* gdf = cv.take<double>(PL);
-            double* gdg = cv.take<double>(PL);
             const int64_t blk = K + 32 * kFp32R + 1;  // look back K + 32R windows
             const int64_t nb = (PL + blk - 1) / blk;
             hazard_block_minima_kernel<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(norm, PL, blk,
@@ -603,16 +597,13 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             MP_LAUNCHED(ctx);
             guard_terms_kernel<<<grid_for(PL), kThreads, 0, st>>>(Apad, m, PL, mean, gdf, gdg);
             MP_LAUNCHED(ctx);
-            P.hazard = hz;
-            P.norm = norm;
-            P.df = gdf;
-            P.dg = gdg;
         }
-        MP_CUDA(ctx, cudaMemcpyAsync(desc, Ps.data(), sizeof(Fp32TileParams) * Ps.size(),
-                                     cudaMemcpyHostToDevice, st));
-        MP_CUDA(ctx, cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
+        if (!single)
+            MP_CUDA(ctx, cudaMemcpyAsync(desc, Ps.data(), sizeof(Fp32TileParams) * Ps.size(),
+                                         cudaMemcpyHostToDevice, st));
         // the guarded form's keys name candidate groups, resolved in FP64 below
-        launch_fp32_join<kFp32R>(desc, (int)Ps.size(), ntiles, counter, st, fp32_way_of(Ps.data(), Ps.size()), guarded);
+        launch_fp32_join<kFp32R>(desc, (int)Ps.size(), ntiles, counter, st,
+                                 fp32_way_of(Ps.data(), Ps.size()), guarded);
         MP_LAUNCHED(ctx);
         if (guarded) {
             // the same tiles again: the FP64 pass evaluates those the FP32 pass skipped
@@ -651,8 +642,8 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
                 MP_LAUNCHED(ctx);
             }
         }
-        // the descriptor copy above reads host stack memory: finish it before returning
-        MP_CUDA(ctx, cudaStreamSynchronize(st));
+        // the descriptor copy above reads host memory: finish it before returning
+        if (!single) MP_CUDA(ctx, cudaStreamSynchronize(st));
     }
     mark(ctx, 2, st);
     if (guarded)  // group keys; the chosen pair's distance from a centred FP64 dot product

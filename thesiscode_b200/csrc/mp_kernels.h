@@ -31,9 +31,12 @@ __global__ void scan_totals_kernel(int* tot, int64_t nblocks);
 __global__ void scan_add_kernel(int* x, int64_t n, const int* tot);
 __global__ void welford_kernel(const double* A, int64_t m, int64_t PL, int64_t chunk,
                                const int* nchg, double* mean_out, double* norm_out);
-__global__ void pack_fp32_kernel(const double* A, int64_t m, int64_t PL, int H, int64_t count,
-                                 const double* mean, const double* norm, float4* rowrec,
-                                 float4* colrec);
+// Window means and inverse norms of the FP32 forms, with `pad` zeros behind the
+// series and both; nchg (n ints) and tot (n / 256 + 2 ints) are used by windows too
+// long for one block's shared memory.  Returns the number of launches.
+int launch_fp32_stats(double* A, int64_t m, int64_t PL, int64_t pad, int* nchg, int* tot, double* mean,
+                      double* norm, cudaStream_t s);
+void configure_stats();  // per-device setup, before a stream capture
 
 // ---- FP64 diagonal-band join (mp_join_fp64.cu) ------------------------------
 // Diagonal g (g_lo <= g < g_hi) meets column j in row r = j + g, for
@@ -184,6 +187,13 @@ __device__ __forceinline__ bool fp32_tile_hazardous(const Fp32TileParams& P, int
     const int64_t rs = min(j0 + gb, P.PL), re = min(j1 + gb + span, P.PL);
     return (P.hazard[j1] - P.hazard[j0]) > 0 || (P.hazard[re] - P.hazard[rs]) > 0;
 }
+
+// Records (count of them), keys (set to init), and optionally the launch's only
+// descriptor P -> *desc and its tile counter.
+__global__ void pack_fp32_kernel(const double* A, int64_t m, int64_t PL, int H, int64_t count,
+                                 const double* mean, const double* norm, float4* rowrec, float4* colrec,
+                                 unsigned long long* key, unsigned long long init, const Fp32TileParams P,
+                                 Fp32TileParams* desc, unsigned long long* counter);
 
 // FP32 profile keys, min-merged: (ordered u << 32) | neighbour.  With group
 // keys (the guarded form) the tile kernel finds a minimum's lane but not which

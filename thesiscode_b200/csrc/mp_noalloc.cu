@@ -102,6 +102,7 @@ int setup_current_device(void** out, int* dev_out, char* err, size_t len) {
                           cudaGetErrorString(e));
         }
         configure_fp32_join<kR>();
+        configure_stats();
         if (cudaGetLastError() != cudaSuccess)
             return report(err, len, MP_ERR_CUDA, "configuring the join kernel failed");
         g_scratch_addr[dev] = p;
@@ -111,10 +112,6 @@ int setup_current_device(void** out, int* dev_out, char* err, size_t len) {
     return MP_OK;
 }
 
-
-// Writes the tile descriptor from a kernel argument, so that nothing on the
-// stream reads host memory after this function has returned.
-__global__ void noalloc_desc_kernel(Fp32TileParams* d, Fp32TileParams P) { *d = P; }
 
 }  // namespace
 }  // namespace mpgpu
@@ -161,7 +158,7 @@ extern "C" int mp_selfjoin_fp32_noalloc(const double* A_dev, int64_t n, int64_t 
     Fp32TileParams* desc = reinterpret_cast<Fp32TileParams*>(b + L.desc);
     unsigned long long* counter = reinterpret_cast<unsigned long long*>(b + L.counter);
 
-    const int64_t PL = n - m + 1, nblk = (n + kThreads - 1) / kThreads;
+    const int64_t PL = n - m + 1;
     const int64_t ex = excl < 0 ? m / 4 : excl;
     const int64_t lo = ex + 1, hi = PL;
     const int64_t K = reanchor_interval(reanchor_k, kR);
@@ -173,23 +170,10 @@ extern "C" int mp_selfjoin_fp32_noalloc(const double* A_dev, int64_t n, int64_t 
     // (set to the "no neighbour" key), the descriptor and the tile counter,
     // which must start at zero.
     cudaMemcpyAsync(Apad, A_dev, 8 * n, cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(Apad + n, 0, 8 * kPad, st);
-    change_flags_kernel<<<grid_for(n), kThreads, 0, st>>>(Apad, n, nchg);
-    scan_blocks_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    scan_totals_kernel<<<1, 1, 0, st>>>(tot, nblk);
-    scan_add_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    cudaMemsetAsync(mean + PL, 0, 8 * kPad, st);
-    cudaMemsetAsync(norm + PL, 0, 8 * kPad, st);
-    const int64_t chunk = 256;
-    welford_kernel<<<grid_for((PL + chunk - 1) / chunk), kThreads, 0, st>>>(Apad, m, PL, chunk, nchg,
-                                                                           mean, norm);
-    pack_fp32_kernel<<<grid_for(PL + kPad), kThreads, 0, st>>>(Apad, m, PL, kR / 2, PL + kPad, mean,
-                                                               norm, rowrec, colrec);
-    const float ulim = (float)(1.0 + 1.0 / (double)m);
-    init_keys_kernel<<<grid_for(PL), kThreads, 0, st>>>(key, PL,
-                                                        (unsigned long long)host_ord_f32(ulim) << 32);
+    launch_fp32_stats(Apad, m, PL, kPad, nchg, tot, mean, norm, st);
+    Fp32TileParams P{};
+    int64_t ntiles = 0;
     if (hi > lo) {
-        Fp32TileParams P{};
         P.rowrec = rowrec;
         P.colrec = colrec;
         P.A = Apad;
@@ -199,14 +183,17 @@ extern "C" int mp_selfjoin_fp32_noalloc(const double* A_dev, int64_t n, int64_t 
         P.g_lo = lo;
         P.g_hi = hi;
         P.K = K;
-        int64_t ntiles = 0;
         fp32_tile_plan(PL, lo, hi, K, kR, P.nbands, P.seg_per_pair, ntiles);
         P.tile_begin = 0;
         P.key = key;
-        noalloc_desc_kernel<<<1, 1, 0, st>>>(desc, P);
-        cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
-        launch_fp32_join<kR>(desc, 1, ntiles, counter, st, fp32_way_of(&P, 1));
     }
+    const float ulim = (float)(1.0 + 1.0 / (double)m);
+    // the descriptor travels as a kernel argument, so that nothing on the stream
+    // reads host memory after this function has returned
+    pack_fp32_kernel<<<grid_for(PL + kPad), kThreads, 0, st>>>(
+        Apad, m, PL, kR / 2, PL + kPad, mean, norm, rowrec, colrec, key,
+        (unsigned long long)host_ord_f32(ulim) << 32, P, desc, counter);
+    if (hi > lo) launch_fp32_join<kR>(desc, 1, ntiles, counter, st, fp32_way_of(&P, 1));
     finalize_fp32_kernel<<<grid_for(PL), kThreads, 0, st>>>(key, PL, (double)m, Apad, mean, norm, 0,
                                                             dist2_dev, idx_dev);
     const cudaError_t e = cudaGetLastError();

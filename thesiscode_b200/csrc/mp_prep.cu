@@ -7,10 +7,12 @@
 //    operations (__dadd_rn/__dmul_rn/... are never contracted into FMAs) so the
 //    result is bit-identical to the reference built with IEEE semantics.  The
 //    prefix sums are a dependent chain and run on one thread.
-//  * FP64 Welford (FP32 form): each thread slides Welford's mean/M2 update
-//    over a chunk of windows, restarting from a fresh Welford pass at every
-//    chunk start; exact zero-variance windows are found with an integer count
-//    of value changes, so a constant window at any level is flagged exactly.
+//  * FP64 Welford (FP32 form): Welford's mean/M2 update slides over chunks of
+//    256 windows, restarting from a fresh Welford pass at every chunk start;
+//    exact zero-variance windows are found from the places where the value
+//    changes, so a constant window at any level is flagged exactly.
+#include <atomic>
+
 #include "mp_common.cuh"
 #include "mp_kernels.h"
 #include "mp_prep_device.cuh"
@@ -201,14 +203,71 @@ __global__ void welford_kernel(const double* __restrict__ A, int64_t m, int64_t 
         welford_chunk(A, m, PL, chunk, t, nchg, mean_out, norm_out);
 }
 
-// Row and column records of the FP32 form (see pack_fp32_record).
+// Welford statistics, one block per 32 chunks (see stat_block); the zeros behind the
+// series and the statistics, too (their places are read by nothing here).
+__global__ void __launch_bounds__(kStatThreads)
+    stat_kernel(double* A, int64_t m, int64_t PL, int64_t pad, double* mean, double* norm) {
+    extern __shared__ __align__(16) char smem_stat[];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < pad;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        A[PL + m - 1 + i] = 0.0;
+        mean[PL + i] = 0.0;
+        norm[PL + i] = 0.0;
+    }
+    stat_block(A, m, PL, (int64_t)blockIdx.x * kStatSpan, mean, norm, smem_stat);
+}
+
+void configure_stats() {
+    cudaFuncSetAttribute(stat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)stat_smem_bytes(kStatMaxM));
+}
+
+int launch_fp32_stats(double* A, int64_t m, int64_t PL, int64_t pad, int* nchg, int* tot, double* mean,
+                      double* norm, cudaStream_t s) {
+    const int64_t n = PL + m - 1;
+    if (m <= kStatMaxM) {
+        // per-device attribute, idempotent: see launch_fp32_join
+        static std::atomic<unsigned long long> configured{0};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (!(configured.load(std::memory_order_acquire) & bit)) {
+            configure_stats();
+            configured.fetch_or(bit, std::memory_order_release);
+        }
+        stat_kernel<<<(unsigned)((PL + kStatSpan - 1) / kStatSpan), kStatThreads, stat_smem_bytes(m), s>>>(
+            A, m, PL, pad, mean, norm);
+        return 1;
+    }
+    constexpr int T = 256;
+    const int64_t nblk = (n + T - 1) / T;
+    cudaMemsetAsync(A + n, 0, 8 * pad, s);
+    cudaMemsetAsync(mean + PL, 0, 8 * pad, s);
+    cudaMemsetAsync(norm + PL, 0, 8 * pad, s);
+    change_flags_kernel<<<grid_for(n), T, 0, s>>>(A, n, nchg);
+    scan_blocks_kernel<<<(unsigned)nblk, T, 0, s>>>(nchg, n, tot);
+    scan_totals_kernel<<<1, 1, 0, s>>>(tot, nblk);
+    scan_add_kernel<<<(unsigned)nblk, T, 0, s>>>(nchg, n, tot);
+    welford_kernel<<<grid_for((PL + kStatChunk - 1) / kStatChunk), T, 0, s>>>(A, m, PL, kStatChunk, nchg, mean,
+                                                                              norm);
+    return 5;
+}
+
+// Row and column records of the FP32 form (see pack_fp32_record), the keys and,
+// for a launch over one descriptor, that descriptor and the tile counter.
 __global__ void pack_fp32_kernel(const double* __restrict__ A, int64_t m, int64_t PL, int H,
                                  int64_t count, const double* __restrict__ mean,
                                  const double* __restrict__ norm, float4* __restrict__ rowrec,
-                                 float4* __restrict__ colrec) {
+                                 float4* __restrict__ colrec, unsigned long long* __restrict__ key,
+                                 unsigned long long init, const Fp32TileParams P,
+                                 Fp32TileParams* __restrict__ desc, unsigned long long* __restrict__ counter) {
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < count;
-         j += (int64_t)gridDim.x * blockDim.x)
+         j += (int64_t)gridDim.x * blockDim.x) {
         pack_fp32_record(A, m, PL, H, mean, norm, j, rowrec, colrec);
+        if (j < PL) key[j] = init;
+        if (j == 0 && desc) *desc = P;
+        if (j == 0 && counter) *counter = 0;
+    }
 }
 
 }  // namespace mpgpu

@@ -69,24 +69,12 @@ cudaError_t serve_prepare(ServeJob& job, const double* series, int64_t n, int64_
     job.colrec = reinterpret_cast<float4*>(b + L.col);
     job.key = reinterpret_cast<unsigned long long*>(b + L.key);
 
-    const int64_t nblk = (n + kThreads - 1) / kThreads;
     if ((e = cudaMemcpyAsync(job.A, series, 8 * n, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(job.A + n, 0, 8 * kPad, st)) != cudaSuccess) return e;
-    change_flags_kernel<<<grid_for(n), kThreads, 0, st>>>(job.A, n, nchg);
-    scan_blocks_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    scan_totals_kernel<<<1, 1, 0, st>>>(tot, nblk);
-    scan_add_kernel<<<(unsigned)nblk, kThreads, 0, st>>>(nchg, n, tot);
-    if ((e = cudaMemsetAsync(job.mean + PL, 0, 8 * kPad, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(job.norm + PL, 0, 8 * kPad, st)) != cudaSuccess) return e;
-    const int64_t chunk = 256;
-    welford_kernel<<<grid_for((PL + chunk - 1) / chunk), kThreads, 0, st>>>(job.A, m, PL, chunk, nchg,
-                                                                           job.mean, job.norm);
-    pack_fp32_kernel<<<grid_for(PL + kPad), kThreads, 0, st>>>(job.A, m, PL, kR / 2, PL + kPad,
-                                                               job.mean, job.norm, job.rowrec,
-                                                               job.colrec);
+    launch_fp32_stats(job.A, m, PL, kPad, nchg, tot, job.mean, job.norm, st);
     const float ulim = (float)(1.0 + 1.0 / (double)m);
-    init_keys_kernel<<<grid_for(PL), kThreads, 0, st>>>(
-        job.key, PL, (unsigned long long)host_ord_f32(ulim) << 32);
+    pack_fp32_kernel<<<grid_for(PL + kPad), kThreads, 0, st>>>(
+        job.A, m, PL, kR / 2, PL + kPad, job.mean, job.norm, job.rowrec, job.colrec, job.key,
+        (unsigned long long)host_ord_f32(ulim) << 32, Fp32TileParams{}, nullptr, nullptr);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
     job.K = reanchor_interval(reanchor_k, kR);
