@@ -17,7 +17,7 @@ int ctx_device(const mp_context* ctx);
 
 // ---- preparation (mp_prep.cu) ----------------------------------------------
 constexpr int kPrefixThreads = 256;  // ref_prefix_kernel: one block of this many threads
-constexpr int kPrefixChunk = 1024;   // elements of A per shared-memory chunk
+constexpr int kPrefixChunk = 736;    // elements of A per shared-memory chunk (48 KB of buffers)
 __global__ void ref_prefix_kernel(const double* A, int64_t n, double* cs, double* cs2);
 __global__ void ref_stats_kernel(const double* cs, const double* cs2, int64_t PL, int64_t m,
                                  double* muS, double* sInv);

@@ -67,11 +67,14 @@ __host__ __device__ constexpr size_t stat_smem_bytes(int64_t m) {
     const size_t S = (size_t)(kStatSpan + m);
     return 8 * (S + S / 256 + 1) + 4 * 8 * kStatBatch + (2 * S + 7) / 8 * 8;
 }
+// Out of line, so that the chain does not carry a division along.
+static __device__ __noinline__ double plain_division(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ double quotient(double a, double b, double r) {
     const double q = __dmul_rn(a, r);
     const double z = __fma_rn(__fma_rn(-b, q, a), r, q);
     const double x = fabs(a);
-    return x > 1e-280 && x < 1e280 ? z : __ddiv_rn(a, b);
+    if (x > 1e-280 && x < 1e280) return z;
+    return plain_division(a, b);
 }
 __device__ __forceinline__ void stat_block(const double* __restrict__ A, int64_t m, int64_t PL, int64_t base,
                                            double* __restrict__ mean_out, double* __restrict__ norm_out,

@@ -19,10 +19,15 @@ namespace mpgpu {
 
 namespace {
 
-constexpr int kQB = 32;    // queries per CTA
-constexpr int kQT = kQB / 4;  // queries per thread
-constexpr int kJB = 256;   // windows per CTA
-constexpr int kKC = 32;    // window elements per shared-memory stage
+constexpr int kQB = 32;          // queries per CTA, all of them in every warp
+constexpr int kJW = 64;          // windows per warp
+constexpr int kRowWarps = 4;     // warps per CTA
+constexpr int kRowThreads = 32 * kRowWarps;
+constexpr int kJB = kRowWarps * kJW;  // windows per CTA; a query's best of them is one merge
+constexpr int kKC = 32;          // window elements per shared-memory stage
+constexpr int kQS = kKC + 4;     // doubles between a stage's queries: conflict-free A fragments
+constexpr int kWN = kJB + kKC;   // series values per stage
+constexpr int kStage = kQB * kQS + kWN;  // doubles per stage
 constexpr unsigned long long kNone = ~0ull;
 
 // Distance keys: ord(d) min-merged (exact); index keys: ord(d) with its low
@@ -69,127 +74,174 @@ __global__ void prescrimp_keys_init_kernel(unsigned long long* __restrict__ a, i
         a[i] = kNone;
 }
 
+// 8-byte asynchronous copy global -> shared that writes zero where !inside.
+static __device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
+                 "r"(inside ? 8 : 0)
+                 : "memory");
+}
+
 // Query rows: CTA b covers windows [wt*256, wt*256+256) and queries
 // [qt*32, qt*32+32), wt = b % window tiles, qt = b / window tiles (a 1-D grid,
-// so any number of queries fits).  Thread (ty, tx) accumulates 8 queries x 4
-// windows (12 shared-memory reads per 32 FMAs).
-__global__ void __launch_bounds__(256) prescrimp_rows_kernel(const PreScrimpParams P) {
-    __shared__ double sq[kQB][kKC + 1];
-    __shared__ double sw[kJB + kKC];
-    __shared__ double cbest[4][kJB];
-    __shared__ int cidx[4][kJB];
-    __shared__ double rbest[64][kQB + 1];
-    __shared__ int ridx[64][kQB + 1];
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+// so any number of queries fits).  The dot products are a matrix product,
+// queries x elements by elements x windows, on the FP64 matrix instruction: a warp
+// takes 32 queries x 64 windows (4 x 8 blocks), each cell accumulated in k order;
+// both operands come straight from stages of the series in shared memory (window w's
+// element k is value w + k), 12 reads per 32 instructions.  The next stage is copied
+// in while one runs.
+// What bounds it: the FP64 pipe, m operations per cell, and the distances, as many
+// instructions per cell as m = 256 matrix ones; three CTAs per SM overlap the two.
+// 200,003 samples, m = 256, stride 0.25 (1.6e11 operations, 8.8 ms at the pipe's
+// rate): 11.5 ms (12.6 with two CTAs, 13.6 with one of 8 warps).  8 queries x 4
+// windows per thread in multiply-adds took 16.0, 8 x 8 with the windows sliding
+// through registers 16.9.
+__global__ void __launch_bounds__(kRowThreads, 3) prescrimp_rows_kernel(const PreScrimpParams P) {
+    extern __shared__ __align__(16) double smem_rows[];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    const int lr = lane >> 2, lc = lane & 3;  // fragment row and column
     const int64_t nwt = (P.PL + kJB - 1) / kJB;
     const int64_t j0 = ((int64_t)blockIdx.x % nwt) * kJB;
     const int64_t t0 = ((int64_t)blockIdx.x / nwt) * kQB;
-    double acc[kQT][4];
+    // a thread copies element threadIdx.x % 32 of queries threadIdx.x / 32 + 4 i, and
+    // series values threadIdx.x + 128 i
+    const int qk = threadIdx.x & 31, q0 = threadIdx.x >> 5;
+    const double* qsrc = P.A + (t0 + q0) * P.step + qk;
+    const int nq = (int)min((int64_t)kQB, P.Q - t0);  // queries of the tile
+    auto load = [&](int64_t k0, int buf) {
+        double* sq = smem_rows + buf * kStage;
+        double* sw = sq + kQB * kQS;
 #pragma unroll
-    for (int r = 0; r < kQT; ++r)
+        for (int i = 0; i < kQB / kRowWarps; ++i) {
+            const int q = q0 + kRowWarps * i;
+            const bool in = q < nq && k0 + qk < P.m;
+            cp_async8_or_zero(sq + q * kQS + qk, in ? qsrc + kRowWarps * i * P.step + k0 : P.A, in);
+        }
+        const int64_t left = P.n - j0 - k0;  // zero past the series: only cells j >= PL read it
+        for (int e = threadIdx.x; e < kWN; e += kRowThreads)
+            cp_async8_or_zero(sw + e, e < left ? P.A + j0 + k0 + e : P.A, e < left);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double acc[4][8][2];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
-    for (int64_t k0 = 0; k0 < P.m; k0 += kKC) {
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[r][c][0] = acc[r][c][1] = 0.0;
+    load(0, 0);
+    int buf = 0;
+    for (int64_t k0 = 0; k0 < P.m; k0 += kKC, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
-        for (int e = threadIdx.x; e < kQB * kKC; e += blockDim.x) {
-            const int qi = e / kKC, kk = e % kKC;
-            const int64_t t = t0 + qi, k = k0 + kk;
-            sq[qi][kk] = (t < P.Q && k < P.m) ? P.A[t * P.step + k] : 0.0;
-        }
-        for (int e = threadIdx.x; e < kJB + kKC; e += blockDim.x) {
-            const int64_t x = j0 + k0 + e;
-            sw[e] = x < P.n ? P.A[x] : 0.0;  // zero past the series: only cells j >= PL read it
-        }
-        __syncthreads();
+        if (k0 + kKC < P.m) load(k0 + kKC, buf ^ 1);
+        const double* sq = smem_rows + buf * kStage + lr * kQS + lc;
+        const double* sw = smem_rows + buf * kStage + kQB * kQS + wi * kJW + lr + lc;
         const int kn = (int)min((int64_t)kKC, P.m - k0);
-        for (int kk = 0; kk < kn; ++kk) {
-            double a[kQT], w[4];
+        auto step = [&](int kk, bool in) {  // elements kk .. kk + 3; in: the lane's is one of the m
+            double a[4], b[8];
 #pragma unroll
-            for (int r = 0; r < kQT; ++r) a[r] = sq[ty * kQT + r][kk];
+            for (int r = 0; r < 4; ++r) a[r] = in ? sq[8 * r * kQS + kk] : 0.0;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) w[c] = sw[tx * 4 + c + kk];
+            for (int c = 0; c < 8; ++c) b[c] = in ? sw[8 * c + kk] : 0.0;
 #pragma unroll
-            for (int r = 0; r < kQT; ++r)
+            for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = __fma_rn(a[r], w[c], acc[r][c]);
-        }
+                for (int c = 0; c < 8; ++c) mma_f64(acc[r][c], a[r], b[c]);
+        };
+        int kk = 0;
+#pragma unroll 2
+        for (; kk + 4 <= kn; kk += 4) step(kk, true);
+        if (kk < kn) step(kk, kk + lc < kn);  // 0 * 0 for the elements past m
     }
-    // distances; per window the best of this thread's 4 queries, per query the
-    // best of its 4 windows
+    // distances; per query the warp's best window, per window its best query
     const double mm = (double)P.m;
-    double cb[4], rb[kQT];
-    int ci[4], ri[kQT];
+    double rb[4];
+    int ri[4];
+    double mi[4], si[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        cb[c] = DBL_MAX;
-        ci[c] = -1;
-    }
-#pragma unroll
-    for (int r = 0; r < kQT; ++r) {
+    for (int r = 0; r < 4; ++r) {
+        const int64_t t = t0 + 8 * r + lr;
         rb[r] = DBL_MAX;
         ri[r] = -1;
+        mi[r] = t < P.Q ? P.mean[t * P.step] : 0.0;
+        si[r] = t < P.Q ? P.sigma[t * P.step] : 0.0;
     }
+    const int i0 = (int)(t0 * P.step), jw = (int)j0 + wi * kJW, PL = (int)P.PL;
+    const int step = (int)min(P.step, P.PL), excl = (int)min(P.excl, P.PL);
 #pragma unroll
-    for (int r = 0; r < kQT; ++r) {
-        const int64_t t = t0 + ty * kQT + r;
-        if (t >= P.Q) continue;
-        const int64_t i = t * P.step;
-        const double mi = P.mean[i], si = P.sigma[i];
+    for (int c = 0; c < 8; ++c) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t j = j0 + tx * 4 + c;
-            if (j >= P.PL) continue;
-            if (j > i - P.excl && j < i + P.excl) continue;  // ScrimpppOrig.cpp:190-193
-            const double d = orig_distance(mm, acc[r][c], P.mean[j], mi, P.sigma[j], si);
-            if (d < cb[c]) {
-                cb[c] = d;
-                ci[c] = (int)i;
+        for (int h = 0; h < 2; ++h) {
+            const int j = jw + 8 * c + 2 * lc + h;
+            double cb = DBL_MAX;
+            int ci = -1;
+            if (j < PL) {
+                const double mj = __dmul_rn(mm, P.mean[j]), sj = P.sigma[j];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int q = 8 * r + lr;
+                    const int i = i0 + q * step;
+                    if (q >= nq || (j > i - excl && j < i + excl)) continue;  // ScrimpppOrig.cpp:190-193
+                    // orig_distance
+                    const double d = __dmul_rn(
+                        2.0, __dsub_rn(mm, __ddiv_rn(__dsub_rn(acc[r][c][h], __dmul_rn(mj, mi[r])),
+                                                     __dmul_rn(sj, si[r]))));
+                    if (d < cb) {
+                        cb = d;
+                        ci = i;
+                    }
+                    if (d < rb[r]) {
+                        rb[r] = d;
+                        ri[r] = j;
+                    }
+                }
             }
-            if (d < rb[r]) {
-                rb[r] = d;
-                ri[r] = (int)j;
+            // over the warp's queries, the smallest among equals
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                const double d = __shfl_xor_sync(kFullMask, cb, o);
+                const int i = __shfl_xor_sync(kFullMask, ci, o);
+                if (i >= 0 && (ci < 0 || d < cb || (d == cb && i < ci))) {
+                    cb = d;
+                    ci = i;
+                }
             }
+            if (lr == 0 && ci >= 0) merge(P.kex, P.kix, j, cb, ci, P.idx_bits);
         }
     }
+    __syncthreads();  // the stages are free
+    double* rbest = smem_rows;                                   // [kRowWarps][kQB]
+    int* ridx = reinterpret_cast<int*>(rbest + kRowWarps * kQB);  // [kRowWarps][kQB]
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        cbest[ty][tx * 4 + c] = cb[c];
-        cidx[ty][tx * 4 + c] = ci[c];
-    }
+    for (int r = 0; r < 4; ++r) {
 #pragma unroll
-    for (int r = 0; r < kQT; ++r) {
-        rbest[tx][ty * kQT + r] = rb[r];
-        ridx[tx][ty * kQT + r] = ri[r];
+        for (int o = 1; o < 4; o <<= 1) {
+            const double d = __shfl_xor_sync(kFullMask, rb[r], o);
+            const int j = __shfl_xor_sync(kFullMask, ri[r], o);
+            if (j >= 0 && (ri[r] < 0 || d < rb[r] || (d == rb[r] && j < ri[r]))) {
+                rb[r] = d;
+                ri[r] = j;
+            }
+        }
+        if (lc == 0) {
+            rbest[wi * kQB + 8 * r + lr] = rb[r];
+            ridx[wi * kQB + 8 * r + lr] = ri[r];
+        }
     }
     __syncthreads();
-    // windows: one thread per window of the tile
-    {
-        const int c = threadIdx.x;
-        double b = cbest[0][c];
-        int bi = cidx[0][c];
-        for (int y = 1; y < 4; ++y)
-            if (cidx[y][c] >= 0 && (bi < 0 || cbest[y][c] < b)) {
-                b = cbest[y][c];
-                bi = cidx[y][c];
-            }
-        if (bi >= 0) merge(P.kex, P.kix, j0 + c, b, bi, P.idx_bits);
-    }
-    // queries: the first 32 threads
     if (threadIdx.x < kQB) {
         const int q = threadIdx.x;
-        const int64_t t = t0 + q;
-        if (t < P.Q) {
-            double b = DBL_MAX;
-            int bi = -1;
-            for (int x = 0; x < 64; ++x)
-                if (ridx[x][q] >= 0 && (bi < 0 || rbest[x][q] < b)) {
-                    b = rbest[x][q];
-                    bi = ridx[x][q];
-                }
-            if (bi >= 0) {
-                merge(P.rex, P.rix, t, b, bi, P.idx_bits);               // the row's own best
-                merge(P.kex, P.kix, t * P.step, b, bi, P.idx_bits);      // profile[i]
+        double b = DBL_MAX;
+        int bj = -1;
+        for (int v = 0; v < kRowWarps; ++v) {
+            const int j = ridx[v * kQB + q];
+            if (j >= 0 && (bj < 0 || rbest[v * kQB + q] < b)) {
+                b = rbest[v * kQB + q];
+                bj = j;
             }
+        }
+        if (bj >= 0) {
+            merge(P.rex, P.rix, t0 + q, b, bj, P.idx_bits);                // the row's own best
+            merge(P.kex, P.kix, (t0 + q) * P.step, b, bj, P.idx_bits);     // profile[i]
         }
     }
 }
@@ -260,7 +312,9 @@ __global__ void prescrimp_finalize_kernel(const unsigned long long* __restrict__
 
 void launch_prescrimp(const PreScrimpParams& P, cudaStream_t s) {
     const int64_t tiles = ((P.PL + kJB - 1) / kJB) * ((P.Q + kQB - 1) / kQB);
-    prescrimp_rows_kernel<<<(unsigned)tiles, 256, 0, s>>>(P);
+    constexpr int smem = 2 * kStage * (int)sizeof(double);
+    static_assert(smem <= 48 * 1024, "two stages within the default shared memory");
+    prescrimp_rows_kernel<<<(unsigned)tiles, kRowThreads, smem, s>>>(P);
     const int64_t threads = 2 * P.Q;
     prescrimp_refine_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(P);
 }
