@@ -321,8 +321,8 @@ int mp_context_create(int device, size_t mem_budget_bytes, mp_context** out) {
         cudaGetLastError();
         return MP_ERR_NO_DEVICE;
     }
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess || prop.major < 10) {
+    int major = 0;  // one attribute: the whole property query takes milliseconds
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess || major < 10) {
         cudaGetLastError();
         return MP_ERR_NO_DEVICE;
     }
