@@ -59,8 +59,7 @@ constexpr int kPad = 9;      // elements between groups: lanes 8 rows apart hit 
 constexpr double kSlack = 1e-6;
 constexpr int kGuardSmem = 2 * kCols * 32 + kGroups * kPad * (16 + 8 + 8 + 8) + 2 * kCols * 4 + kGroups * 4;
 static_assert(kGuardSmem % 16 == 0, "warps' areas stay 16-byte aligned");
-constexpr int kAnchorChunk = 512;
-static_assert(8 * (kAnchorChunk + (32 * kTileR + kAnchorChunk) * 9 / 8) <= kGuardSmem, "anchor staging fits");
+static_assert(kAnchorBytes <= kGuardSmem, "anchor staging fits");
 constexpr int kGuardWarps = 4;
 constexpr int kGuardBlocksPerSm = 3;  // 8.2 ms against 8.8 at 2 (no spill) on the series above
 __device__ __forceinline__ int wrap_group(int s) { return s < kGroups ? s : s - kGroups; }
@@ -232,7 +231,7 @@ __device__ void tile_guard(const Fp32TileParams& P, int64_t band, int64_t seg, i
     const int minlim = __reduce_min_sync(kFullMask, ghi_rel < R ? 0 : min(lim0 - (R - 1), ncols));
 
     double nc[R];  // m mean_j mean_r - sum A[j+k] A[r+k]  (= -covariance)
-    tile_anchor<kAnchorChunk>(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), nc);
+    tile_anchor(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), nc);
 
     // groups 0 .. 33 and the first pass's columns; from here on lanes 0 - 15 look
     // after rows, lanes 16 - 31 after columns

@@ -140,9 +140,6 @@ __device__ __forceinline__ void flush_row(const Fp32TileParams& P, float v, int6
     }
 }
 
-// Terms of the FP64 anchor staged per pass.
-constexpr int kAnchorChunk = 320;
-constexpr int kAnchorBytes = 8 * (kAnchorChunk + (32 * 8 + kAnchorChunk) * 9 / 8);
 static_assert(kAnchorBytes <= kRecRingBytes, "anchor staging fits the record ring");
 
 // ---- every pass with the selection (see fp32_gate_pays) ----------------------
@@ -303,7 +300,7 @@ __device__ void tile_dense(const Fp32TileParams& P, int64_t band, int64_t seg, i
     for (int a = 0; a < R; ++a) tag[a] = ((unsigned)lane << 3) | (unsigned)a;
 
     double anchor[R];
-    tile_anchor<kAnchorChunk>(P, j0, gb, g0, lane, rring, anchor);
+    tile_anchor(P, j0, gb, g0, lane, rring, anchor);
     float nc[R];
 #pragma unroll
     for (int a = 0; a < R; ++a) nc[a] = (float)anchor[a];
@@ -677,7 +674,7 @@ __device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, in
     const int minlim = __reduce_min_sync(kFullMask, ghi_rel < R ? 0 : min(lim0 - (R - 1), ncols));
 
     double anchor[R];
-    tile_anchor<kAnchorChunk>(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), anchor);
+    tile_anchor(P, j0, gb, g0, lane, reinterpret_cast<char*>(sm.col), anchor);
     float nc[R];
 #pragma unroll
     for (int a = 0; a < R; ++a) nc[a] = (float)anchor[a];
