@@ -459,6 +459,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             const int R = pick_fp64_R(nd);
             P.colrec = rec;
             P.rowrec = rec;
+            P.colgate = sInv;
             P.qt0 = qt0 + qoff;
             qoff += nd;
             P.qt_out = nullptr;
@@ -941,6 +942,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     Fp64BandParams P{};
     P.colrec = colrec;
     P.rowrec = rowrec;
+    P.colgate = sh;
     P.qt0 = q;
     P.qt_out = qout;
     P.g_lo = 0;

@@ -41,22 +41,27 @@
 // its row's best).  So the first wave takes every spread-th band of the whole
 // list; the bands between them then meet rows whose bests are nearly final.
 //
-// Passes inside the 4-wide part test in integers, once per kU * R columns: a lane
-// takes the maximum of its scores' high words and compares it with the smallest
-// high word among the best scores of the rows and the thresholds of the columns
-// that it meets in the pass (fp64_gate; high words order like non-negative
-// doubles, and a negative bound opens the gate).  When some lane of the warp
-// passes, the pass is evaluated again with the selection.  That takes R/2 integer
-// maxima per column in place of 2R FP64 compares and two votes, and no branch
-// between the columns.
+// Passes (16 columns) inside the 4-wide part only look for a cell that could select:
+// a column's gate is the score in the form s' (q s - w W'), W' = w' / s', whose last
+// product is taken once for the lane's R cells: 4 FP64 operations per cell in place of
+// 5.  Its high word is compared with those of the column's threshold and of the
+// smallest best score among the R rows (fp64_gate and the functions beside it: the
+// bounds lie below by more than the two forms' rounding differs).  When some lane
+// of the warp passes, the pass is evaluated again with the reference's arithmetic and
+// the selection.  High words take R/2 integer maxima and two additions per column
+// where doubles took 2R compares, and no branch between the columns.
 //
-// What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 5
-// per cell (40 of a step's 62 instructions at R = 8); other instructions cost it
-// about 0.7 cycles each.  n = 1,048,576, m = 256: 254 ms, from 441 ms with the
-// selection tested per step in FP64 and the bands in order of length (gate per
-// step 269 ms; a pass's two chunks as a loop 271 ms; 3 CTAs of 4 warps per SM at
-// 168 registers spill, 273 ms).  With fewer bands than resident warps the longest
-// band sets the time; then the bands are cut into tiles (Fp64Split).
+// What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 4
+// per cell (33 of a step's 60 instructions at R = 8); other instructions cost it
+// about 0.7 cycles each.  n = 1,048,576, m = 256: 243 ms, from 441 ms with the
+// selection tested per step in FP64 and the bands in order of length (one gate per
+// pass and 5 operations: 254 ms; that with a pass's two chunks as a loop 271 ms;
+// 3 CTAs of 4 warps per SM at 168 registers spill, 273 ms).  Short windows have rows
+// of unlike best scores side by side, and one bound for a pass's 23 rows and 16
+// columns opened a quarter of the passes at m = 64 where 2% select (n = 600,000: 164
+// ms; a bound per 15 rows and 8 columns 134; per 8 rows and a column 101).  With
+// fewer bands than resident warps the longest band sets the time; then the bands
+// are cut into tiles (Fp64Split).
 #include <float.h>
 #include <limits.h>
 
@@ -83,6 +88,10 @@ __device__ __forceinline__ double4 ring_rec(const char* p) {
 __device__ __forceinline__ void cp_async16(char* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
+// Scale and mean term of a record.
+__device__ __forceinline__ double2 scale_mean(const double4* rec) {
+    return __ldg(reinterpret_cast<const double2*>(rec) + 1);
 }
 // A threshold as it stands (other warps raise it with atomics meanwhile; any
 // value it has held is a valid lower bound).
@@ -127,14 +136,6 @@ __device__ __forceinline__ void finish_row(const Fp64BandParams& P, int shard, i
     }
 }
 
-// A bound's high word for the integer gate: scores at or above a non-negative
-// bound have a high word at or above its high word (as signed integers); a
-// negative bound lets every cell through.
-__device__ __forceinline__ int fp64_gate(double bound) {
-    const int h = __double2hiint(bound);
-    return h < 0 ? INT_MIN : h;
-}
-
 // One warp's shared memory.  Rows of the band go in groups of R (row t of the
 // tile, counted from its first column's row on the band's first diagonal, is
 // element t % R of group t / R); kGroups slots of R rows form a ring, in which
@@ -142,24 +143,32 @@ __device__ __forceinline__ int fp64_gate(double bound) {
 // groups meanwhile.  Every
 // array is padded by one element per group, so that lanes reading the same
 // element of consecutive groups hit distinct banks (a multiple of 8 groups, so
-// that a wrap keeps that for the 16-byte halves of the records).
-constexpr int kGroups = 40;
-constexpr int kU = 2;  // chunks per pass
-static_assert(kGroups % kU == 0 && kGroups >= 32 + 2 * kU, "a pass's incoming groups fit the ring");
-__device__ __forceinline__ int wrap_group(int s) { return s < kGroups ? s : s - kGroups; }
+// that a wrap keeps that for the 16-byte halves of the records).  A pass is 16
+// columns for every R: half a warp brings in its columns, the other half its rows,
+// and what a pass costs by itself is spread over as many columns (passes of 2R
+// columns at R = 2, a block of 500 diagonals: the same 1.46 ms, but a pass's own
+// instructions then weigh 4 times as much).
 template <int R>
 struct BandSmem {
+    static constexpr int kU = 16 / R;  // chunks per pass
+    static constexpr int kGroups = (32 + 2 * kU + 7) / 8 * 8;
+    static_assert(kGroups % kU == 0 && kU * R <= kFp64SplitUnit, "tiles end with a pass");
+    __device__ static __forceinline__ int wrap(int s) { return s < kGroups ? s : s - kGroups; }
     static constexpr int kRecStride = 32 * R + 16;  // bytes of a group's records
+    static constexpr int kGateStride = R == 8 ? 12 : R;  // lanes hit distinct banks
     static constexpr int kUsed = kGroups * kRecStride + 2 * 32 * R * kU +
                                  kGroups * (R + 1) * (int)(sizeof(double) + sizeof(int)) +
-                                 2 * R * kU * (int)sizeof(double) + kGroups * (int)sizeof(int);
+                                 2 * R * kU * (int)sizeof(double) +
+                                 (kGroups * kGateStride + 2 * R * kU + kGroups / kU) * (int)sizeof(int);
     static constexpr int kBytes = (kUsed + 15) / 16 * 16;  // warps' areas stay aligned
     char* rec;     // row records
-    char* col;     // column records, two buffers of kU * R
+    char* col;     // column records {A[j], A[j+m], s, fp64_gate_mean}, two buffers of kU * R
     double* best;  // best score of each row (its threshold while src < 0)
-    double* cthr;  // column thresholds, two buffers of kU * R
+    double* cmean; // column mean terms, two buffers of kU * R
     int* src;      // column of a row's best score, -1: none yet
-    int* gate;     // per group: smallest gate among the rows' best scores
+    int* gate;     // per row: smallest gate among the best scores of R rows from it on
+    int* cgate;    // gates of the columns' thresholds, two buffers of kU * R
+    int* err;      // per kU groups: largest fp64_gate_error among the rows
     __device__ __forceinline__ BandSmem(char* p) {
         rec = p;
         p += kGroups * kRecStride;
@@ -167,18 +176,30 @@ struct BandSmem {
         p += 2 * 32 * R * kU;
         best = reinterpret_cast<double*>(p);
         p += kGroups * (R + 1) * sizeof(double);
-        cthr = reinterpret_cast<double*>(p);
+        cmean = reinterpret_cast<double*>(p);
         p += 2 * R * kU * sizeof(double);
         src = reinterpret_cast<int*>(p);
         p += kGroups * (R + 1) * sizeof(int);
         gate = reinterpret_cast<int*>(p);
+        cgate = gate + kGroups * kGateStride;
+        err = cgate + 2 * R * kU;
     }
-    // smallest gate among the R rows of the group in slot s
-    __device__ __forceinline__ int group_gate(int s) const {
-        int g = INT_MAX;
+    // gates of the rows of the group in slot s, from the best scores as they stand
+    __device__ __forceinline__ void group_gates(int s, double m) const {
+        const double *b0 = best + s * (R + 1), *b1 = best + wrap(s + 1) * (R + 1);
+        const int hmin = fp64_gate_high_from(m);
+        int x[2 * R - 1], run = INT_MIN;
 #pragma unroll
-        for (int k = 0; k < R; ++k) g = min(g, fp64_gate(best[s * (R + 1) + k]));
-        return g;
+        for (int k = 0; k < 2 * R - 1; ++k)
+            x[k] = fp64_gate_high(__double2hiint(k < R ? b0[k] : b1[k - R]), hmin);
+#pragma unroll
+        for (int k = R - 2; k >= 0; --k) x[k] = max(x[k], x[k + 1]);
+        int* g = gate + s * kGateStride;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            if (k > 0) run = max(run, x[R - 1 + k]);
+            g[k] = max(x[k], run);
+        }
     }
 };
 
@@ -218,9 +239,10 @@ __device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard
 // scores.  On entry rwin holds the records of the lane's first group (slot s1 - 1),
 // on return those of its second.
 template <int R>
-__device__ __forceinline__ int gate_chunk(const BandSmem<R>& sm, int s1, const char* col,
-                                          double4 (&rwin)[R], double (&qt)[R]) {
-    int top = INT_MIN;
+__device__ __forceinline__ int gate_chunk(const BandSmem<R>& sm, int s0, int s1, const char* col,
+                                          const int* cgate, double4 (&rwin)[R], double (&qt)[R]) {
+    int over = INT_MIN;
+    const int* gate = sm.gate + s0 * BandSmem<R>::kGateStride;
     const char* rec1 = sm.rec + s1 * BandSmem<R>::kRecStride;
     double4 cv = ring_rec(col);
 #pragma unroll
@@ -233,19 +255,38 @@ __device__ __forceinline__ int gate_chunk(const BandSmem<R>& sm, int s1, const c
             const double4 rv = rwin[(b + a) % R];
             // the window moves on: element b + R replaces element b
             if (a == 0) rwin[b] = ring_rec(rec1 + 32 * b);
-            // kernels.cpp:206-225
-            const double ss = __dmul_rn(rv.z, cv.z);
-            const double mm = __dmul_rn(cv.w, rv.w);
-            sc[a] = __fma_rn(qt[a], ss, -mm);
+            // score / s of the column; the running dot product is the reference's
+            // (kernels.cpp:206-225)
+            sc[a] = __fma_rn(-rv.w, cv.w, __dmul_rn(rv.z, qt[a]));
             qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
         }
-        cv = cn;
+        int top = 0;
         if (R == 1) top = max(top, __double2hiint(sc[0]));
 #pragma unroll
         for (int a = 0; a + 1 < R; a += 2)
             top = __vimax3_s32(top, __double2hiint(sc[a]), __double2hiint(sc[a + 1]));
+        top = fp64_gate_value(top, cv.z);
+        cv = cn;
+        over = __viaddmax_s32(top, gate[b], over);
+        over = __viaddmax_s32(top, cgate[b], over);
     }
-    return top;
+    return over;
+}
+
+// Whether a lane's pass with errors above the gates' slack opens (`over`: its largest
+// value over its gate).
+template <int R>
+__device__ __noinline__ int widen_gate(const BandSmem<R>& sm, int s0, const int* cgate, int err,
+                                       int over) {
+    constexpr int kU = BandSmem<R>::kU;
+    int g = cgate[0];
+#pragma unroll
+    for (int b = 1; b < kU * R; ++b) g = max(g, cgate[b]);
+#pragma unroll
+    for (int u = 0; u < kU; ++u)  // each covers R rows from its own on
+        g = max(g, sm.gate[BandSmem<R>::wrap(s0 + u) * BandSmem<R>::kGateStride]);
+    g = max(g, sm.gate[BandSmem<R>::wrap(s0 + kU - 1) * BandSmem<R>::kGateStride + R - 1]);
+    return fp64_gate_lowered(g, err, over) ? 0 : -1;
 }
 
 // A pass of kU chunks with the selection, s0 the slot of the lane's first group:
@@ -260,20 +301,22 @@ __device__ __forceinline__ int gate_chunk(const BandSmem<R>& sm, int s1, const c
 template <int R, bool EDGE>
 __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, unsigned jc,
                                             const BandSmem<R>& sm, int s0, const char* col,
-                                            const double* cthr, double (&qt)[R], int gate,
+                                            const double* cmean,
+                                            const int* cgate, double (&qt)[R],
                                             unsigned geo, int64_t gb, int lane) {
-    constexpr int RS = BandSmem<R>::kRecStride;
+    constexpr int RS = BandSmem<R>::kRecStride, kU = BandSmem<R>::kU;
     bool sel = false;
 #pragma unroll 1
     for (int b = 0; b < kU * R; ++b) {
         const unsigned j = jc + b;
         const int k = b % R;  // cell a lies in element k + a of the lane's groups
-        const int sa = wrap_group(s0 + b / R), sb = wrap_group(sa + 1);
+        const int sa = BandSmem<R>::wrap(s0 + b / R), sb = BandSmem<R>::wrap(sa + 1);
         const char* rec0 = sm.rec + sa * RS + 32 * k;
         const char* rec1 = sm.rec + sb * RS + 32 * (k - R);
         const double4 cv = ring_rec(col + 32 * b);
+        const double cw = cmean[b];
         double sc[R];
-        int top = INT_MIN;
+        int top = 0;
 #pragma unroll
         for (int a = 0; a < R; ++a) {
             const double4 rv = ring_rec((k + a < R ? rec0 : rec1) + 32 * a);
@@ -283,12 +326,13 @@ __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, 
             if (!EDGE || (code != 15u && left > 0)) {
                 const double ss = __dmul_rn(rv.z, cv.z);
                 if (!EDGE || (code != 7u && left >= 4 - (int)code)) {
-                    const double mm = __dmul_rn(cv.w, rv.w);
+                    // kernels.cpp:206-225
+                    const double mm = __dmul_rn(cw, rv.w);
                     score = __fma_rn(qt[a], ss, -mm);
                     qt[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, qt[a]));
                 } else {
                     // scalar remainder (kernels.cpp:282-289), no fusion
-                    score = __dsub_rn(__dmul_rn(qt[a], ss), __dmul_rn(rv.w, cv.w));
+                    score = __dsub_rn(__dmul_rn(qt[a], ss), __dmul_rn(rv.w, cw));
                     qt[a] = __dsub_rn(__dadd_rn(qt[a], __dmul_rn(rv.y, cv.y)),
                                       __dmul_rn(rv.x, cv.x));
                 }
@@ -296,8 +340,9 @@ __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, 
             sc[a] = score;
             top = max(top, __double2hiint(score));
         }
-        if (!EDGE && !__any_sync(kFullMask, top >= gate)) continue;
-        sel = true;
+        if (!EDGE &&
+            !__any_sync(kFullMask, top + max(sm.gate[sa * BandSmem<R>::kGateStride + k], cgate[b]) >= 0))
+            continue;
         __syncwarp();  // rows move from lane to lane between steps
         const int e0 = sa * (R + 1) + k, e1 = sb * (R + 1) + k - R;
         double best[R];
@@ -308,11 +353,12 @@ __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, 
             if (sc[a] > best[a]) {
                 sm.best[(k + a < R ? e0 : e1) + a] = sc[a];
                 sm.src[(k + a < R ? e0 : e1) + a] = (int)j;
+                sel = true;
             }
-        if (__any_sync(kFullMask, top >= fp64_gate(cthr[b])))
+        if (__any_sync(kFullMask, top + cgate[b] >= 0))
             select_column<R>(P, shard, j, sc, gb + lane * R, lane);
     }
-    return sel;
+    return __any_sync(kFullMask, sel);
 }
 
 // Columns [j0, jend) of a band.  lt: the tile's number when the band is cut into
@@ -321,7 +367,7 @@ template <int R>
 __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band, int64_t lt,
                                           int64_t seg, int lane, int shard,
                                           const BandSmem<R>& sm) {
-    constexpr int RS = BandSmem<R>::kRecStride;
+    constexpr int RS = BandSmem<R>::kRecStride, kU = BandSmem<R>::kU, kGroups = BandSmem<R>::kGroups;
     const int64_t gb = P.g_lo + band * (int64_t)(32 * R);
     const int64_t g0 = gb + (int64_t)lane * R;
     const int64_t jmax = P.Tbase - gb;  // length of the band's longest diagonal
@@ -342,49 +388,75 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     double qt[R];
     unsigned geo = 0;
     int minpsw = INT_MAX;
+    int64_t delta = (g0 - P.blk_origin) % P.B;
 #pragma unroll
     for (int a = 0; a < R; ++a) {
         const int64_t g = g0 + a;
         unsigned code = 15;
         qt[a] = -__longlong_as_double(0x7ff0000000000000ll);
         if (g < P.g_hi && (int64_t)j0 < P.Tbase - g) {
-            const int64_t delta = (g - P.blk_origin) % P.B;
             qt[a] = seg == 0 ? P.qt0[g - P.g_lo]
                              : P.split.seeds[(seg - 1) * (P.g_hi - P.g_lo) + (g - P.g_lo)];
             code = delta < (P.B & ~3ll) ? (unsigned)(delta & 3) : 7u;
             minpsw = min(minpsw, code == 7u ? -1 : (int)(P.Tbase - g) - 4 + (int)code);
         }
         geo |= code << (4 * a);
+        delta = delta + 1 == P.B ? 0 : delta + 1;
     }
     minpsw = __reduce_min_sync(kFullMask, minpsw);
 
-    // Groups 0 .. 32 + kU - 1 and the first pass's columns.  In a pass of kU
-    // chunks, lanes 0 - 15 bring in the next rows' thresholds, lanes 16 - 31 the
-    // next columns': part = lane % 16.
-    const int part = lane & 15;
-    const bool isrow = lane < 16;
+    // Groups 0 .. 32 + kU - 1 and the first pass's columns.  In a pass, lanes R to
+    // R + 15 bring in what belongs to the next 16 rows, the others to the next 16
+    // columns; part: which one.
+    static_assert(kU * R == 16, "half a warp each");
+    const bool isrow = lane >= R && lane < R + 16;
+    const int part = isrow ? lane - R : lane & 15;
     const uint4* rsrc = reinterpret_cast<const uint4*>(P.rowrec + rb);
     const uint4* crec = reinterpret_cast<const uint4*>(P.colrec + j0);
     const double* tsrc = P.thr + rb + P.row_key_off;  // threshold of row t
     const double* csrc = P.thr + j0 + P.col_key_off;  // threshold of column j0
+    const int64_t wlast = P.Tbase - 1;                // colgate ends there
+    const int errfree = fp64_gate_errfree(P.m);
     for (int i = lane; i < (32 + kU) * 2 * R; i += 32)
-        *reinterpret_cast<uint4*>(sm.rec + (i / (2 * R)) * RS + 16 * (i % (2 * R))) =
-            __ldg(rsrc + i);
-    for (int i = lane; i < (32 + kU) * R; i += 32) {
-        sm.best[(i / R) * (R + 1) + i % R] = ld_thr(tsrc + i);
-        sm.src[(i / R) * (R + 1) + i % R] = -1;
+        cp_async16(sm.rec + (i / (2 * R)) * RS + 16 * (i % (2 * R)), rsrc + i);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    constexpr int kOwn = (32 * R + 16 + 31) / 32;  // rows that a lane brings in
+    double thr[kOwn];
+    double2 sw[kOwn];
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {  // all in flight together (the last ones may be past the tile's)
+        thr[k] = ld_thr(tsrc + lane + 32 * k);
+        sw[k] = scale_mean(P.rowrec + rb + lane + 32 * k);
     }
-    if (lane < 2 * R * kU) *reinterpret_cast<uint4*>(sm.col + 16 * lane) = __ldg(crec + lane);
-    int cgate = INT_MAX;
+    int rerr = 0;  // one bound for all rows that the tile starts with
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {
+        const int i = lane + 32 * k;
+        if (i < (32 + kU) * R) {
+            sm.best[(i / R) * (R + 1) + i % R] = thr[k];
+            sm.src[(i / R) * (R + 1) + i % R] = -1;
+            rerr = max(rerr, fp64_gate_error(sw[k].x, sw[k].y));
+        }
+    }
+    rerr = __reduce_max_sync(kFullMask, rerr);
+    int cerr = 0;
     if (lane < R * kU) {
         const double t = ld_thr(csrc + lane);
-        sm.cthr[lane] = t;
-        cgate = fp64_gate(t);
+        const double2 sw = scale_mean(P.colrec + j0 + lane);
+        *reinterpret_cast<uint4*>(sm.col + 32 * lane) = __ldg(crec + 2 * lane);
+        *reinterpret_cast<double2*>(sm.col + 32 * lane + 16) =
+            make_double2(sw.x, __ldg(P.colgate + min((int64_t)j0 + lane, wlast)));
+        sm.cmean[lane] = sw.y;
+        sm.cgate[lane] = fp64_gate(t, P.m);
+        cerr = fp64_gate_error(sw.x, sw.y);
     }
-    cgate = __reduce_min_sync(kFullMask, cgate);
+    cerr = __reduce_max_sync(kFullMask, cerr);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncwarp();
-    sm.gate[lane] = sm.group_gate(lane);
-    if (lane < kU) sm.gate[32 + lane] = sm.group_gate(32 + lane);
+    for (int s = lane; s + 1 < 32 + kU; s += 32) sm.group_gates(s, P.m);
+    if (lane < kGroups / kU) sm.err[lane] = rerr;
+    // lanes 0 to R - 1: gates of the last group brought in
+    int lastg = fp64_gate(sm.best[(32 + kU - 1) * (R + 1) + lane % R], P.m);
     __syncwarp();
     // register window of row records: slot (k mod R) holds element k of the
     // lane's first group
@@ -395,40 +467,45 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     // what the lane copies in next: records of groups c + 32 + kU .. and of the
     // next pass's columns, and their thresholds
     const uint4* nrow = rsrc + (32 + kU) * 2 * R + lane;
-    const uint4* ncol = crec + kU * 2 * R + lane;
     const double* nthr = isrow ? tsrc + (32 + kU) * R + part : csrc + kU * R + part;
+    const double4* nrec = isrow ? P.rowrec + rb + (32 + kU) * R + part : P.colrec + j0 + kU * R + part;
+    int64_t nw = (int64_t)j0 + kU * R + part;  // its index in colgate (columns)
     int s0 = lane;  // slot of the lane's first group
     int sf = 0;     // slot of group c, the first that the pass finishes
     int cbuf = 0;
     bool sel = false;
     for (unsigned jc = j0; jc < jend; jc += kU * R) {
-        const int sn = wrap_group(sf + 32 + kU);  // slots of the incoming groups (kU divides kGroups)
-        double t = 0.0;
-        if (lane < 2 * R * kU) {
-            cp_async16(sm.rec + (sn + lane / (2 * R)) * RS + 16 * (lane % (2 * R)), nrow);
-            cp_async16(sm.col + (cbuf ^ 1) * (32 * R * kU) + 16 * lane, ncol);
+        const int sn = BandSmem<R>::wrap(sf + 32 + kU);  // slots of the incoming groups (kU divides kGroups)
+        double w = 0.0;
+        cp_async16(sm.rec + (sn + lane / (2 * R)) * RS + 16 * (lane % (2 * R)), nrow);
+        const double t = ld_thr(nthr);
+        const double2 sw = scale_mean(nrec);
+        if (!isrow) {
+            w = __ldg(P.colgate + min(nw, wlast));
+            cp_async16(sm.col + (cbuf ^ 1) * (32 * R * kU) + 32 * part, nrec);
         }
-        if (part < R * kU) t = ld_thr(nthr);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         nrow += kU * 2 * R;
-        ncol += kU * 2 * R;
         nthr += kU * R;
-        int gate = cgate;
-#pragma unroll
-        for (int u = 0; u <= kU; ++u) gate = min(gate, sm.gate[wrap_group(s0 + u)]);
+        nrec += kU * R;
+        nw += kU * R;
         const char* col = sm.col + cbuf * (32 * R * kU);
-        const double* cthr = sm.cthr + cbuf * (R * kU);
+        const int* cgate = sm.cgate + cbuf * (R * kU);
+        const double* cmean = sm.cmean + cbuf * (R * kU);
         const bool fused = (int64_t)jc + (kU * R - 1) <= minpsw;
         bool open = !fused || sel;  // a pass after one that selected goes straight to selecting
         if (!open) {
             double q0[R];
 #pragma unroll
             for (int a = 0; a < R; ++a) q0[a] = qt[a];
-            int top = INT_MIN;
+            int over = INT_MIN;
+            const int err = max(cerr, max(sm.err[s0 / kU], sm.err[BandSmem<R>::wrap(s0 + kU) / kU]));
 #pragma unroll
             for (int u = 0; u < kU; ++u)
-                top = max(top, gate_chunk<R>(sm, wrap_group(s0 + u + 1), col + u * 32 * R, rwin, qt));
-            open = __any_sync(kFullMask, top >= gate);
+                over = max(over, gate_chunk<R>(sm, BandSmem<R>::wrap(s0 + u), BandSmem<R>::wrap(s0 + u + 1),
+                                               col + u * 32 * R, cgate + u * R, rwin, qt));
+            if (err > errfree) over = widen_gate<R>(sm, s0, cgate, err, over);
+            open = __any_sync(kFullMask, over >= 0);
             if (open) {
 #pragma unroll
                 for (int a = 0; a < R; ++a) qt[a] = q0[a];
@@ -436,9 +513,9 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         }
         sel = false;
         if (open) {
-            sel = fused ? select_pass<R, false>(P, shard, jc, sm, s0, col, cthr, qt, gate, geo, gb, lane)
-                        : select_pass<R, true>(P, shard, jc, sm, s0, col, cthr, qt, gate, geo, gb, lane);
-            const char* r0 = sm.rec + wrap_group(s0 + kU) * RS;
+            sel = fused ? select_pass<R, false>(P, shard, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane)
+                        : select_pass<R, true>(P, shard, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane);
+            const char* r0 = sm.rec + BandSmem<R>::wrap(s0 + kU) * RS;
 #pragma unroll
             for (int a = 0; a < R; ++a) rwin[a] = ring_rec(r0 + 32 * a);
         }
@@ -450,34 +527,46 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
             finish_row<R>(P, shard, lt, seg, more, rb, (int64_t)(jc - j0) + lane, sm.best[e], j);
         }
         // the incoming groups and columns begin at their thresholds
-        if (part < R * kU) {
-            if (isrow) {
-                const int e = (sn + part / R) * (R + 1) + part % R;
-                sm.best[e] = t;
-                sm.src[e] = -1;
-            } else {
-                sm.cthr[(cbuf ^ 1) * (R * kU) + part] = t;
-            }
+        const int x = fp64_gate(t, P.m);
+        if (isrow) {
+            const int e = (sn + part / R) * (R + 1) + part % R;
+            sm.best[e] = t;
+            sm.src[e] = -1;
+        } else {
+            *reinterpret_cast<double2*>(sm.col + (cbuf ^ 1) * (32 * R * kU) + 32 * part + 16) =
+                make_double2(sw.x, w);
+            sm.cmean[(cbuf ^ 1) * (R * kU) + part] = sw.y;
+            sm.cgate[(cbuf ^ 1) * (R * kU) + part] = x;
         }
-        const int x = part < R * kU ? fp64_gate(t) : INT_MAX;
+        // one bound of the errors for the rows and the columns
+        cerr = __reduce_max_sync(kFullMask, fp64_gate_error(sw.x, sw.y));
+        if (lane == 0) sm.err[sn / kU] = cerr;
+        // gates of the last incoming group of the pass before (its rows' minima reach
+        // into this one's) and of all but the last of this one's: its rows are in
+        // lanes 0 to R - 1, this one's follow
+        int win = lane < R ? lastg : isrow ? x : INT_MIN;
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int g = __reduce_min_sync(kFullMask, isrow && part / R == u ? x : INT_MAX);
-            if (lane == 0) sm.gate[sn + u] = g;
+        for (int d = 1; d < R; d *= 2) win = max(win, __shfl_down_sync(kFullMask, win, d));
+        if (lane < kU * R) {
+            const int s = lane < R ? (sn == 0 ? kGroups : sn) - 1 : sn + lane / R - 1;
+            sm.gate[s * BandSmem<R>::kGateStride + lane % R] = win;
         }
-        cgate = __reduce_min_sync(kFullMask, isrow ? INT_MAX : x);
-        s0 = wrap_group(s0 + kU);
-        if (sel) sm.gate[s0] = sm.group_gate(s0);  // best scores of groups c + kU .. c + kU + 31 rose
+        lastg = __shfl_sync(kFullMask, x, (lane + 16) & 31);
+        s0 = BandSmem<R>::wrap(s0 + kU);
+        if (sel) {  // best scores of groups c + kU .. c + kU + 31 rose
+            __syncwarp();
+            sm.group_gates(s0, P.m);
+        }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncwarp();
-        sf = wrap_group(sf + kU);
+        sf = BandSmem<R>::wrap(sf + kU);
         cbuf ^= 1;
     }
 
     // drain: rows of groups c .. c + 31 (the last chunk's second groups)
     const int64_t tend = ((int64_t)(jend - j0) + kU * R - 1) / (kU * R) * (kU * R);  // row t of group c
     for (int i = lane; i < 32 * R; i += 32) {
-        const int e = wrap_group(sf + i / R) * (R + 1) + i % R;
+        const int e = BandSmem<R>::wrap(sf + i / R) * (R + 1) + i % R;
         const int j = sm.src[e];
         finish_row<R>(P, shard, lt, seg, more, rb, tend + i, sm.best[e], j);
     }

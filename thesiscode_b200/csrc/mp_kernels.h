@@ -2,10 +2,12 @@
 // translation units (device code and the C-ABI layer).
 #pragma once
 
+#include <float.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <cmath>
+#include <cstring>
 
 struct mp_context;
 
@@ -23,7 +25,7 @@ __global__ void ref_stats_kernel(const double* cs, const double* cs2, int64_t PL
                                  double* muS, double* sInv);
 __global__ void first_qt_kernel(const double* A, int64_t m, int64_t d_lo, int64_t d_hi,
                                 double* qt);
-__global__ void pack_fp64_kernel(const double* Apad, int64_t m, int64_t count, const double* sInv,
+__global__ void pack_fp64_kernel(const double* Apad, int64_t m, int64_t count, double* sInv,
                                  const double* muS, double4* rec);
 __global__ void change_flags_kernel(const double* A, int64_t n, int* chg);
 __global__ void scan_blocks_kernel(int* x, int64_t n, int* block_tot);
@@ -82,9 +84,95 @@ __host__ __device__ inline bool tile_of_pair(int64_t lt, int64_t PL, int64_t g_l
     seg = s;
     return s < nseg1;
 }
+// The gate's tests are integer ones, on high words: those of non-negative doubles order
+// like the doubles.  (Host-callable, so the rule can be checked without a GPU.)
+__host__ __device__ inline int high_word(double x) {
+#ifdef __CUDA_ARCH__
+    return __double2hiint(x);
+#else
+    int64_t b;
+    std::memcpy(&b, &x, 8);
+    return (int)(b >> 32);
+#endif
+}
+__host__ __device__ inline double from_words(int hi, int lo) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(hi, lo);
+#else
+    const int64_t b = (int64_t)(((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo);
+    double x;
+    std::memcpy(&x, &b, 8);
+    return x;
+#endif
+}
+// A window's scale s = 1 / deviation and mean term w for which s, its products and
+// quotients with w stay far from the ends of a double's range (a small w may vanish:
+// what it adds lies below the gates' slack).
+__host__ __device__ inline bool fp64_ordinary(double s, double w) {
+    return (unsigned)(high_word(s) - ((1023 - 450) << 20)) < (unsigned)(900 << 20) &&
+           (high_word(w) & 0x7fffffff) < ((1023 + 200) << 20);
+}
+// A constant window with a mean: s = +inf, w = +-inf.
+__host__ __device__ inline bool fp64_flat(double s, double w) {
+    return s > DBL_MAX && (w > DBL_MAX || w < -DBL_MAX);
+}
+// A column's mean term in the FP64 join's gate, which tests s' (q s - w W') in place of
+// the score q (s s') - w w': W' = w' / s'.  A constant column's scores are -inf, NaN, or
+// +inf where w w' < 0; with the largest double as W' the gate's value is positive there.
+__host__ __device__ inline double fp64_gate_mean(double s, double w) {
+    if (fp64_ordinary(s, w)) return w / s;
+    if (fp64_flat(s, w)) return w > 0.0 ? DBL_MAX : -DBL_MAX;
+    return w != w ? w : 0.0;  // the gate stands open (fp64_gate_error), or the score is NaN
+}
+// A bound's gate: minus the high word of a value below it by more than the rounding
+// of the gate's values (kFp64GateSlack m, and 2^-34 of the bound).  A negative bound, or
+// one so large that a product may leave the range of doubles, lets every cell through.
+constexpr double kFp64GateSlack = 0x1p-25;
+constexpr int kFp64GateEnd = (1023 + 500) << 20;
+__host__ __device__ inline int fp64_gate(double bound, double m) {
+    const int h = high_word(fma(bound, 1.0 - 0x1p-34, -kFp64GateSlack * m));
+    return h < kFp64GateEnd && h > 0 ? -h : 0;
+}
+// The same from the bound's high word h alone, a unit lower: from m / 16 on a unit is
+// more than the slack.
+__host__ __device__ inline int fp64_gate_high_from(double m) { return high_word(m * 0x1p-4) + 1; }
+__host__ __device__ inline int fp64_gate_high(int h, int from) {
+    return h >= from && h < kFp64GateEnd ? 1 - h : 0;
+}
+// High word of the gate's value, from the largest high word among a column's
+// q s - w W' (0 if all are negative): rounded up, an infinity or NaN as the largest
+// double.  The cell passes if the sum with its bound's gate is not negative.
+__host__ __device__ inline int fp64_gate_value(int top, double s) {
+    return high_word(from_words(top < 0x7fefffff ? top : 0x7fefffff, -1) * s);
+}
+// What the gate's value may lie below a cell's score because of a window with scale s
+// and mean term w, as the high word of an upper bound; an infinite one lets every cell
+// through.  With u = 2^-53, the score is off its exact value S by 2u|S| + 2u|w w'|,
+// the gate's value by 3u|S| + 2u|w w'|; |w w'| <= (w^2 + w'^2) / 2 parts the rounding
+// of the mean terms between the two windows, 2^-51 w^2 for each with room.
+__host__ __device__ inline int fp64_gate_error(double s, double w) {
+    if (fp64_ordinary(s, w)) {
+        const int h = high_word(w * w) + 1 - (51 << 20);
+        return h > 0 ? h : 0;
+    }
+    // NaN never selects; infinite terms give the score's own infinities and NaN
+    return s != s || w != w || fp64_flat(s, w) ? 0 : 0x7ff00000;
+}
+// Errors up to here are within the gates' slack.
+__host__ __device__ inline int fp64_gate_errfree(double m) { return high_word(kFp64GateSlack / 8 * m); }
+// For larger ones (err: the larger of a pass's rows' and columns'): whether the largest
+// value over its gate lets the pass open when every gate lies lower by the units that
+// take the smallest bound (gate g) below it by both errors; the units of larger bounds
+// are at least as wide.
+__host__ __device__ inline bool fp64_gate_lowered(int g, int err, int over) {
+    if (err >= 0x7ff00000) return true;
+    const int h = high_word(from_words(-g, 0) - 2.0 * from_words(err, 0));
+    return h <= 0 || over >= h + g - 1;
+}
 struct Fp64BandParams {
     const double4* colrec;  // colrec[j] = {A_hor[j], A_hor[j+m], s_hor[j], mu_hor[j]}
     const double4* rowrec;  // rowrec[r] = {A_vert[r], A_vert[r+m], s_vert[r], mu_vert[r]}
+    const double* colgate;  // colgate[j] = fp64_gate_mean(s_hor[j], mu_hor[j]), Tbase values
     const double* qt0;      // qt0[g - g_lo]: running dot product at j = 0
     double* qt_out;         // optional: dot product after the last cell, per diagonal
     int64_t g_lo, g_hi, nbands;

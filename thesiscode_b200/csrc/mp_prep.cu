@@ -156,15 +156,18 @@ __global__ void first_qt_kernel(const double* __restrict__ A, int64_t m, int64_t
     }
 }
 
-// Row/column record of the FP64 join: {A[i], A[i+m], sInv[i], muS[i]}.
+// Row/column record of the FP64 join: {A[i], A[i+m], sInv[i], muS[i]}; sInv[i], no
+// longer needed, becomes Fp64BandParams::colgate.
 // `Apad` holds n+1 values (A[n] = 0 feeds only the update after a diagonal's
 // last cell, whose result is never used).
 __global__ void pack_fp64_kernel(const double* __restrict__ Apad, int64_t m, int64_t count,
-                                 const double* __restrict__ sInv, const double* __restrict__ muS,
+                                 double* __restrict__ sInv, const double* __restrict__ muS,
                                  double4* __restrict__ rec) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
          i += (int64_t)gridDim.x * blockDim.x) {
-        rec[i] = make_double4(Apad[i], Apad[i + m], sInv[i], muS[i]);
+        const double s = sInv[i];
+        sInv[i] = fp64_gate_mean(s, muS[i]);
+        rec[i] = make_double4(Apad[i], Apad[i + m], s, muS[i]);
     }
 }
 
