@@ -667,7 +667,7 @@ __device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, in
     if (P.hazard && fp32_tile_hazardous(P, gb, j0, j1, 32 * R)) return;
     const float ulim = (float)(1.0 + 1.0 / (double)P.m);
     const unsigned ulim_ord = ord_f32(ulim);
-    // extents of the tile's cells, as in tile_fp32
+    // extents of the tile's cells, as in tile_dense
     const int ncols = (int)(j1 - j0);
     const int lim0 = (int)min(P.PL - g0 - j0, (int64_t)ncols + R);
     const int ghi_rel = (int)max(min(P.g_hi - g0, (int64_t)R), (int64_t)0);
