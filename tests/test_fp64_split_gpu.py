@@ -65,3 +65,14 @@ def test_block_in_tiles_equals_whole_bands(gpu_ctx, blocklen, diag):
             got.append((prof, idx, tq))
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+# The series' prefix sums run beside the tiles' first columns, in chunks of 192 values,
+# 16 ahead; the first chunk starts at its second round.
+@pytest.mark.parametrize("n", [191, 192, 193, 207, 208, 209, 383, 384, 385, 400, 577])
+def test_prefix_sums_beside_the_tiles_equal_oracle(gpu_ctx, oracle, n):
+    x, m = series("walk", n) + 40.0, 8
+    p = gpu_ctx.selfjoin(x, m)
+    d2, idx = oracle.selfjoin(x, m)
+    assert np.array_equal(p.dist2, d2)
+    check_fp64_indices(oracle, x, m, p.dist2, p.index, idx)

@@ -430,10 +430,6 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
                                                            : cudaMemcpyHostToDevice, st));
         mark(ctx, 0, st);
         MP_CUDA(ctx, cudaMemsetAsync(Apad + n, 0, 8, st));
-        ref_prefix_kernel<<<1, kPrefixThreads, 0, st>>>(Apad, n, cs, cs2);
-        MP_LAUNCHED(ctx);
-        ref_stats_kernel<<<grid_for(PL), kThreads, 0, st>>>(cs, cs2, PL, m, muS, sInv);
-        MP_LAUNCHED(ctx);
         {
             int64_t off = 0;
             for (const DiagRange& r : ranges) {
@@ -443,17 +439,8 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
                 off += r.hi - r.lo;
             }
         }
-        MP_CUDA(ctx, cudaMemsetAsync(rec + PL, 0, 32 * kFp64Pad, st));
-        pack_fp64_kernel<<<grid_for(PL), kThreads, 0, st>>>(Apad, m, PL, sInv, muS, rec);
-        MP_LAUNCHED(ctx);
-        MP_CUDA(ctx, cudaMemsetAsync(kex, 0, 8 * (size_t)PL * shards, st));
-        MP_CUDA(ctx, cudaMemsetAsync(kid, 0, 8 * (size_t)PL * shards, st));
-        init_keys_kernel<<<grid_for(PL + kFp64ThrPad), kThreads, 0, st>>>(
-            reinterpret_cast<unsigned long long*>(thr), PL + kFp64ThrPad, no_threshold_bits());
-        MP_LAUNCHED(ctx);
-        mark(ctx, 1, st);
-        int64_t qoff = 0;
-        for (const DiagRange& r : ranges) {
+        auto params = [&](size_t i, int64_t qoff) {
+            const DiagRange& r = ranges[i];
             Fp64BandParams P{};
             const int64_t nd = r.hi - r.lo;
             const int R = pick_fp64_R(nd);
@@ -461,7 +448,6 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             P.rowrec = rec;
             P.colgate = sInv;
             P.qt0 = qt0 + qoff;
-            qoff += nd;
             P.qt_out = nullptr;
             P.g_lo = r.lo;
             P.g_hi = r.hi;
@@ -481,14 +467,49 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             P.thr_eps = fp64_threshold_eps(P.idx_bits);
             P.thr_tiny = fp64_threshold_tiny(P.m);
             P.counter = counter;
-            if (split && splits[&r - ranges.data()].L > 0) {
-                P.split = splits[&r - ranges.data()];
+            if (split && splits[i].L > 0) {
+                P.split = splits[i];
                 fp64_split_carve(P.split, nd, R, (char*)ctx->arena + align_up(base));
-                launch_fp64_seeds(P, Apad, n + 1, Apad, n + 1, m, st);
-                MP_LAUNCHED(ctx);
+            }
+            return P;
+        };
+        // The prefix sums run beside the first tiled range's seeds; the other ranges' seeds
+        // follow in their turn (one buffer serves them all).
+        size_t first = 0;
+        int64_t qfirst = 0;
+        while (first < ranges.size() && !(split && splits[first].L > 0)) {
+            qfirst += ranges[first].hi - ranges[first].lo;
+            ++first;
+        }
+        if (first < ranges.size())
+            launch_fp64_seeds(params(first, qfirst), Apad, n + 1, Apad, n + 1, m,
+                              PrefixSums{Apad, n, cs, cs2}, st);
+        else
+            ref_prefix_kernel<<<1, kPrefixThreads, 0, st>>>(Apad, n, cs, cs2);
+        MP_LAUNCHED(ctx);
+        ref_stats_kernel<<<grid_for(PL), kThreads, 0, st>>>(cs, cs2, PL, m, muS, sInv);
+        MP_LAUNCHED(ctx);
+        MP_CUDA(ctx, cudaMemsetAsync(rec + PL, 0, 32 * kFp64Pad, st));
+        pack_fp64_kernel<<<grid_for(PL), kThreads, 0, st>>>(Apad, m, PL, sInv, muS, rec);
+        MP_LAUNCHED(ctx);
+        MP_CUDA(ctx, cudaMemsetAsync(kex, 0, 8 * (size_t)PL * shards, st));
+        MP_CUDA(ctx, cudaMemsetAsync(kid, 0, 8 * (size_t)PL * shards, st));
+        init_keys_kernel<<<grid_for(PL + kFp64ThrPad), kThreads, 0, st>>>(
+            reinterpret_cast<unsigned long long*>(thr), PL + kFp64ThrPad, no_threshold_bits());
+        MP_LAUNCHED(ctx);
+        mark(ctx, 1, st);
+        int64_t qoff = 0;
+        for (size_t i = 0; i < ranges.size(); ++i) {
+            const Fp64BandParams P = params(i, qoff);
+            qoff += P.g_hi - P.g_lo;
+            if (P.split.L > 0) {
+                if (i != first) {  // the first one's are there
+                    launch_fp64_seeds(P, Apad, n + 1, Apad, n + 1, m, PrefixSums{}, st);
+                    MP_LAUNCHED(ctx);
+                }
                 ++ctx->launches;  // the rows that two tiles meet
             }
-            launch_band(R, P, st);
+            launch_band(pick_fp64_R(P.g_hi - P.g_lo), P, st);
             MP_LAUNCHED(ctx);
         }
         mark(ctx, 2, st);
@@ -971,7 +992,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     if (has_split) {
         P.split = split;
         fp64_split_carve(P.split, nq, R, (char*)ctx->arena + align_up(need));
-        launch_fp64_seeds(P, ah, T + m, av, T + m, m, st);
+        launch_fp64_seeds(P, ah, T + m, av, T + m, m, PrefixSums{}, st);
         MP_LAUNCHED(ctx);
         ++ctx->launches;  // the rows that two tiles meet
     }

@@ -233,8 +233,14 @@ void fp64_split_carve(Fp64Split& S, int64_t ndiag, int R, char* base);
 // Running dot products at the tiles' first columns: Ah the series along columns,
 // Av along rows (nh and nv values; zero is read past them), P.qt0 the dot products
 // at column 0.
+// X.n > 0: one more block takes the reference-order prefix sums of X.A.
+struct PrefixSums {
+    const double* A;
+    int64_t n;
+    double *cs, *cs2;
+};
 void launch_fp64_seeds(const Fp64BandParams& P, const double* Ah, int64_t nh, const double* Av,
-                       int64_t nv, int64_t m, cudaStream_t s);
+                       int64_t nv, int64_t m, const PrefixSums& X, cudaStream_t s);
 
 // ---- FP32 re-anchored tile join (mp_join_fp32.cu) ---------------------------
 // One series of a (batched) join.  Its tiles are numbered

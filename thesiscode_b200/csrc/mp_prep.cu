@@ -21,106 +21,11 @@ namespace mpgpu {
 
 // ---- reference-exact statistics -------------------------------------------
 
-// cs[i] = A[i] + cs[i-1], cs2[i] = A[i]*A[i] + cs2[i-1] in index order
-// (ScrimpSequOpt.cpp:43-49).  Each chain is inherently serial, 8 cycles per
-// addition (4.3 ms for n = 1M), so one lane of warp 0 and one of warp 1 do nothing
-// else, out of shared memory and 16 values ahead: the block's other warps load the
-// next chunk of A, square it and write the previous chunk's sums back (all coalesced)
-// meanwhile.  n = 1,048,576: 5.4 ms; 8.8 with both chains on two lanes of one
-// warp, which squared and selected between the additions.  Launch with kPrefixThreads
-// threads in one block.
-__device__ __forceinline__ double prefix_chain(const double* src, double* dst, int cnt, double acc) {
-    constexpr int U = 16;
-    double2 v[U / 2];
-    int k = 0;
-    if (cnt >= U) {
-#pragma unroll
-        for (int i = 0; i < U / 2; ++i) v[i] = reinterpret_cast<const double2*>(src)[i];
-    }
-    for (; k + U <= cnt; k += U) {
-        // values of the next round (past the chunk: read from the array's padding, unused)
-        double2 w[U / 2];
-#pragma unroll
-        for (int i = 0; i < U / 2; ++i) {
-            const double2 x = v[i];
-            w[i] = reinterpret_cast<const double2*>(src + k + U)[i];
-            double2 o;
-            o.x = __dadd_rn(x.x, acc);
-            o.y = __dadd_rn(x.y, o.x);
-            acc = o.y;
-            reinterpret_cast<double2*>(dst + k)[i] = o;
-        }
-#pragma unroll
-        for (int i = 0; i < U / 2; ++i) v[i] = w[i];
-    }
-    for (; k < cnt; ++k) {
-        acc = __dadd_rn(src[k], acc);
-        dst[k] = acc;
-    }
-    return acc;
-}
 __global__ void __launch_bounds__(kPrefixThreads)
     ref_prefix_kernel(const double* __restrict__ A, int64_t n, double* __restrict__ cs,
                       double* __restrict__ cs2) {
-    constexpr int C = kPrefixChunk;
-    // [chain][buffer][k]: chain 0 takes A, chain 1 takes A*A
-    __shared__ __align__(16) double in[2][2][C + 16];
-    __shared__ __align__(16) double out[2][2][C];
-    if (blockIdx.x != 0) return;
-    const int t = threadIdx.x;
-    const int64_t nch = (n + C - 1) / C;
-    for (int k = t; k < C; k += blockDim.x) {
-        const double a = k < n ? A[k] : 0.0;
-        in[0][0][k] = a;
-        in[1][0][k] = __dmul_rn(a, a);
-    }
-    __syncthreads();
-    double acc = 0.0;
-    for (int64_t c = 0; c < nch; ++c) {
-        const int b = (int)(c & 1);
-        const int cnt = (int)min((int64_t)C, n - c * C);
-        if (t < 64) {
-            if ((t & 31) == 0) {
-                const int h = t >> 5;
-                if (c == 0) {  // the first sum is the first value itself
-                    acc = in[h][0][0];
-                    out[h][0][0] = acc;
-                    int k = 1;
-                    for (; k < cnt && k < 16; ++k) {
-                        acc = __dadd_rn(in[h][0][k], acc);
-                        out[h][0][k] = acc;
-                    }
-                    if (cnt > 16) acc = prefix_chain(in[h][0] + 16, out[h][0] + 16, cnt - 16, acc);
-                } else {
-                    acc = prefix_chain(in[h][b], out[h][b], cnt, acc);
-                }
-            }
-        } else {
-            const int tt = t - 64, nt = blockDim.x - 64;
-            if (c + 1 < nch)
-                for (int k = tt; k < C; k += nt) {
-                    const int64_t i = (c + 1) * C + k;
-                    const double a = i < n ? A[i] : 0.0;
-                    in[0][b ^ 1][k] = a;
-                    in[1][b ^ 1][k] = __dmul_rn(a, a);
-                }
-            if (c >= 1)
-                for (int k = tt; k < C; k += nt) {
-                    const int64_t i = (c - 1) * C + k;
-                    cs[i] = out[0][b ^ 1][k];
-                    cs2[i] = out[1][b ^ 1][k];
-                }
-        }
-        __syncthreads();
-    }
-    const int64_t c = nch - 1;
-    for (int k = t; k < C; k += blockDim.x) {
-        const int64_t i = c * C + k;
-        if (i < n) {
-            cs[i] = out[0][c & 1][k];
-            cs2[i] = out[1][c & 1][k];
-        }
-    }
+    __shared__ __align__(16) char buf[PrefixSmem<kPrefixChunk>::kBytes];
+    if (blockIdx.x == 0) prefix_block<kPrefixChunk>(A, n, cs, cs2, buf);
 }
 
 // Window sums from prefix differences, mean = S/m, var = S2/m - mean^2,
