@@ -848,14 +848,15 @@ Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R) {
     const int64_t nbands = (nd + span - 1) / span;
     // Whole bands keep the chip busy once there are about as many as resident
     // warps (8 per SM), and the dot products of the tiles' first columns cost two
-    // more FP64 operations per cell.  Join phase, tiles against whole bands: n =
-    // 2,500 0.11 / 0.83 ms; 16,384 0.57 / 2.2; 65,536 (256 bands) 2.8 / 6.6;
-    // 200,000 (780 bands) 17.1 / 19.5; 260,000 (1,015) 27.5 / 26.8; 300,000 36 / 31.
+    // more FP64 operations per cell.  Whole calls, tiles against whole bands: n =
+    // 2,500 0.14 / 1.0 ms; 16,384 0.64 / 2.7; 65,536 (256 bands) 2.8 / 6.8;
+    // 200,000 (780 bands) 15.8 / 19.5; 260,000 (1,015) 25.5 / 26.5; 300,000 33.5 / 31.3.
     const int64_t warps = (int64_t)sm_count() * 8;
     if (nbands > warps * 4 / 5) return S;
-    // About 5 tiles per warp (10 and 20 measured the same); at least 32 columns,
-    // for the smallest series, whose tiles are all resident at once (n = 2,500:
-    // 32 columns 0.105 ms, 64 0.127, 256 0.26).
+    // About 5 tiles per warp (10 and 20 measured the same; 2 per warp 16.8 ms at n =
+    // 200,000, bands in 4 parts 16.4); at least 32 columns, for the smallest series,
+    // whose tiles are all resident at once (n = 2,500: 32 columns 0.105 ms, 64 0.127,
+    // 256 0.26).
     const int64_t cols = nbands * (Tbase - g_lo) - span * (nbands * (nbands - 1) / 2);
     int64_t L = std::max<int64_t>(cols / (5 * warps), 32);
     L = (L + kFp64SplitUnit - 1) / kFp64SplitUnit * kFp64SplitUnit;
