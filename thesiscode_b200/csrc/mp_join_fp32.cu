@@ -46,7 +46,7 @@
 // with three different operands takes the register file 1.5 cycles (measured;
 // packed f32x2 pairs cost the same words, their pair records twice the
 // shared-memory bandwidth, and minima in place of sign bits three cycles each).
-// n = 1,048,576, m = 256, K = 1024: 128 ms (100 the columns, 10 the passes' ends, 8
+// n = 1,048,576, m = 256, K = 1024: 127 ms (100 the columns, 10 the passes' ends, 8
 // passes evaluated again, the rest anchors), 178 ms with every pass selecting,
 // which stays the better way for short windows and short series (fp32_gate_pays).
 //
