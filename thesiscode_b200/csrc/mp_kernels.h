@@ -380,14 +380,14 @@ void launch_fp32_join(const Fp32TileParams* series_dev, int nseries, int64_t tot
 // candidates, each time over a run of lags that grows shorter with the window; the
 // gate opens for the loosest of 24 rows and 16 columns, which lie further apart
 // with short windows.  Random walks, K = 1024, gate / every pass selecting (ms):
-//   m = 64    n = 500,000 50.2 / 39.0
-//   m = 128   262,144 11.1 / 10.9     500,000 37.8 / 39.5
-//   m = 192   65,536 0.81 / 0.75      131,072 2.71 / 2.83     500,000 32.5 / 40.1
-//   m = 256   65,536 0.77 / 0.76      131,072 2.53 / 2.86     500,000 30.8 / 40.5
-//   m = 400   32,768 0.28 / 0.28      65,536 0.75 / 0.79      500,000 31.0 / 41.9
-//   m = 1024  16,384 0.16 / 0.12      32,768 0.27 / 0.30      500,000 35.8 / 47.4
+//   m = 64    n = 500,000 41.9 / 39.0
+//   m = 96    262,144 10.2 / 10.8     500,000 35.4 / 39.1
+//   m = 128   65,536 0.76 / 0.73      131,072 2.48 / 2.76     500,000 32.1 / 39.3
+//   m = 160   32,768 0.25 / 0.26      65,536 0.71 / 0.73      262,144 8.7 / 10.9
+//   m = 256   16,384 0.12 / 0.10      32,768 0.24 / 0.30      131,072 2.19 / 2.80
+//   m = 1024  16,384 0.13 / 0.11      32,768 0.25 / 0.29
 __host__ __device__ inline bool fp32_gate_pays(int64_t m, int64_t PL) {
-    return (m >= 160 && m * PL >= 25000000) || (m >= 128 && PL >= 400000);
+    return m >= 96 && PL >= (m >= 160 ? 25000 : m >= 128 ? 90000 : 200000);
 }
 // The way of a launch over these series.
 inline Fp32Way fp32_way_of(const Fp32TileParams* P, size_t n) {
