@@ -1,0 +1,44 @@
+"""Index arithmetic of the tile kernels beyond 32-bit counts (host programs against the
+kernels' headers; sizes that no test could run)."""
+from __future__ import annotations
+
+import subprocess
+
+from thesiscode_b200 import build
+
+HEAD = r"""
+#include <cstdint>
+#include <cstdio>
+#include "mp_common.cuh"
+#include "mp_kernels.h"
+#include "mp_tile.cuh"
+using namespace mpgpu;
+"""
+
+# An anchor's 32-bit term count is the window's, or 0 (the plain way, which counts in 64
+# bits), and the stages' positions past it stay in range.
+ANCHOR = HEAD + r"""
+int main() {
+    int bad = 0;
+    const long long e = 1ll << 31;
+    for (const long long m : {2ll, 1000ll, e / 2 - 1, e / 2, e - 264, e - 8, e - 7, e, e + 5, 2 * e, 2 * e + 9, 1ll << 40}) {
+        const int64_t terms = anchor_terms(m);
+        const bool ok = terms == 0 ? m > 100000000 : terms == m + 7 && terms + 3 * kAnchorStep < e;
+        if (!ok) std::printf("m %lld: %lld terms\n", m, (long long)terms);
+        bad += !ok;
+    }
+    return bad;
+}
+"""
+
+
+def run(tmp_path, program):
+    src, exe = tmp_path / "index.cu", tmp_path / "index"
+    src.write_text(program)
+    subprocess.run([build.NVCC, *build.NVCC_FLAGS, str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_anchor_of_a_window_beyond_32_bits(tmp_path):
+    run(tmp_path, ANCHOR)
