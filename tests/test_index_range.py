@@ -31,6 +31,21 @@ int main() {
 }
 """
 
+# Records a re-anchor interval of 2^28 columns or more away, from a tile's first.
+RECORD = HEAD + r"""
+int main() {
+    int bad = 0;
+    const long long far = 1ll << 28;
+    for (const long long c : {0ll, 1000ll, far - 16, far, far + 304, 4 * far, 8 * far - 32}) {
+        const int jr = (int)c;  // the tile's column count is a 32-bit one
+        const uintptr_t base = 1ull << 40;
+        const uintptr_t got = (uintptr_t)fp32_record((const float*)base, jr + 16);
+        bad += got - base != (uintptr_t)(32 * (c + 16));
+    }
+    return bad;
+}
+"""
+
 
 def run(tmp_path, program):
     src, exe = tmp_path / "index.cu", tmp_path / "index"
@@ -42,3 +57,7 @@ def run(tmp_path, program):
 
 def test_anchor_of_a_window_beyond_32_bits(tmp_path):
     run(tmp_path, ANCHOR)
+
+
+def test_records_beyond_32_bit_offsets(tmp_path):
+    run(tmp_path, RECORD)

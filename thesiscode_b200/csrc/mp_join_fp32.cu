@@ -66,9 +66,7 @@ namespace mpgpu {
 
 namespace {
 
-// A row or column record in global memory: (x[j], x[j+4]) pairs of df, dg, nn for
-// rows, (-df, -df, -dg, -dg, nn, nn, 1/nn, 1/nn) for columns.
-constexpr int kRecFloats = 8;
+constexpr int kRecFloats = kFp32RecFloats;
 constexpr int kR = kTileR;  // 8: tags of 3 + 5 bits
 
 constexpr unsigned kTagMask = 0xffu;
@@ -357,10 +355,10 @@ __device__ void tile_dense(const Fp32TileParams& P, int64_t band, int64_t seg, i
         // copied straight into shared memory while the pair runs
         {
             const int s = rec_slot(fill + (lane >> 1));
-            const uint4* src = rsrc + 2 * fill + lane;
+            const uint4* src = rsrc + 2 * (int64_t)fill + lane;
             cp_async16(rring + rec_off(s) + 16 * (lane & 1), src);
             if (s < kRecMirror) cp_async16(rring + rec_off(s + kRecRing) + 16 * (lane & 1), src);
-            cp_async16(cring + (cb ^ 1) * 64 * R + 16 * lane, csrc + 2 * (jr + 2 * R) + lane);
+            cp_async16(cring + (cb ^ 1) * 64 * R + 16 * lane, csrc + 2 * (int64_t)(jr + 2 * R) + lane);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         }
         int colkey = 0x7fffffff;
@@ -703,9 +701,9 @@ __device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, in
     // groups 0 .. 33 and the first pass's columns; from here on lanes 0 - 15 look
     // after rows, lanes 16 - 31 after columns
     const int64_t rb = j0 + gb;  // row of element 0 of group 0
-    const float* nrow = reinterpret_cast<const float*>(P.rowrec) + rb * kRecFloats;
-    const float* ncol = reinterpret_cast<const float*>(P.colrec) + j0 * kRecFloats;
-    for (int i = 0; i < 17; ++i) sm.stage_rows(2 * i, nrow + 16 * kRecFloats * i, lane);
+    const float* nrow = fp32_record(reinterpret_cast<const float*>(P.rowrec), rb);
+    const float* ncol = fp32_record(reinterpret_cast<const float*>(P.colrec), j0);
+    for (int i = 0; i < 17; ++i) sm.stage_rows(2 * i, fp32_record(nrow, 16 * i), lane);
     sm.stage_cols(0, ncol, lane);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     for (int i = lane; i < 34 * R; i += 32) {
@@ -738,8 +736,8 @@ __device__ void tile_gate(const Fp32TileParams& P, int64_t band, int64_t seg, in
     for (; jr < ncols; jr += kPassCols) {
         // what the next pass appends: 16 rows, 16 columns and their keys
         const int sn = wrap_group(sf + 34);
-        sm.stage_rows(sn, nrow + (34 * R + jr) * kRecFloats, lane);
-        sm.stage_cols(cb ^ 1, ncol + (jr + kPassCols) * kRecFloats, lane);
+        sm.stage_rows(sn, fp32_record(nrow, 34 * R + (int64_t)jr), lane);
+        sm.stage_cols(cb ^ 1, fp32_record(ncol, jr + kPassCols), lane);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         const int64_t inc = inc0 + jr;
         unsigned f = 0;

@@ -269,6 +269,13 @@ struct Fp32TileParams {
     const double* dg;
 };
 #ifdef __CUDACC__
+// A row or column record in global memory: (x[j], x[j+4]) pairs of df, dg, nn for
+// rows, (-df, -df, -dg, -dg, nn, nn, 1/nn, 1/nn) for columns.  Record i from `base` on:
+// with 2^28 columns between re-anchors its offset passes 32 bits.
+constexpr int kFp32RecFloats = 8;
+__host__ __device__ __forceinline__ const float* fp32_record(const float* base, int64_t i) {
+    return base + i * kFp32RecFloats;
+}
 // Local tile lt of a series -> (band, column segment), see tile_of_pair.
 __host__ __device__ __forceinline__ bool fp32_tile_of(const Fp32TileParams& P, int64_t lt, int64_t span,
                                              int64_t& band, int64_t& seg) {
