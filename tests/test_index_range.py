@@ -46,6 +46,24 @@ int main() {
 }
 """
 
+# PreSCRIMP's exclusion zone beside the largest window numbers: the reference's rule.
+ZONE = HEAD + r"""
+int main() {
+    int bad = 0;
+    const long long last = (1ll << 31) - 2;
+    for (const long long excl : {0ll, 1ll, 16ll, 250ll, 1ll << 30, last})
+        for (const long long i : {0ll, 1ll, 300ll, last / 2, last - 300, last - 1, last})
+            for (const long long d : {0ll, 1ll, 15ll, 16ll, 17ll, 249ll, 250ll, 251ll, 1ll << 30, last})
+                for (int s = -1; s <= 1; s += 2) {
+                    const long long j = i + s * d;
+                    if (j < 0 || j > last) continue;
+                    const bool want = j > i - excl && j < i + excl;
+                    bad += prescrimp_excluded((unsigned)i, (unsigned)j, (unsigned)excl) != want;
+                }
+    return bad;
+}
+"""
+
 
 def run(tmp_path, program):
     src, exe = tmp_path / "index.cu", tmp_path / "index"
@@ -61,3 +79,7 @@ def test_anchor_of_a_window_beyond_32_bits(tmp_path):
 
 def test_records_beyond_32_bit_offsets(tmp_path):
     run(tmp_path, RECORD)
+
+
+def test_prescrimp_exclusion_zone_of_the_last_windows(tmp_path):
+    run(tmp_path, ZONE)

@@ -500,6 +500,11 @@ struct PreScrimpParams {
     unsigned long long* rix;  // [Q] ... (neighbour)
     int idx_bits;
 };
+// Whether the windows i and j lie within the exclusion zone (ScrimpppOrig.cpp:190-193).
+// (Host-callable, so the rule can be checked without a GPU.)
+__host__ __device__ inline bool prescrimp_excluded(unsigned i, unsigned j, unsigned excl) {
+    return (j > i ? j - i : i - j) < excl;
+}
 __global__ void orig_stats_kernel(const double* cs, const double* cs2, int64_t PL, int64_t m,
                                   double* mean, double* sigma);
 __global__ void prescrimp_keys_init_kernel(unsigned long long* a, int64_t count);

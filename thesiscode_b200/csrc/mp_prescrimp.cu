@@ -165,13 +165,14 @@ __global__ void __launch_bounds__(kRowThreads, 3) prescrimp_rows_kernel(const Pr
         mi[r] = t < P.Q ? P.mean[t * P.step] : 0.0;
         si[r] = t < P.Q ? P.sigma[t * P.step] : 0.0;
     }
-    const int i0 = (int)(t0 * P.step), jw = (int)j0 + wi * kJW, PL = (int)P.PL;
-    const int step = (int)min(P.step, P.PL), excl = (int)min(P.excl, P.PL);
+    // positions as unsigned numbers: a tile may reach beyond 2^31 - 1
+    const unsigned i0 = (unsigned)(t0 * P.step), jw = (unsigned)j0 + wi * kJW, PL = (unsigned)P.PL;
+    const unsigned step = (unsigned)min(P.step, P.PL), excl = (unsigned)min(P.excl, P.PL);
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int j = jw + 8 * c + 2 * lc + h;
+            const unsigned j = jw + 8 * c + 2 * lc + h;
             double cb = DBL_MAX;
             int ci = -1;
             if (j < PL) {
@@ -179,19 +180,19 @@ __global__ void __launch_bounds__(kRowThreads, 3) prescrimp_rows_kernel(const Pr
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const int q = 8 * r + lr;
-                    const int i = i0 + q * step;
-                    if (q >= nq || (j > i - excl && j < i + excl)) continue;  // ScrimpppOrig.cpp:190-193
+                    const unsigned i = i0 + q * step;
+                    if (q >= nq || prescrimp_excluded(i, j, excl)) continue;
                     // orig_distance
                     const double d = __dmul_rn(
                         2.0, __dsub_rn(mm, __ddiv_rn(__dsub_rn(acc[r][c][h], __dmul_rn(mj, mi[r])),
                                                      __dmul_rn(sj, si[r]))));
                     if (d < cb) {
                         cb = d;
-                        ci = i;
+                        ci = (int)i;
                     }
                     if (d < rb[r]) {
                         rb[r] = d;
-                        ri[r] = j;
+                        ri[r] = (int)j;
                     }
                 }
             }
