@@ -1,0 +1,50 @@
+"""What a call costs on other data than random walks, beside a walk of the same size: series
+of constant stretches, with a NaN, with a short pattern that comes again and again."""
+from __future__ import annotations
+
+import time
+
+import numpy as np
+import pytest
+
+from thesiscode_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def series(kind, n):
+    x = workloads.random_walk(n, n)
+    if kind == "nan":  # prefix sums: every window from its first one on is NaN
+        x[n // 2] = np.nan
+    elif kind == "constant":
+        x[:] = 3.7
+    return x
+
+
+def on_gpu(x, m):
+    import torch
+    return torch.from_numpy(x).cuda(), (torch.empty(x.size - m + 1, dtype=torch.float64, device="cuda"),
+                                        torch.empty(x.size - m + 1, dtype=torch.int64, device="cuda"))
+
+
+def ms(call, runs=7):
+    import torch
+    best = 1e9
+    for _ in range(runs):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        call()  # returns when the result is there
+        best = min(best, time.perf_counter() - t)
+    return 1e3 * best
+
+
+# Walks take 5.5 ms here, and 7.0 where the rows ran without the matrix instruction; these
+# series took 7.5 and 7.7 then.
+@pytest.mark.parametrize("kind", ["nan", "constant"])
+def test_prescrimp_of_degenerate_windows(gpu_ctx, kind):
+    n, m = 100000, 64
+    t = []
+    for k in ("walk", kind):
+        x, out = on_gpu(series(k, n), m)
+        t.append(ms(lambda: gpu_ctx.prescrimp(x, m, 0.25, out=out)))
+    assert t[1] < 1.35 * t[0], t
