@@ -18,6 +18,10 @@ def series(kind, n):
         x[n // 2] = np.nan
     elif kind == "constant":
         x[:] = 3.7
+    elif kind == "sine":
+        x = np.sin(2 * np.pi * np.arange(n) / 97.3) + 0.1 * np.random.default_rng(n).standard_normal(n)
+    elif kind == "steps":
+        x = np.repeat(np.random.default_rng(n).integers(-5, 6, n // 150 + 1), 150)[:n].astype(np.float64)
     return x
 
 
@@ -48,3 +52,16 @@ def test_prescrimp_of_degenerate_windows(gpu_ctx, kind):
         x, out = on_gpu(series(k, n), m)
         t.append(ms(lambda: gpu_ctx.prescrimp(x, m, 0.25, out=out)))
     assert t[1] < 1.35 * t[0], t
+
+
+# 280,000 samples (whole bands): a walk with m = 256 takes about 28 ms; with every step tested
+# in FP64 all of these took 43 ms, the steps 60.
+@pytest.mark.parametrize("kind,m,limit", [("walk", 16, 1.9), ("sine", 32, 1.9), ("nan", 64, 1.9),
+                                          ("steps", 256, 3.0)])
+def test_fp64_join_where_gates_open(gpu_ctx, kind, m, limit):
+    n = 280000
+    t = []
+    for k, w in (("walk", 256), (kind, m)):
+        x, out = on_gpu(series(k, n), w)
+        t.append(ms(lambda: gpu_ctx.selfjoin(x, w, out=out), runs=3))
+    assert t[1] < limit * t[0], t

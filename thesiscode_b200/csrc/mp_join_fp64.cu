@@ -51,15 +51,28 @@
 // the selection.  High words take R/2 integer maxima and two additions per column
 // where doubles took 2R compares, and no branch between the columns.
 //
+// How often a gate opens depends on the data: noisy patterns, short windows and series of few
+// levels have rows of unlike best scores side by side, and the smallest of R opens many
+// passes in which no cell selects.  So whole bands (WHOLE) back off: after gates that opened
+// in a row, and after a pass that selected, passes go straight to the reference's
+// arithmetic, 4 columns at a time, each cell tested against its own row's best
+// (test_chunk); only columns from such a cell on, to the end of 8, are evaluated with the
+// selection.  300,000 samples: noisy sine, m = 64 61 -> 47 ms (46 with every step tested in
+// FP64), half NaN 117 -> 44 (46), steps of 150 samples, m = 256 97 -> 77 (67); 280,000, m = 16,
+// walk 81 -> 45 (43), sine 106 -> 44 (43).  Tiles, short and young, select more of what they
+// test, and evaluate an open pass with the selection throughout (n = 65,536: 1.58 ms;
+// as whole bands do 1.77).
+//
 // What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 4
 // per cell (33 of a step's 60 instructions at R = 8); other instructions cost it
-// about 0.7 cycles each.  n = 1,048,576, m = 256: 243 ms, from 441 ms with the
+// about 0.7 cycles each.  n = 1,048,576, m = 256: 237 ms, from 441 ms with the
 // selection tested per step in FP64 and the bands in order of length (one gate per
 // pass and 5 operations: 254 ms; that with a pass's two chunks as a loop 271 ms;
 // 3 CTAs of 4 warps per SM at 168 registers spill, 273 ms).  Short windows have rows
 // of unlike best scores side by side, and one bound for a pass's 23 rows and 16
 // columns opened a quarter of the passes at m = 64 where 2% select (n = 600,000: 164
-// ms; a bound per 15 rows and 8 columns 134; per 8 rows and a column 101).  With
+// ms; a bound per 15 rows and 8 columns 134; per 8 rows and a column 101, 96 with the passes
+// after an open one straight).  With
 // fewer bands than resident warps the longest band sets the time; then the bands
 // are cut into tiles (Fp64Split).
 #include <float.h>
@@ -159,13 +172,15 @@ struct BandSmem {
     static constexpr int kGateStride = R == 8 ? 12 : R;  // lanes hit distinct banks
     static constexpr int kUsed = kGroups * kRecStride + 2 * 32 * R * kU +
                                  kGroups * (R + 1) * (int)(sizeof(double) + sizeof(int)) +
-                                 2 * R * kU * (int)sizeof(double) +
+                                 3 * R * kU * (int)sizeof(double) + R * kU * (int)sizeof(int) +
                                  (kGroups * kGateStride + 2 * R * kU + kGroups / kU) * (int)sizeof(int);
     static constexpr int kBytes = (kUsed + 15) / 16 * 16;  // warps' areas stay aligned
     char* rec;     // row records
     char* col;     // column records {A[j], A[j+m], s, fp64_gate_mean}, two buffers of kU * R
-    double* best;  // best score of each row (its threshold while src < 0)
+    double* best;  // best score of each row (fp64_bound of its threshold while src < 0)
     double* cmean; // column mean terms, two buffers of kU * R
+    double* cbest; // best scores of the pass's columns ...
+    int* cdiag;    // ... and their diagonals
     int* src;      // column of a row's best score, -1: none yet
     int* gate;     // per row: smallest gate among the best scores of R rows from it on
     int* cgate;    // gates of the columns' thresholds, two buffers of kU * R
@@ -179,11 +194,14 @@ struct BandSmem {
         p += kGroups * (R + 1) * sizeof(double);
         cmean = reinterpret_cast<double*>(p);
         p += 2 * R * kU * sizeof(double);
+        cbest = reinterpret_cast<double*>(p);
+        p += R * kU * sizeof(double);
         src = reinterpret_cast<int*>(p);
         p += kGroups * (R + 1) * sizeof(int);
         gate = reinterpret_cast<int*>(p);
         cgate = gate + kGroups * kGateStride;
         err = cgate + 2 * R * kU;
+        cdiag = err + kGroups / kU;
     }
     // gates of the rows of the group in slot s, from the best scores as they stand
     __device__ __forceinline__ void group_gates(int s, double m) const {
@@ -205,11 +223,12 @@ struct BandSmem {
 };
 
 // The column's best cell over the warp, from two REDUX instructions (high, then
-// low word of the ordered score; ties go to the smallest diagonal); the winning
-// lane merges it.
+// low word of the ordered score; ties go to the smallest diagonal), left for the pass's
+// end, which merges its 16 columns side by side (one lane's merge after each column took
+// 107 of 274 ms where three of five columns select).  Returns whether there is one.
 template <int R>
-__device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard, unsigned j,
-                                              const double (&sc)[R], int64_t g0, int lane) {
+__device__ __forceinline__ bool select_column(const double (&sc)[R], double floor, double* best, int* diag,
+                                              int lane) {
     // lane's best cell of the column.  A NaN cell (a constant window) never
     // selects under the reference's '>'; as -DBL_MAX it also cannot hide the
     // cell it is paired with in the tree.
@@ -221,7 +240,7 @@ __device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard
 #pragma unroll
         for (int a = 0; a + w < R; a += 2 * w) cb[a] = cb[a + w] > cb[a] ? cb[a + w] : cb[a];
     const double cbest = cb[0];
-    const unsigned long long key = (cbest > P.floor) ? ord_f64(cbest) : 0ull;
+    const unsigned long long key = (cbest > floor) ? ord_f64(cbest) : 0ull;
     const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
     const unsigned mhi = __reduce_max_sync(kFullMask, hi);
     const unsigned mlo = __reduce_max_sync(kFullMask, hi == mhi ? lo : 0u);
@@ -231,8 +250,41 @@ __device__ __forceinline__ void select_column(const Fp64BandParams& P, int shard
         int ca = R - 1;
 #pragma unroll
         for (int a = R - 2; a >= 0; --a) ca = sc[a] == cbest ? a : ca;
-        flush_fp64(P, shard, j + P.col_key_off, cbest, j + g0 + ca + P.row_nb_off);
+        *best = cbest;
+        *diag = lane * R + ca;
     }
+    return tops != 0u;
+}
+
+// A column step's selection: every cell above its row's best replaces it (strict '>', the
+// reference's rule; a step's cells lie in distinct rows), and where some lane's cells may
+// exceed the column's threshold (`col`) the column is reduced over the warp.  Cell a lies
+// in element k + a of the lane's groups, which start at e0 and e1 + R; b: the column in
+// the pass.  Returns kRose if a row's best rose in the lane, and bit b if the column has a
+// best cell.
+constexpr int kRose = 1 << 16;
+template <int R>
+struct Cells {
+    double s[R];
+};
+template <int R>
+__device__ __forceinline__ int select_cells(const Cells<R>& sc, double floor, unsigned j, const BandSmem<R>& sm,
+                                            int e0, int e1, int k, int b, bool col, int lane) {
+    __syncwarp();  // rows move from lane to lane between steps
+    int did = 0;
+    double best[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) best[a] = sm.best[(k + a < R ? e0 : e1) + a];
+#pragma unroll
+    for (int a = 0; a < R; ++a)
+        if (sc.s[a] > best[a]) {
+            sm.best[(k + a < R ? e0 : e1) + a] = sc.s[a];
+            sm.src[(k + a < R ? e0 : e1) + a] = (int)j;
+            did = kRose;
+        }
+    if (__any_sync(kFullMask, col) && select_column<R>(sc.s, floor, sm.cbest + b, sm.cdiag + b, lane))
+        did |= 1 << b;
+    return did;
 }
 
 // One chunk = R consecutive columns, all their cells in the reference's 4-wide
@@ -290,25 +342,70 @@ __device__ __noinline__ int widen_gate(const BandSmem<R>& sm, int s0, const int*
     return fp64_gate_lowered(g, err, over) ? 0 : -1;
 }
 
-// A pass of kU chunks with the selection, s0 the slot of the lane's first group:
-// EDGE evaluates every cell with its own geometry and selects in every step;
-// otherwise all cells are fused and a step selects behind the gate.  A step's
-// selection: every cell above its row's best replaces it (strict '>', the
-// reference's rule; a step's cells lie in distinct rows), and a column whose
-// largest high word reaches its threshold's is reduced over the warp.  Returns
-// whether a step selected.  One loop over the columns with the records read from
-// shared memory: unrolled like gate_chunk, this path's code pushed the passes
-// without selection out of the instruction cache.
+// The same with the reference's arithmetic, a test of C columns at a time against the rows'
+// own best scores: stops before the first C that hold a cell which may select.  Returns
+// that column, R if there is none.
+template <int R>
+__device__ __forceinline__ int test_chunk(const BandSmem<R>& sm, int s0, int s1, const char* col,
+                                          const double* cmean, const int* cgate, double4 (&rwin)[R],
+                                          int (&gwin)[R], double (&qt)[R]) {
+    const char* rec1 = sm.rec + s1 * BandSmem<R>::kRecStride;
+    const double* best1 = sm.best + s1 * (R + 1);
+    constexpr int C = R < 4 ? R : 4;
+#pragma unroll
+    for (int b0 = 0; b0 < R; b0 += C) {
+        int over = INT_MIN;
+        double q[R];
+#pragma unroll
+        for (int a = 0; a < R; ++a) q[a] = qt[a];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+            const int b = b0 + i;
+            const double4 cv = ring_rec(col + 32 * b);
+            const double cw = cmean[b];
+            int top = 0, hi[R], o[2] = {INT_MIN, INT_MIN};
+#pragma unroll
+            for (int a = 0; a < R; ++a) {
+                const double4 rv = rwin[(b + a) % R];
+                const int rg = gwin[(b + a) % R];
+                if (a == 0) {
+                    rwin[b] = ring_rec(rec1 + 32 * b);
+                    gwin[b] = fp64_best_gate(__double2hiint(best1[b]));
+                }
+                // kernels.cpp:206-225
+                const double mm = __dmul_rn(cw, rv.w);
+                const double sc = __fma_rn(q[a], __dmul_rn(rv.z, cv.z), -mm);
+                q[a] = __fma_rn(-rv.x, cv.x, __fma_rn(rv.y, cv.y, q[a]));
+                hi[a] = fp64_cell_high(__double2hiint(sc));
+                o[a & 1] = __viaddmax_s32(hi[a], rg, o[a & 1]);
+            }
+            if (R == 1) top = hi[0];
+#pragma unroll
+            for (int a = 0; a + 1 < R; a += 2) top = __vimax3_s32(top, hi[a], hi[a + 1]);
+            over = __vimax3_s32(over, o[0], o[1]);
+            over = __viaddmax_s32(top, fp64_cell_gate(cgate[b]), over);
+        }
+        if (__any_sync(kFullMask, over >= kFp64Pass)) return b0;
+#pragma unroll
+        for (int a = 0; a < R; ++a) qt[a] = q[a];
+    }
+    return R;
+}
+
+// Columns `from` to `to` of a pass with the selection, s0 the slot of the lane's first
+// group: EDGE evaluates every cell with its own geometry and selects in every step;
+// otherwise all cells are fused and a step selects behind the gate.  Returns the steps'
+// select_cells.  One loop over the columns with the records read from shared memory:
+// unrolled like gate_chunk, this path's code pushed the passes without selection out of
+// the instruction cache.
 template <int R, bool EDGE>
-__device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, unsigned jc,
-                                            const BandSmem<R>& sm, int s0, const char* col,
-                                            const double* cmean,
-                                            const int* cgate, double (&qt)[R],
-                                            unsigned geo, int64_t gb, int lane) {
-    constexpr int RS = BandSmem<R>::kRecStride, kU = BandSmem<R>::kU;
-    bool sel = false;
+__device__ __forceinline__ int select_pass(const Fp64BandParams& P, unsigned jc, const BandSmem<R>& sm, int s0,
+                                           const char* col, const double* cmean, const int* cgate,
+                                           double (&qt)[R], unsigned geo, int64_t gb, int lane, int from, int to) {
+    constexpr int RS = BandSmem<R>::kRecStride;
+    int did = 0;
 #pragma unroll 1
-    for (int b = 0; b < kU * R; ++b) {
+    for (int b = from; b < to; ++b) {
         const unsigned j = jc + b;
         const int k = b % R;  // cell a lies in element k + a of the lane's groups
         const int sa = BandSmem<R>::wrap(s0 + b / R), sb = BandSmem<R>::wrap(sa + 1);
@@ -316,8 +413,8 @@ __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, 
         const char* rec1 = sm.rec + sb * RS + 32 * (k - R);
         const double4 cv = ring_rec(col + 32 * b);
         const double cw = cmean[b];
-        double sc[R];
-        int top = 0;
+        Cells<R> sc;
+        int top = kFp64NoNan;
 #pragma unroll
         for (int a = 0; a < R; ++a) {
             const double4 rv = ring_rec((k + a < R ? rec0 : rec1) + 32 * a);
@@ -338,33 +435,22 @@ __device__ __forceinline__ bool select_pass(const Fp64BandParams& P, int shard, 
                                       __dmul_rn(rv.x, cv.x));
                 }
             }
-            sc[a] = score;
-            top = max(top, __double2hiint(score));
+            sc.s[a] = score;
+            top = __viaddmax_s32(__double2hiint(score), kFp64NoNan, top);
         }
+        top -= kFp64NoNan;
         if (!EDGE &&
             !__any_sync(kFullMask, top + max(sm.gate[sa * BandSmem<R>::kGateStride + k], cgate[b]) >= 0))
             continue;
-        __syncwarp();  // rows move from lane to lane between steps
-        const int e0 = sa * (R + 1) + k, e1 = sb * (R + 1) + k - R;
-        double best[R];
-#pragma unroll
-        for (int a = 0; a < R; ++a) best[a] = sm.best[(k + a < R ? e0 : e1) + a];
-#pragma unroll
-        for (int a = 0; a < R; ++a)
-            if (sc[a] > best[a]) {
-                sm.best[(k + a < R ? e0 : e1) + a] = sc[a];
-                sm.src[(k + a < R ? e0 : e1) + a] = (int)j;
-                sel = true;
-            }
-        if (__any_sync(kFullMask, top + cgate[b] >= 0))
-            select_column<R>(P, shard, j, sc, gb + lane * R, lane);
+        did |= select_cells<R>(sc, P.floor, j, sm, sa * (R + 1) + k, sb * (R + 1) + k - R, k, b,
+                               top + cgate[b] >= 0, lane);
     }
-    return __any_sync(kFullMask, sel);
+    return did;
 }
 
 // Columns [j0, jend) of a band.  lt: the tile's number when the band is cut into
-// tiles (then jend - j0 = L, or less for the band's last tile).
-template <int R>
+// tiles (then jend - j0 = L, or less for the band's last tile).  WHOLE: see above.
+template <int R, bool WHOLE>
 __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band, int64_t lt,
                                           int64_t seg, int lane, int shard,
                                           const BandSmem<R>& sm) {
@@ -434,7 +520,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     for (int k = 0; k < kOwn; ++k) {
         const int i = lane + 32 * k;
         if (i < (32 + kU) * R) {
-            sm.best[(i / R) * (R + 1) + i % R] = thr[k];
+            sm.best[(i / R) * (R + 1) + i % R] = fp64_bound(thr[k], sw[k].x, sw[k].y);
             sm.src[(i / R) * (R + 1) + i % R] = -1;
             rerr = max(rerr, fp64_gate_error(sw[k].x, sw[k].y));
         }
@@ -448,7 +534,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         *reinterpret_cast<double2*>(sm.col + 32 * lane + 16) =
             make_double2(sw.x, __ldg(P.colgate + min((int64_t)j0 + lane, wlast)));
         sm.cmean[lane] = sw.y;
-        sm.cgate[lane] = fp64_gate(t, P.m);
+        sm.cgate[lane] = fp64_gate(fp64_bound(t, sw.x, sw.y), P.m);
         cerr = fp64_gate_error(sw.x, sw.y);
     }
     cerr = __reduce_max_sync(kFullMask, cerr);
@@ -462,8 +548,11 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     // register window of row records: slot (k mod R) holds element k of the
     // lane's first group
     double4 rwin[R];
+    auto load_window = [&](int s) {
 #pragma unroll
-    for (int k = 0; k < R; ++k) rwin[k] = ring_rec(sm.rec + lane * RS + 32 * k);
+        for (int k = 0; k < R; ++k) rwin[k] = ring_rec(sm.rec + s * RS + 32 * k);
+    };
+    load_window(lane);
 
     // what the lane copies in next: records of groups c + 32 + kU .. and of the
     // next pass's columns, and their thresholds
@@ -475,6 +564,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     int sf = 0;     // slot of group c, the first that the pass finishes
     int cbuf = 0;
     bool sel = false;
+    int skip = 0, streak = 0;
     for (unsigned jc = j0; jc < jend; jc += kU * R) {
         const int sn = BandSmem<R>::wrap(sf + 32 + kU);  // slots of the incoming groups (kU divides kGroups)
         double w = 0.0;
@@ -494,7 +584,10 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         const int* cgate = sm.cgate + cbuf * (R * kU);
         const double* cmean = sm.cmean + cbuf * (R * kU);
         const bool fused = (int64_t)jc + (kU * R - 1) <= minpsw;
-        bool open = !fused || sel;  // a pass after one that selected goes straight to selecting
+        // A pass after one that selected goes straight to selecting; so do the next 1, 2,
+        // 4 .. 16 passes after gates that opened in a row.
+        bool open = !fused || sel || skip > 0;
+        skip -= skip > 0;
         if (!open) {
             double q0[R];
 #pragma unroll
@@ -507,18 +600,43 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
                                                col + u * 32 * R, cgate + u * R, rwin, qt));
             if (err > errfree) over = widen_gate<R>(sm, s0, cgate, err, over);
             open = __any_sync(kFullMask, over >= 0);
+            streak = WHOLE && open ? min(max(2 * streak, 1), 16) : 0;
+            skip = streak;
             if (open) {
 #pragma unroll
                 for (int a = 0; a < R; ++a) qt[a] = q0[a];
+                if (WHOLE) load_window(s0);
             }
         }
         sel = false;
-        if (open) {
-            sel = fused ? select_pass<R, false>(P, shard, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane)
-                        : select_pass<R, true>(P, shard, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane);
-            const char* r0 = sm.rec + BandSmem<R>::wrap(s0 + kU) * RS;
+        int did = 0;
+        if (open && !(WHOLE && fused)) {
+            did = fused ? select_pass<R, false>(P, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane, 0, kU * R)
+                        : select_pass<R, true>(P, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane, 0, kU * R);
+            load_window(BandSmem<R>::wrap(s0 + kU));
+        } else if (open) {
+#pragma unroll 1
+            for (int u = 0; u < kU; ++u) {
+                const int sa = BandSmem<R>::wrap(s0 + u), sb = BandSmem<R>::wrap(sa + 1);
+                int gwin[R];  // gates of the rows in rwin
 #pragma unroll
-            for (int a = 0; a < R; ++a) rwin[a] = ring_rec(r0 + 32 * a);
+                for (int a = 0; a < R; ++a) gwin[a] = fp64_best_gate(__double2hiint(sm.best[sa * (R + 1) + a]));
+                const int b = test_chunk<R>(sm, sa, sb, col + u * 32 * R, cmean + u * R, cgate + u * R, rwin,
+                                            gwin, qt);
+                if (b < R) {
+                    did |= select_pass<R, false>(P, jc, sm, s0, col, cmean, cgate, qt, geo, gb, lane, u * R + b,
+                                                 (u + 1) * R);
+                    load_window(sb);
+                }
+            }
+        }
+        if (open) {
+            sel = __any_sync(kFullMask, did & kRose);
+            __syncwarp();
+            if ((did & (kRose - 1)) >> lane & 1) {  // column jc + lane
+                const int64_t j = (int64_t)jc + lane;
+                flush_fp64(P, shard, j + P.col_key_off, sm.cbest[lane], j + gb + sm.cdiag[lane] + P.row_nb_off);
+            }
         }
         __syncwarp();
         // groups c .. c + kU - 1 have met every lane: merge their rows
@@ -528,10 +646,11 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
             finish_row<R>(P, shard, lt, seg, more, rb, (int64_t)(jc - j0) + lane, sm.best[e], j);
         }
         // the incoming groups and columns begin at their thresholds
-        const int x = fp64_gate(t, P.m);
+        const double bound = fp64_bound(t, sw.x, sw.y);
+        const int x = fp64_gate(bound, P.m);
         if (isrow) {
             const int e = (sn + part / R) * (R + 1) + part % R;
-            sm.best[e] = t;
+            sm.best[e] = bound;
             sm.src[e] = -1;
         } else {
             *reinterpret_cast<double2*>(sm.col + (cbuf ^ 1) * (32 * R * kU) + 32 * part + 16) =
@@ -587,7 +706,7 @@ constexpr int fp64_smem_bytes() {
     return kFp64WarpsPerBlock * BandSmem<R>::kBytes;
 }
 
-template <int R>
+template <int R, bool WHOLE>
 __global__ void __launch_bounds__(32 * kFp64WarpsPerBlock, R == 8 ? 2 : 4)
     fp64_band_kernel(const Fp64BandParams P) {
     extern __shared__ __align__(128) char smem_fp64[];
@@ -608,7 +727,7 @@ __global__ void __launch_bounds__(32 * kFp64WarpsPerBlock, R == 8 ? 2 : 4)
                                32 * R, band, seg);
         else
             band = fp64_band_of(rank, P.nbands, P.spread);
-        if (any) band_fp64<R>(P, band, rank, seg, lane, shard, sm);
+        if (any) band_fp64<R, WHOLE>(P, band, rank, seg, lane, shard, sm);
         unsigned next = 0;
         if (lane == 0) next = atomicAdd(P.counter, 1u);
         rank = (int64_t)gridDim.x * kFp64WarpsPerBlock + __shfl_sync(kFullMask, next, 0);
@@ -894,8 +1013,8 @@ void launch_fp64_seeds(const Fp64BandParams& P, const double* Ah, int64_t nh, co
                                                                                     X);
 }
 
-template <int R>
-void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
+template <int R, bool WHOLE>
+void launch_band_kernel(const Fp64BandParams& Q, cudaStream_t s) {
     constexpr int smem = fp64_smem_bytes<R>();
     // per-device attribute and occupancy, idempotent: see launch_fp32_join
     static std::atomic<unsigned long long> configured{0};
@@ -904,9 +1023,9 @@ void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
     cudaGetDevice(&dev);
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        cudaFuncSetAttribute(fp64_band_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(fp64_band_kernel<R, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fp64_band_kernel<R>,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fp64_band_kernel<R, WHOLE>,
                                                           32 * kFp64WarpsPerBlock, smem) != cudaSuccess ||
             per_sm < 1) {
             cudaGetLastError();
@@ -924,8 +1043,19 @@ void launch_fp64_band(const Fp64BandParams& Q, cudaStream_t s) {
     Fp64BandParams P = Q;
     P.spread = (P.nbands + blocks * kFp64WarpsPerBlock - 1) / (blocks * kFp64WarpsPerBlock);
     cudaMemsetAsync(P.counter, 0, sizeof(unsigned), s);
-    fp64_band_kernel<R><<<(unsigned)blocks, 32 * kFp64WarpsPerBlock, smem, s>>>(P);
+    fp64_band_kernel<R, WHOLE><<<(unsigned)blocks, 32 * kFp64WarpsPerBlock, smem, s>>>(P);
     if (P.split.L > 0) fp64_seam_kernel<R><<<(unsigned)P.split.ntiles, 128, 0, s>>>(P);
+}
+
+// Whole bands of 256 diagonals take the kernel that backs off (m = 16, n = 280,000: 45 ms, 80
+// without); narrower bands come from a few hundred diagonals, which are cut into tiles
+// wherever there is room.
+template <int R>
+void launch_fp64_band(const Fp64BandParams& P, cudaStream_t s) {
+    if (R == 8 && P.split.L == 0)
+        launch_band_kernel<R, R == 8>(P, s);
+    else
+        launch_band_kernel<R, false>(P, s);
 }
 
 template void launch_fp64_band<1>(const Fp64BandParams&, cudaStream_t);

@@ -116,29 +116,57 @@ __host__ __device__ inline bool fp64_ordinary(double s, double w) {
 __host__ __device__ inline bool fp64_flat(double s, double w) {
     return s > DBL_MAX && (w > DBL_MAX || w < -DBL_MAX);
 }
+// A window without a finite score: its scores are NaN, or with a constant window NaN or
+// infinite.  No score of it is between a finite bound and the largest double, so that
+// serves as the bound of every one of its cells, and its gate stays shut for finite ones.
+__host__ __device__ inline bool fp64_degenerate(double s, double w) {
+    return s != s || w != w || fp64_flat(s, w);
+}
+__host__ __device__ inline double fp64_bound(double threshold, double s, double w) {
+    return !fp64_ordinary(s, w) && fp64_degenerate(s, w) ? DBL_MAX : threshold;
+}
 // A column's mean term in the FP64 join's gate, which tests s' (q s - w W') in place of
 // the score q (s s') - w w': W' = w' / s'.  A constant column's scores are -inf, NaN, or
 // +inf where w w' < 0; with the largest double as W' the gate's value is positive there.
 __host__ __device__ inline double fp64_gate_mean(double s, double w) {
-    if (fp64_ordinary(s, w)) return w / s;
+    if (fp64_ordinary(s, w)) {
+        const double x = w / s;
+        return x != 0.0 || w == 0.0 ? x : copysign(DBL_MIN, w);  // its product with an infinite term keeps its sign
+    }
     if (fp64_flat(s, w)) return w > 0.0 ? DBL_MAX : -DBL_MAX;
     return w != w ? w : 0.0;  // the gate stands open (fp64_gate_error), or the score is NaN
 }
 // A bound's gate: minus the high word of a value below it by more than the rounding
-// of the gate's values (kFp64GateSlack m, and 2^-34 of the bound).  A negative bound, or
-// one so large that a product may leave the range of doubles, lets every cell through.
+// of the gate's values (kFp64GateSlack m, and 2^-34 of the bound).  A negative bound lets
+// every cell through; past kFp64GateEnd, where a product may leave the range of doubles
+// (and the gate's value counts as the largest one), a bound's gate is that end's.
 constexpr double kFp64GateSlack = 0x1p-25;
 constexpr int kFp64GateEnd = (1023 + 500) << 20;
 __host__ __device__ inline int fp64_gate(double bound, double m) {
     const int h = high_word(fma(bound, 1.0 - 0x1p-34, -kFp64GateSlack * m));
-    return h < kFp64GateEnd && h > 0 ? -h : 0;
+    return h > 0 ? -(h < kFp64GateEnd ? h : kFp64GateEnd) : 0;
 }
 // The same from the bound's high word h alone, a unit lower: from m / 16 on a unit is
 // more than the slack.
 __host__ __device__ inline int fp64_gate_high_from(double m) { return high_word(m * 0x1p-4) + 1; }
 __host__ __device__ inline int fp64_gate_high(int h, int from) {
-    return h >= from && h < kFp64GateEnd ? 1 - h : 0;
+    return h >= from ? 1 - (h < kFp64GateEnd ? h : kFp64GateEnd) : 0;
 }
+// Added to a score's high word, kFp64NoNan takes a NaN (0x7ff8 or above, or its negative)
+// to a negative number or 0 and leaves the order of all other values.  A score passes a
+// gate if fp64_cell_high + fp64_cell_gate >= kFp64Pass (the largest sum is 0x7fffffff).
+constexpr int kFp64NoNan = 0x80000, kFp64Pass = kFp64NoNan - 1;
+__host__ __device__ inline int fp64_cell_high(int h) {
+#ifdef __CUDA_ARCH__
+    return __viaddmax_s32(h, kFp64NoNan, 0);
+#else
+    const int x = (int)((unsigned)h + (unsigned)kFp64NoNan);
+    return x > 0 ? x : 0;
+#endif
+}
+__host__ __device__ inline int fp64_cell_gate(int gate) { return gate < 0 ? gate - 1 : kFp64Pass; }
+// The same from the high word of a best score of the same arithmetic, which needs no slack.
+__host__ __device__ inline int fp64_best_gate(int h) { return h > 0 ? -h - 1 : kFp64Pass; }
 // High word of the gate's value, from the largest high word among a column's
 // q s - w W' (0 if all are negative): rounded up, an infinity or NaN as the largest
 // double.  The cell passes if the sum with its bound's gate is not negative.
@@ -156,7 +184,7 @@ __host__ __device__ inline int fp64_gate_error(double s, double w) {
         return h > 0 ? h : 0;
     }
     // NaN never selects; infinite terms give the score's own infinities and NaN
-    return s != s || w != w || fp64_flat(s, w) ? 0 : 0x7ff00000;
+    return fp64_degenerate(s, w) ? 0 : 0x7ff00000;
 }
 // Errors up to here are within the gates' slack.
 __host__ __device__ inline int fp64_gate_errfree(double m) { return high_word(kFp64GateSlack / 8 * m); }
