@@ -2,6 +2,8 @@
 score: the oracle's bits, and those of bands cut into tiles."""
 from __future__ import annotations
 
+import re
+
 import numpy as np
 import pytest
 
@@ -46,3 +48,49 @@ def test_whole_bands_equal_oracle_and_tiles(gpu_ctx, oracle, kind, n, m):
     assert np.array_equal(p.dist2, d2, equal_nan=True)
     if kind not in ("steps", "signs"):  # infinite or equal scores tie by the thousand there
         check_fp64_indices(oracle, x, m, p.dist2, p.index, idx)
+
+
+# Above 947 bands of 256 diagonals the bands stay whole; two ranges of half the diagonals
+# each are cut into tiles.
+@pytest.mark.parametrize("kind", ["walk", "noise", "sine", "steps", "nan", "signs"])
+@pytest.mark.parametrize("m", [8, 100])
+def test_wide_whole_bands_equal_two_ranges_in_tiles(gpu_ctx, kind, m):
+    n = 243000 + m
+    x = series(kind, n)
+    p = gpu_ctx.selfjoin(x, m)
+    launches = gpu_ctx.last_launch_count
+    pl, mid = n - m + 1, 100001
+    q = gpu_ctx.selfjoin_ranges(x, m, [(m // 4 + 1, mid), (mid, pl)])
+    assert gpu_ctx.last_launch_count >= launches + 4  # another join, seeds and seams twice
+    assert np.array_equal(p.dist2, q.dist2, equal_nan=True) and np.array_equal(p.index, q.index)
+
+
+def block(ctx, x, m, diag, blocklen, q, mu, si):
+    pl = x.size - m + 1
+    t = pl - diag
+    xp = np.append(x, 0.0)
+    prof, idx, tq = np.full(pl, -1.0), np.zeros(pl, dtype=np.int64), q.copy()
+    ctx.eval_diag_block_triangle(prof[:t], idx[:t], prof[diag:], idx[diag:], tq, blocklen, t, xp,
+                                 xp[diag:], m, si, mu, si[diag:], mu[diag:], diag, 0)
+    return prof, idx, tq
+
+
+# The budget that leaves no room for tiles is what the call itself says it needs.
+@pytest.mark.parametrize("kind", ["walk", "steps"])
+@pytest.mark.parametrize("blocklen,diag", [(1, 5), (31, 900), (100, 40), (500, 3000), (777, 17), (2100, 60)])
+def test_block_in_tiles_equals_whole_bands_by_path(gpu_ctx, kind, blocklen, diag):
+    m = 32
+    x = series(kind, 12000)
+    with np.errstate(all="ignore"):
+        mu, si = gpu_ctx.window_stats(x, m)
+    q = gpu_ctx.first_qt(x, m, diag, diag + blocklen)
+    got = block(gpu_ctx, x, m, diag, blocklen, q, mu, si)
+    launches = gpu_ctx.last_launch_count
+    with mp.Context(0, mem_budget_bytes=1) as none, pytest.raises(mp.MpError) as e:
+        block(none, x, m, diag, blocklen, q, mu, si)
+    need = int(re.search(r"needs (\d+) bytes", str(e.value)).group(1))
+    with mp.Context(0, mem_budget_bytes=need) as whole:
+        want = block(whole, x, m, diag, blocklen, q, mu, si)
+        assert whole.last_launch_count == launches - 2  # seeds and seams
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f")

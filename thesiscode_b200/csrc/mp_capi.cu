@@ -153,12 +153,11 @@ int fp64_shards(int64_t PL) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(16, s));
 }
 
-// Diagonals per lane.  Every band walks all of its columns, so the longest
-// band's column count is the critical path whatever R is; R = 8 does the most
-// cells per step and was fastest at every size measured on a B200 (FP64 join,
-// m = 256: n = 16,384 -> 3.2 ms vs 3.6 ms at R = 4 and 5.2 ms at R = 2, even
-// with 63 bands for 148 SMs; n = 524,288 -> 121 vs 190 vs 482 ms).  Only a few
-// hundred diagonals (the kernel API's blocks) leave most lanes of an R = 8
+// Diagonals per lane.  R = 8 does the most cells per step: joins in tiles, R = 8 / 4 / 2,
+// n = 2,500 0.051 / 0.039 / 0.033 ms, 16,384 0.30 / 0.25 / 0.25, 65,536 1.58 / 1.60 / 4.6, 100,000
+// 2.97 / 3.32 / 8.2; whole bands of 180,000 16.4 / 18.8 / 19.3.  (The width of a band decides
+// which of several equal scores it keeps, so the smallest series stay with theirs.)  Only a
+// few hundred diagonals (the kernel API's blocks) leave most lanes of an R = 8
 // band idle; there narrower bands spread the same steps over more warps.
 int pick_fp64_R(int64_t ndiag) {
 #ifdef MPGPU_FP64_FORCE_R

@@ -142,7 +142,7 @@ template <int R>
 __device__ __forceinline__ void finish_row(const Fp64BandParams& P, int shard, int64_t lt, int64_t seg,
                                            bool more, int64_t rb, int64_t t, double score, int j) {
     if (seam_row<R>(t, P.split.L, seg, more)) {
-        const int64_t i = lt * (P.split.L + 32 * R) + t;
+        const int64_t i = lt * fp64_seam_rows(P.split.L, 32 * R) + fp64_seam_slot(t, P.split.L, 32 * R);
         P.split.seam_s[i] = score;
         P.split.seam_j[i] = j;
     } else if (j >= 0) {
@@ -739,7 +739,8 @@ __global__ void __launch_bounds__(32 * kFp64WarpsPerBlock, R == 8 ? 2 : 4)
 // wins ties, as within a tile.
 template <int R>
 __global__ void fp64_seam_kernel(const Fp64BandParams P) {
-    const int64_t lt = blockIdx.x, L = P.split.L, stride = L + 32 * R;
+    const int64_t lt = blockIdx.x, L = P.split.L, stride = L + 32 * R;  // rows of a tile
+    const int64_t slots = fp64_seam_rows(L, 32 * R);
     int64_t band, seg;
     if (!tile_of_pair(lt, P.Tbase, P.g_lo, L, P.nbands, P.split.seg_per_pair, 32 * R, band, seg) ||
         seg == 0)
@@ -755,7 +756,7 @@ __global__ void fp64_seam_kernel(const Fp64BandParams P) {
         for (int64_t k = max((int64_t)0, (x - stride) / L); k <= seg; ++k) {
             const int64_t tk = x - k * L;
             if (tk >= stride || !seam_row<R>(tk, L, k, k < last)) continue;
-            const int64_t i = (lt - (seg - k)) * stride + tk;
+            const int64_t i = (lt - (seg - k)) * slots + fp64_seam_slot(tk, L, 32 * R);
             const int jk = P.split.seam_j[i];
             if (jk >= 0 && (j < 0 || P.split.seam_s[i] > s)) {
                 s = P.split.seam_s[i];
@@ -989,7 +990,7 @@ Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R) {
 
 size_t fp64_split_bytes(const Fp64Split& S, int64_t ndiag, int R) {
     if (S.L == 0) return 0;
-    const size_t rows = (size_t)(S.ntiles * (S.L + 32 * R));
+    const size_t rows = (size_t)(S.ntiles * fp64_seam_rows(S.L, 32 * R));
     return align_up(8 * (size_t)((S.nseg - 1) * ndiag)) + align_up(8 * rows) + align_up(4 * rows);
 }
 
@@ -997,7 +998,7 @@ void fp64_split_carve(Fp64Split& S, int64_t ndiag, int R, char* p) {
     S.seeds = reinterpret_cast<double*>(p);
     p += align_up(8 * (size_t)((S.nseg - 1) * ndiag));
     S.seam_s = reinterpret_cast<double*>(p);
-    p += align_up(8 * (size_t)(S.ntiles * (S.L + 32 * R)));
+    p += align_up(8 * (size_t)(S.ntiles * fp64_seam_rows(S.L, 32 * R)));
     S.seam_j = reinterpret_cast<int*>(p);
 }
 

@@ -57,10 +57,16 @@ struct Fp64Split {
     int64_t seg_per_pair;  // tile numbering: see tile_of_pair
     int64_t ntiles;
     double* seeds;         // [nseg - 1][g_hi - g_lo]: dot product at column (s + 1) L
-    double* seam_s;        // [ntiles][L + 32R] best score of the tile's row t ...
+    double* seam_s;        // [ntiles][fp64_seam_rows] best score of a seam row of the tile ...
     int* seam_j;           // ... and its column, -1: none
 };
 constexpr int64_t kFp64SplitUnit = 16;
+// Rows of a tile that a tile of its band before or after it may meet, too: the first and
+// the last `span` (= 32R) of its L + span.  Their number, and row t's place among them.
+__host__ __device__ inline int64_t fp64_seam_rows(int64_t L, int64_t span) { return span + (L < span ? L : span); }
+__host__ __device__ inline int64_t fp64_seam_slot(int64_t t, int64_t L, int64_t span) {
+    return t < span || L < span ? t : t - L + span;
+}
 // Number of a tile in a list of band pairs (k, nbands - 1 - k), whose lengths are
 // nearly complementary: pair p = lt / seg_per_pair holds the tiles of K columns of
 // band p, then those of band nbands - 1 - p.  False for the unused tail of a pair.
