@@ -9,6 +9,7 @@ import thesiscode_b200 as mp
 from thesiscode_b200 import build
 
 PROGRAM = r"""
+#include <algorithm>
 #include <cstdio>
 #include <vector>
 #include "mp_common.cuh"
@@ -45,6 +46,17 @@ int main() {
                 ++bad;
             }
         }
+    // in the place of a join's key shards but one (16 bytes per window each, 32 MB in all)
+    for (int64_t n : {600, 1000, 2500, 4000, 8000, 16384, 40000, 65536, 100000, 131072, 180000, 240000}) {
+        const int64_t shards = std::max<int64_t>(1, std::min<int64_t>(16, 2000000 / n));
+        const size_t room = (size_t)(16 * n * (shards - 1));
+        const int R = n < 2065 ? 4 : 8;
+        const Fp64Split S = fp64_split_plan(n, 17, n, R, room), T = fp64_split_plan(n, 17, n, R);
+        const bool ok = S.L >= T.L && S.L % kFp64SplitUnit == 0 && S.L < n - 17 &&
+                        fp64_split_bytes(S, n - 17, R) <= room && fp64_split_plan(n, 17, n, R, 1000).L == 0;
+        if (!ok) std::printf("n %lld: L %lld (%lld with room)\n", (long long)n, (long long)S.L, (long long)T.L);
+        bad += !ok;
+    }
     return bad != 0;
 }
 """

@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(kSeedThreads)
 
 }  // namespace
 
-Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R) {
+Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R, size_t room) {
     Fp64Split S{};
     const int64_t span = 32 * R, nd = g_hi - g_lo;
     if (nd <= 0) return S;
@@ -980,12 +980,14 @@ Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R) {
     const int64_t cols = nbands * (Tbase - g_lo) - span * (nbands * (nbands - 1) / 2);
     int64_t L = std::max<int64_t>(cols / (5 * warps), 32);
     L = (L + kFp64SplitUnit - 1) / kFp64SplitUnit * kFp64SplitUnit;
-    if (Tbase - g_lo <= L) return S;
-    S.L = L;
-    S.nseg = (Tbase - g_lo + L - 1) / L;
-    int64_t nb = 0;
-    fp32_tile_plan(Tbase, g_lo, g_hi, L, R, nb, S.seg_per_pair, S.ntiles);
-    return S;
+    for (; L < Tbase - g_lo; L += (L / 2 + kFp64SplitUnit - 1) / kFp64SplitUnit * kFp64SplitUnit) {
+        S.L = L;
+        S.nseg = (Tbase - g_lo + L - 1) / L;
+        int64_t nb = 0;
+        fp32_tile_plan(Tbase, g_lo, g_hi, L, R, nb, S.seg_per_pair, S.ntiles);
+        if (fp64_split_bytes(S, nd, R) <= room) return S;
+    }
+    return Fp64Split{};
 }
 
 size_t fp64_split_bytes(const Fp64Split& S, int64_t ndiag, int R) {

@@ -260,8 +260,9 @@ inline double fp64_threshold_tiny(double m) { return std::ldexp(m, -40); }
 template <int R>
 void launch_fp64_band(const Fp64BandParams& P, cudaStream_t s);
 // Split plan of a band join over diagonals [g_lo, g_hi) of Tbase columns (L = 0:
-// whole bands), the bytes its buffers need, and the buffers carved from `base`.
-Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R);
+// whole bands), with tiles long enough for buffers of `room` bytes; the bytes its buffers
+// need, and the buffers carved from `base`.
+Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R, size_t room = SIZE_MAX);
 size_t fp64_split_bytes(const Fp64Split& S, int64_t ndiag, int R);
 void fp64_split_carve(Fp64Split& S, int64_t ndiag, int R, char* base);
 // Running dot products at the tiles' first columns: Ah the series along columns,
