@@ -417,8 +417,11 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
         // Without room for the tiles' buffers (a budget or lent scratch of just the size that
         // mp_selfjoin_scratch_bytes states), longer tiles take the place of the key shards: join
         // of 2,500 samples 0.23 ms, 0.05 with room, 0.89 as whole bands; 65,536 1.77, 1.58, 6.4;
-        // 240,000 18.1, 14.7, 23.0.
-        if (!split && extra > 0) {
+        // 240,000 18.1, 14.7, 23.0.  Not for a lent scratch and many bands, though: the server's
+        // requests run side by side, and the whole bands of several keep the chip busy without
+        // the tiles' first dot products (8 of 200,000 samples on 4 slots 88 ms, 106 in tiles; 4 of
+        // 130,000 26.8, 25.2).
+        if (!split && extra > 0 && !(ctx->lent && ndiag > 600 * 256)) {
             shards = 1;
             base = fp64_scratch(n, m, ndiag, !o_dev, shards);
             plan(ctx->arena_bytes - std::min(ctx->arena_bytes, align_up(base)));
