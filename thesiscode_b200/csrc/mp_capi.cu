@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/mpgpu.h"
+#include "mp_arena.h"
 #include "mp_common.cuh"
 #include "mp_kernels.h"
 #include "mp_serve.h"
@@ -26,13 +27,11 @@ struct mp_context {
     size_t budget = 0;
     std::string last_error;
     int64_t launches = 0;
-    void* arena = nullptr;
-    size_t arena_bytes = 0;
+    Arena arena;
     // while a caller's buffer is lent as the scratch (ctx_lend_scratch), the
     // context's own arena waits here
     bool lent = false;
-    void* own_arena = nullptr;
-    size_t own_bytes = 0;
+    Arena own;
     bool timing = false;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     double phase_ms[3] = {-1.0, -1.0, -1.0};
@@ -46,17 +45,15 @@ void ctx_lend_scratch(mp_context* ctx, void* scratch, size_t bytes) {
     if (!ctx) return;
     if (scratch) {
         if (!ctx->lent) {
-            ctx->own_arena = ctx->arena;
-            ctx->own_bytes = ctx->arena_bytes;
+            ctx->own = ctx->arena;
             ctx->lent = true;
         }
-        ctx->arena = scratch;
-        ctx->arena_bytes = bytes;
+        ctx->arena = Arena{};
+        ctx->arena.p = scratch;
+        ctx->arena.bytes = bytes;
     } else if (ctx->lent) {
-        ctx->arena = ctx->own_arena;
-        ctx->arena_bytes = ctx->own_bytes;
-        ctx->own_arena = nullptr;
-        ctx->own_bytes = 0;
+        ctx->arena = ctx->own;
+        ctx->own = Arena{};
         ctx->lent = false;
     }
 }
@@ -108,40 +105,47 @@ struct Carve {
     }
 };
 
+// Device memory as an Arena sees it.
+struct DeviceMem {
+    cudaError_t error = cudaSuccess;
+    void* alloc(size_t bytes) {
+        void* p = nullptr;
+        error = cudaMalloc(&p, bytes);
+        if (error != cudaSuccess) cudaGetLastError();
+        return error == cudaSuccess ? p : nullptr;
+    }
+    void free(void* p) { cudaFree(p); }
+    size_t room() {
+        size_t left = 0, total = 0;
+        if (cudaMemGetInfo(&left, &total) != cudaSuccess) cudaGetLastError();
+        return left;
+    }
+};
+
 int reserve(mp_context* ctx, size_t bytes) {
     if (ctx->budget && bytes > ctx->budget)
         return fail(ctx, MP_ERR_BUDGET, "request needs %zu bytes of device scratch, budget is %zu",
                     bytes, ctx->budget);
-    if (bytes <= ctx->arena_bytes) return MP_OK;
+    if (bytes <= ctx->arena.bytes) return MP_OK;
     if (ctx->lent)  // a lent scratch is never replaced
         return fail(ctx, MP_ERR_BUDGET, "lent scratch holds %zu bytes, the call needs %zu",
-                    ctx->arena_bytes, bytes);
-    if (ctx->arena) cudaFree(ctx->arena);
-    ctx->arena = nullptr;
-    ctx->arena_bytes = 0;
-    cudaError_t e = cudaMalloc(&ctx->arena, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
+                    ctx->arena.bytes, bytes);
+    DeviceMem mem;
+    if (!arena_reserve(ctx->arena, bytes, mem))
         return fail(ctx, MP_ERR_OUT_OF_MEMORY, "cudaMalloc(%zu) failed: %s", bytes,
-                    cudaGetErrorString(e));
-    }
-    ctx->arena_bytes = bytes;
+                    cudaGetErrorString(mem.error));
     return MP_OK;
 }
-
 
 // reserve() of `base` bytes and, where the budget, a lent scratch and the device
 // have room, `extra` more from align_up(base) on that the call can do without
 // (`has_extra`: they are there).
 int reserve_with(mp_context* ctx, size_t base, size_t extra, bool& has_extra) {
-    has_extra = false;
     const size_t all = align_up(base) + extra;
-    if (extra > 0 && (!ctx->budget || all <= ctx->budget) &&
-        (all <= ctx->arena_bytes || (!ctx->lent && reserve(ctx, all) == MP_OK))) {
-        has_extra = true;
-        return MP_OK;
-    }
-    return reserve(ctx, base);
+    DeviceMem mem;
+    has_extra = extra > 0 && (!ctx->budget || all <= ctx->budget) &&
+                (all <= ctx->arena.bytes || (!ctx->lent && arena_try(ctx->arena, base, all, mem)));
+    return has_extra ? MP_OK : reserve(ctx, base);
 }
 
 // Key shards spread the 64-bit max reductions of concurrently running bands
@@ -334,7 +338,7 @@ int mp_context_create(int device, size_t mem_budget_bytes, mp_context** out) {
 int mp_context_destroy(mp_context* ctx) {
     if (!ctx) return MP_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
-    void* own = ctx->lent ? ctx->own_arena : ctx->arena;
+    void* own = ctx->lent ? ctx->own.p : ctx->arena.p;
     if (own) cudaFree(own);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
@@ -424,11 +428,11 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
         if (!split && extra > 0 && !(ctx->lent && ndiag > 600 * 256)) {
             shards = 1;
             base = fp64_scratch(n, m, ndiag, !o_dev, shards);
-            plan(ctx->arena_bytes - std::min(ctx->arena_bytes, align_up(base)));
+            plan(ctx->arena.bytes - std::min(ctx->arena.bytes, align_up(base)));
             split = extra > 0;
             if (!split) shards = fp64_shards(PL);
         }
-        Carve cv{(char*)ctx->arena};
+        Carve cv{(char*)ctx->arena.p};
         double* Apad = cv.take<double>(n + 1);
         double* cs = cv.take<double>(n);
         double* cs2 = cv.take<double>(n);
@@ -486,7 +490,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
             P.counter = counter;
             if (split && splits[i].L > 0) {
                 P.split = splits[i];
-                fp64_split_carve(P.split, nd, R, (char*)ctx->arena + align_up(base));
+                fp64_split_carve(P.split, nd, R, (char*)ctx->arena.p + align_up(base));
             }
             return P;
         };
@@ -554,7 +558,7 @@ int selfjoin_ranges(mp_context* ctx, const double* A, int64_t n, int64_t m, int 
                                         kFp32R);
     rc = reserve(ctx, fp32_scratch(n, m, !o_dev, ranges.size()) + (guarded ? guard_scratch(n, m) : 0));
     if (rc) return rc;
-    Carve cv{(char*)ctx->arena};
+    Carve cv{(char*)ctx->arena.p};
     double* Apad = cv.take<double>(n + kFp32Pad);
     int* nchg = cv.take<int>(n);
     const int64_t nblk = (n + kThreads - 1) / kThreads;
@@ -749,7 +753,7 @@ int mp_window_stats(mp_context* ctx, const double* A, int64_t n, int64_t m, doub
     const int64_t PL = n - m + 1;
     int rc = reserve(ctx, align_up(8 * n) * 3 + align_up(8 * PL) * 2 + 4096);
     if (rc) return rc;
-    Carve cv{(char*)ctx->arena};
+    Carve cv{(char*)ctx->arena.p};
     double* Ad = cv.take<double>(n);
     double* cs = cv.take<double>(n);
     double* cs2 = cv.take<double>(n);
@@ -801,7 +805,7 @@ int mp_prescrimp(mp_context* ctx, const double* A, int64_t n, int64_t m, double 
     if (!o_dev) bytes += align_up(8 * (size_t)PL) * 2;
     int rc = reserve(ctx, bytes);
     if (rc) return rc;
-    Carve cv{(char*)ctx->arena};
+    Carve cv{(char*)ctx->arena.p};
     double* Ad = cv.take<double>(n);
     double* cs = cv.take<double>(n);
     double* cs2 = cv.take<double>(n);
@@ -866,7 +870,7 @@ int mp_first_qt(mp_context* ctx, const double* A, int64_t n, int64_t m, int64_t 
     const int64_t nd = d_hi - d_lo;
     int rc = reserve(ctx, align_up(8 * n) + align_up(8 * std::max<int64_t>(nd, 1)) + 4096);
     if (rc) return rc;
-    Carve cv{(char*)ctx->arena};
+    Carve cv{(char*)ctx->arena.p};
     double* Ad = cv.take<double>(n);
     double* q = cv.take<double>(nd);
     MP_CUDA(ctx, cudaMemcpyAsync(Ad, A, 8 * n, cudaMemcpyDefault, st));
@@ -931,7 +935,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     bool has_split = false;
     int rc = reserve_with(ctx, need, fp64_split_bytes(split, nq, R), has_split);
     if (rc) return rc;
-    Carve cv{(char*)ctx->arena};
+    Carve cv{(char*)ctx->arena.p};
     double4* colrec = cv.take<double4>(nrec);
     double4* rowrec = cv.take<double4>(nrec);
     double* q = cv.take<double>(nq);
@@ -1008,7 +1012,7 @@ int mp_eval_diag_block_triangle(mp_context* ctx, double* prof_colmin, int64_t* i
     P.counter = counter;
     if (has_split) {
         P.split = split;
-        fp64_split_carve(P.split, nq, R, (char*)ctx->arena + align_up(need));
+        fp64_split_carve(P.split, nq, R, (char*)ctx->arena.p + align_up(need));
         launch_fp64_seeds(P, ah, T + m, av, T + m, m, PrefixSums{}, st);
         MP_LAUNCHED(ctx);
         ++ctx->launches;  // the rows that two tiles meet
