@@ -77,3 +77,14 @@ def test_fp64_join_in_its_stated_scratch(gpu_ctx):
     with mp.Context(0, mem_budget_bytes=budget) as stated:
         t = [ms(lambda: c.selfjoin(x, m, out=out), runs=30) for c in (gpu_ctx, stated)]
     assert t[1] < 4.0 * t[0], t
+
+
+# A walk takes 1.7 ms a call; with a NaN, whose stretches' anchors are summed the plain way,
+# 2.4 where every anchor was, and 7.1 where both ways were taken one after the other.
+def test_fp32_join_with_a_nan_in_long_windows(gpu_ctx):
+    n, m = 60000, 8192
+    t = []
+    for kind in ("walk", "nan"):
+        x, out = on_gpu(series(kind, n), m)
+        t.append(ms(lambda: gpu_ctx.selfjoin(x, m, precision=mp.FP32_REANCHOR, out=out)))
+    assert t[1] < 3.0 * t[0], t

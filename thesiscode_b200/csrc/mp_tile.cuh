@@ -21,7 +21,9 @@ constexpr int kTileR = 8;  // diagonals per lane
 // Four instructions per 4 terms leave the other warps the issue slots and registers
 // that 32 multiply-adds and their operands took.  n = 300,007, m = 1000, K = 256
 // (3.9 products per cell): 23.5 -> 19.0 ms.
-// A stretch with an infinity or NaN is summed the plain way: 0 times it is NaN.
+// A stretch with an infinity or NaN is summed the plain way from its first term on: 0
+// times it is NaN (60,000 samples, m = 8192, a NaN in the middle: 1.4 ms a join; 4.7 with
+// all stages before it and its sums kept in memory).
 constexpr int kAnchorStep = 128;                       // terms k' per stage
 constexpr int kAnchorY = (kAnchorStep + 256) / 8 * 12;  // element i at i + 4 (i / 8): conflict-free
 constexpr int kAnchorBytes = 8 * (kAnchorStep + 8 + kAnchorY + 256);
@@ -32,13 +34,15 @@ static_assert(8 * (kAnchorChunk + (32 * kTileR + kAnchorChunk) * 9 / 8) <= kAnch
 // (Host-callable, so the rule can be checked without a GPU.)
 __host__ __device__ inline int anchor_terms(int64_t m) { return m < (int64_t(1) << 30) ? (int)m + 7 : 0; }
 
-// The plain way.  The series terms are staged CHUNK at a time: the column's A[j0 + k]
-// and the warp's rows A[j0 + gb + i], i < 32R + chunk, skewed by one double per 8 so
-// that lanes reading rows 8 apart hit distinct banks.
+// The plain way, the lane's sums to out[0 .. 7] (in `area` too, once the terms have been
+// read).  The series terms are staged CHUNK at a time: the column's A[j0 + k] and the
+// warp's rows A[j0 + gb + i], i < 32R + chunk, skewed by one double per 8 so that lanes
+// reading rows 8 apart hit distinct banks.
 template <int CHUNK>
 __device__ __noinline__ void tile_anchor_scalar(const double* A, int64_t m, int64_t j0, int64_t gb, int lane,
-                                                char* area, double (&q)[kTileR]) {
+                                                char* area, double* out) {
     constexpr int R = kTileR;
+    double q[R];
 #pragma unroll
     for (int a = 0; a < R; ++a) q[a] = 0.0;
     {
@@ -83,6 +87,8 @@ __device__ __noinline__ void tile_anchor_scalar(const double* A, int64_t m, int6
         }
         __syncwarp();
     }
+#pragma unroll
+    for (int a = 0; a < R; ++a) out[a] = q[a];
 }
 
 // FP64 re-anchor of a tile: minus the covariance at its first column j0 of the lane's
@@ -125,7 +131,7 @@ __device__ __forceinline__ void tile_anchor(const Fp32TileParams& P, int64_t j0,
             finite = finite && isfinite(ry[i]);
             sy[32 * i + lane + 4 * (4 * i + (lane >> 3))] = ry[i];
         }
-        __syncwarp();
+        if (!__all_sync(kFullMask, finite)) break;
         if (k0 + kAnchorStep < terms) fetch(k0 + kAnchorStep);
         const double* x = sx + 8 + lc - lr;
         const double* y = sy + 12 * lr + lc;
@@ -138,7 +144,6 @@ __device__ __forceinline__ void tile_anchor(const Fp32TileParams& P, int64_t j0,
             for (int p = 0; p < 4; ++p) mma_f64(c[p], a, y[96 * p + e]);
         }
     }
-    double q[kTileR];
     if (__all_sync(kFullMask, finite)) {
         // c[p][h] is diagonal 8 (8p + 2 lc + h) + lr of the band
 #pragma unroll
@@ -146,12 +151,13 @@ __device__ __forceinline__ void tile_anchor(const Fp32TileParams& P, int64_t j0,
             sq[8 * (8 * p + 2 * lc) + lr] = c[p][0];
             sq[8 * (8 * p + 2 * lc + 1) + lr] = c[p][1];
         }
-        __syncwarp();
-#pragma unroll
-        for (int a = 0; a < kTileR; ++a) q[a] = sq[8 * lane + a];
     } else {
-        tile_anchor_scalar<kAnchorChunk>(P.A, P.m, j0, gb, lane, area, q);
+        tile_anchor_scalar<kAnchorChunk>(P.A, P.m, j0, gb, lane, area, sq + 8 * lane);
     }
+    __syncwarp();
+    double q[kTileR];
+#pragma unroll
+    for (int a = 0; a < kTileR; ++a) q[a] = sq[8 * lane + a];
     __syncwarp();
     const double mu0 = (double)P.m * __ldg(P.mean + j0);
 #pragma unroll
