@@ -177,8 +177,8 @@ __device__ __forceinline__ double quotient(double a, double b, double r) {
     const double q = __dmul_rn(a, r);
     const double z = __fma_rn(__fma_rn(-b, q, a), r, q);
     const double x = fabs(a);
-    if (x > 1e-280 && x < 1e280) return z;
-    return plain_division(a, b);
+    if (x <= 1e-280 || x >= 1e280) return plain_division(a, b);
+    return z;  // NaN, too
 }
 __device__ __forceinline__ void stat_block(const double* __restrict__ A, int64_t m, int64_t PL, int64_t base,
                                            double* __restrict__ mean_out, double* __restrict__ norm_out,
