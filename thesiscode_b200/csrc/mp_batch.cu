@@ -118,7 +118,9 @@ __global__ void batch_pack_kernel(const BatchSeries* __restrict__ S, const doubl
     FOR_SERIES_ELEMS(s.PL + kPad) {
         pack_fp32_record(A + s.a_off, s.m, s.PL, kR / 2, mean + s.w_off, norm + s.w_off, i,
                          rowrec + 2 * s.r_off, colrec + 2 * s.r_off);
-        if (i < s.PL) key[s.k_off + i] = (unsigned long long)ulim_key[blockIdx.y] << 32;
+        if (i < s.PL)
+            key[s.k_off + i] =
+                fp32_first_key((unsigned long long)ulim_key[blockIdx.y] << 32, norm[s.w_off + i]);
     }
 }
 

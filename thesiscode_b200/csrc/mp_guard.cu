@@ -77,10 +77,8 @@ __device__ __forceinline__ unsigned long long ld_key(const unsigned long long* k
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(key));
     return v;
 }
-// Bit pattern of the key's distance, 0 where it is negative (any such cell goes on).
 __device__ __forceinline__ unsigned key_bound(unsigned long long key) {
-    const unsigned hi = (unsigned)(key >> 32);
-    return (hi & 0x80000000u) ? hi & 0x7fffffffu : 0u;
+    return fp32_key_bound((unsigned)(key >> 32), false);
 }
 
 struct GuardSmem {

@@ -480,11 +480,8 @@ __device__ __forceinline__ unsigned ld_key_hi(const unsigned long long* key) {
                  : "l"(reinterpret_cast<const unsigned*>(key) + 1));
     return v;
 }
-// Where a row starts: just above every tagged distance that could tie the key
-// (2^-15 steps), 0 for a key below 0 (every negative distance goes on).
-__device__ __forceinline__ unsigned key_bound(unsigned hi) {
-    return (hi & 0x80000000u) ? (hi & 0x7fffff00u) + 0x100u : 0u;
-}
+// Where a row starts.
+__device__ __forceinline__ unsigned key_bound(unsigned hi) { return fp32_key_bound(hi, true); }
 
 // The warp's shared memory for a tile.
 struct TileSmem {

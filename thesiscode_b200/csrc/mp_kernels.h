@@ -331,6 +331,23 @@ __global__ void pack_fp32_kernel(const double* A, int64_t m, int64_t PL, int H, 
                                  unsigned long long* key, unsigned long long init, const Fp32TileParams P,
                                  Fp32TileParams* desc, unsigned long long* counter);
 
+// A window's key before any candidate: no neighbour, at u = 1 + 1/m (`init`).  A flat
+// window (NaN inverse norm), which never gets one, starts at the largest key, so that the
+// gates need not wait for its first.
+constexpr unsigned long long kFp32FlatKey = ~0ull;
+__host__ __device__ __forceinline__ unsigned long long fp32_first_key(unsigned long long init, double norm) {
+    return norm == norm ? init : kFp32FlatKey;
+}
+// Bit pattern of the largest distance u that still concerns a key's window, from the
+// key's high word: 0 where the key's own is negative (any such cell goes on), and for a
+// flat window.  With `tags`, just above every tagged distance that could tie the key
+// (2^-15 steps).
+__host__ __device__ __forceinline__ unsigned fp32_key_bound(unsigned hi, bool tags) {
+    if (!(hi & 0x80000000u)) return 0u;
+    if (tags) return ((hi & 0x7fffff00u) + 0x100u) & 0x7fffffffu;  // a flat window's wraps to 0
+    return hi == 0xffffffffu ? 0u : hi & 0x7fffffffu;
+}
+
 // FP32 profile keys, min-merged: (ordered u << 32) | neighbour.  With group
 // keys (the guarded form) the tile kernel finds a minimum's lane but not which
 // of the lane's R diagonals holds it, so its keys name a group of adjacent

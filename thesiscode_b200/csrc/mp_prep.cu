@@ -202,7 +202,7 @@ __global__ void pack_fp32_kernel(const double* __restrict__ A, int64_t m, int64_
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < count;
          j += (int64_t)gridDim.x * blockDim.x) {
         pack_fp32_record(A, m, PL, H, mean, norm, j, rowrec, colrec);
-        if (j < PL) key[j] = init;
+        if (j < PL) key[j] = fp32_first_key(init, norm[j]);
         if (j == 0 && desc) *desc = P;
         if (j == 0 && counter) *counter = 0;
     }
