@@ -1,5 +1,5 @@
-"""Rules of the FP32 forms' gates on CPU: what bound a key sets (a host program against the
-header's functions)."""
+"""Rules of the FP32 forms' gates on CPU: what bound a key sets, and which joins go behind the
+gate (host programs against the header's functions)."""
 from __future__ import annotations
 
 import subprocess
@@ -44,10 +44,42 @@ int main() {
 }
 """
 
+# Joins whose tiles of 1,024 columns are one wave of the selecting passes' resident warps (12
+# on each of 148 SMs) select in every pass.
+WAY = r"""
+#include <cstdio>
+#include "mp_common.cuh"
+#include "mp_kernels.h"
+using namespace mpgpu;
+int main() {
+    int bad = 0;
+    for (const long long m : {170ll, 256ll, 400ll, 1024ll})
+        for (long long n = 24000; n < 60000; n += 500) {
+            Fp32TileParams P{};
+            P.m = m;
+            P.PL = n - m + 1;
+            long long tiles = 0;  // with work (a pair of bands leaves some numbers unused)
+            for (long long g = m / 4 + 1; g < P.PL; g += 256) tiles += (P.PL - g + 1023) / 1024;
+            const Fp32Way way = fp32_way_of(&P, 1);
+            if (tiles <= 148 * 12 - 60 && way != kFp32Dense) ++bad, std::printf("%lld / %lld dense\n", n, m);
+            if (tiles > 148 * 12 + 120 && way != kFp32Gate) ++bad, std::printf("%lld / %lld gate\n", n, m);
+        }
+    return bad != 0;
+}
+"""
 
-def test_bounds_of_keys(tmp_path):
+
+def run(tmp_path, program):
     src, exe = tmp_path / "rule.cu", tmp_path / "rule"
-    src.write_text(PROGRAM)
+    src.write_text(program)
     subprocess.run([build.NVCC, *build.NVCC_FLAGS, str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_bounds_of_keys(tmp_path):
+    run(tmp_path, PROGRAM)
+
+
+def test_one_wave_of_tiles_selects(tmp_path):
+    run(tmp_path, WAY)

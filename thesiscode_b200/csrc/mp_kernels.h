@@ -445,8 +445,12 @@ void launch_fp32_join(const Fp32TileParams* series_dev, int nseries, int64_t tot
 //   m = 160   32,768 0.25 / 0.26      65,536 0.71 / 0.73      262,144 8.7 / 10.9
 //   m = 256   16,384 0.12 / 0.10      32,768 0.24 / 0.30      131,072 2.19 / 2.80
 //   m = 1024  16,384 0.13 / 0.11      32,768 0.25 / 0.29
+// (30,000 / 170: 0.24 / 0.18.)  Up to about 30,700 samples the selecting passes' tiles are one
+// wave of their 1,776 resident warps; the gate, which spreads over more, gains nothing there.
+// Other data moves the lines: noisy steps of 150 samples, m = 96 to 130 0.86 to 0.89 times as
+// fast behind the gate, white noise 1.2 to 1.3 times.
 __host__ __device__ inline bool fp32_gate_pays(int64_t m, int64_t PL) {
-    return m >= 96 && PL >= (m >= 160 ? 25000 : m >= 128 ? 90000 : 200000);
+    return m >= 96 && PL >= (m >= 160 ? 30700 : m >= 128 ? 90000 : 200000);
 }
 // The way of a launch over these series.
 inline Fp32Way fp32_way_of(const Fp32TileParams* P, size_t n) {
