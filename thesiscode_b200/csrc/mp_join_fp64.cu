@@ -65,13 +65,13 @@
 //
 // What bounds it: the FP64 pipe takes a warp's instruction every 2.2 cycles, 4
 // per cell (33 of a step's 60 instructions at R = 8); other instructions cost it
-// about 0.7 cycles each.  n = 1,048,576, m = 256: 237 ms, from 441 ms with the
+// about 0.7 cycles each.  n = 1,048,576, m = 256: 243 ms, from 441 ms with the
 // selection tested per step in FP64 and the bands in order of length (one gate per
 // pass and 5 operations: 254 ms; that with a pass's two chunks as a loop 271 ms;
 // 3 CTAs of 4 warps per SM at 168 registers spill, 273 ms).  Short windows have rows
 // of unlike best scores side by side, and one bound for a pass's 23 rows and 16
 // columns opened a quarter of the passes at m = 64 where 2% select (n = 600,000: 164
-// ms; a bound per 15 rows and 8 columns 134; per 8 rows and a column 101, 96 with the passes
+// ms; a bound per 15 rows and 8 columns 134; per 8 rows and a column 101, 97 with the passes
 // after an open one straight).  With
 // fewer bands than resident warps the longest band sets the time; then the bands
 // are cut into tiles (Fp64Split).
@@ -138,10 +138,10 @@ template <int R>
 __host__ __device__ __forceinline__ bool seam_row(int64_t t, int64_t L, int64_t seg, bool more) {
     return (seg > 0 && t < 32 * R) || (more && t >= L);
 }
-template <int R>
+template <int R, bool WHOLE>
 __device__ __forceinline__ void finish_row(const Fp64BandParams& P, int shard, int64_t lt, int64_t seg,
                                            bool more, int64_t rb, int64_t t, double score, int j) {
-    if (seam_row<R>(t, P.split.L, seg, more)) {
+    if (!WHOLE && seam_row<R>(t, P.split.L, seg, more)) {
         const int64_t i = lt * fp64_seam_rows(P.split.L, 32 * R) + fp64_seam_slot(t, P.split.L, 32 * R);
         P.split.seam_s[i] = score;
         P.split.seam_j[i] = j;
@@ -461,7 +461,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     const int64_t L = P.split.L;
     const unsigned j0 = (unsigned)(seg * L);
     if ((int64_t)j0 >= jmax) return;
-    const bool more = L > 0 && j0 + L < jmax;  // the band goes on in the next tile
+    const bool more = !WHOLE && L > 0 && j0 + L < jmax;  // the band goes on in the next tile
     const unsigned jend = more ? j0 + (unsigned)L : (unsigned)jmax;
     const int64_t rb = gb + j0;  // row t = 0 of the tile
 
@@ -643,7 +643,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
         if (lane < R * kU) {
             const int e = (sf + lane / R) * (R + 1) + lane % R;
             const int j = sm.src[e];
-            finish_row<R>(P, shard, lt, seg, more, rb, (int64_t)(jc - j0) + lane, sm.best[e], j);
+            finish_row<R, WHOLE>(P, shard, lt, seg, more, rb, (int64_t)(jc - j0) + lane, sm.best[e], j);
         }
         // the incoming groups and columns begin at their thresholds
         const double bound = fp64_bound(t, sw.x, sw.y);
@@ -688,7 +688,7 @@ __device__ __forceinline__ void band_fp64(const Fp64BandParams& P, int64_t band,
     for (int i = lane; i < 32 * R; i += 32) {
         const int e = BandSmem<R>::wrap(sf + i / R) * (R + 1) + i % R;
         const int j = sm.src[e];
-        finish_row<R>(P, shard, lt, seg, more, rb, tend + i, sm.best[e], j);
+        finish_row<R, WHOLE>(P, shard, lt, seg, more, rb, tend + i, sm.best[e], j);
     }
     __syncwarp();
 
@@ -968,9 +968,9 @@ Fp64Split fp64_split_plan(int64_t Tbase, int64_t g_lo, int64_t g_hi, int R, size
     const int64_t nbands = (nd + span - 1) / span;
     // Whole bands keep the chip busy once there are about as many as resident
     // warps (8 per SM), and the dot products of the tiles' first columns cost two
-    // more FP64 operations per cell.  Whole calls, tiles against whole bands: n =
-    // 2,500 0.14 / 1.0 ms; 16,384 0.64 / 2.7; 65,536 (256 bands) 2.8 / 6.8;
-    // 200,000 (780 bands) 15.8 / 19.5; 260,000 (1,015) 25.5 / 26.5; 300,000 33.5 / 31.3.
+    // more FP64 operations per cell.  Joins in tiles (with their seeds) against whole bands: n =
+    // 2,500 0.08 / 0.81 ms; 16,384 0.6 / 2.2; 65,536 (256 bands) 2.3 / 6.4; 180,000 (702)
+    // 12 / 16.4; 240,000 (936) 21 / 23.3; whole calls of 260,000 25.5 / 26.5, 300,000 33.5 / 31.3.
     const int64_t warps = (int64_t)sm_count() * 8;
     if (nbands > warps * 4 / 5) return S;
     // About 5 tiles per warp (10 and 20 measured the same; 2 per warp 16.8 ms at n =
