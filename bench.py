@@ -266,9 +266,9 @@ def c3_sample(ctx, width: int, k: int):
         j64 = ctx.last_phase_ms()[1]
         rec = {"diagonals": [lo, hi], "cells": cells,
                "fp64_cells_per_s": cells / (j64 * 1e-3),
-               "note": "a sample of few long diagonals: the FP64 form's bands (256 diagonals "
-                       "each) fill under one wave of the GPU, so its rate here is not the full "
-                       "join's; the FP32 form's tiles fill it"}
+               "note": "a sample of few long diagonals: the FP64 form cuts its 128 bands (256 "
+                       "diagonals each) into tiles of columns, whose first dot products it "
+                       "computes beforehand, so its rate here is not the full join's"}
         # each form at its re-anchor interval: k for the FP32 form, the guarded
         # form's own default (512) for it
         for form, prec, kf in (("fp32", mp.FP32_REANCHOR, k), ("guarded", mp.FP32_GUARDED, 512)):

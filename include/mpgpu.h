@@ -70,7 +70,9 @@ int mp_context_destroy(mp_context* ctx);
 /* Text of the last error recorded on ctx (never NULL). */
 const char* mp_last_error(const mp_context* ctx);
 const char* mp_status_string(int status);
-/* Device bytes one self-join of (n, m, precision) needs in ctx's scratch. */
+/* Device bytes one self-join of (n, m, precision) needs in ctx's scratch: the
+ * smallest budget that admits it.  MP_PREC_FP64 takes up to 64 MB more where the
+ * budget and the device have it, and is then faster. */
 size_t mp_selfjoin_scratch_bytes(int64_t n, int64_t m, int precision);
 
 /*

@@ -6,7 +6,7 @@
 //    scrimppp/src/ScrimpSequOpt.cpp:33-79, evaluated with explicitly rounded
 //    operations (__dadd_rn/__dmul_rn/... are never contracted into FMAs) so the
 //    result is bit-identical to the reference built with IEEE semantics.  The
-//    prefix sums are a dependent chain and run on one thread.
+//    two prefix sums are dependent chains, each on a lane of its own (prefix_block).
 //  * FP64 Welford (FP32 form): Welford's mean/M2 update slides over chunks of
 //    256 windows, restarting from a fresh Welford pass at every chunk start;
 //    exact zero-variance windows are found from the places where the value

@@ -273,7 +273,7 @@ __device__ __forceinline__ void stat_block(const double* __restrict__ A, int64_t
 // Row records are stored as pairs (x[j], x[j+H]) for the f32x2 datapath:
 //   rowrec[j] = {df[j], df[j+H], dg[j], dg[j+H], nn[j], nn[j+H], 1, 1}
 // Column records duplicate and negate the column terms:
-//   colrec[p] = {-df[p], -df[p], -dg[p], -dg[p], nn[p], nn[p], 0, 0}
+//   colrec[p] = {-df[p], -df[p], -dg[p], -dg[p], nn[p], nn[p], 1/nn[p], 1/nn[p]}
 // Entries past PL read as df = dg = 0, nn = NaN.
 __device__ __forceinline__ void fp32_terms(const double* A, int64_t m, int64_t PL,
                                            const double* mean, const double* norm, int64_t i,
