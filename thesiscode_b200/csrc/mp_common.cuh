@@ -198,6 +198,14 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
     return d;
 }
 
+// 8-byte asynchronous copy global -> shared that writes zero where !inside.
+__device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
+                 "r"(inside ? 8 : 0)
+                 : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // FP64 matrix instruction: C (8 x 8) += A (8 x 4) B (4 x 8) over a warp.  Lane l
 // holds A[l / 4][l % 4], B[l % 4][l / 4] and C[l / 4][2 (l % 4) + {0, 1}].  Each

@@ -64,13 +64,6 @@ constexpr int kGuardWarps = 4;
 constexpr int kGuardBlocksPerSm = 3;  // 8.2 ms against 8.8 at 2 (no spill) on the series above
 __device__ __forceinline__ int wrap_group(int s) { return s < kGroups ? s : s - kGroups; }
 
-// 8-byte asynchronous copy that writes zero where !inside.
-__device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
-                 "r"(inside ? 8 : 0)
-                 : "memory");
-}
 // A key as it stands (merged meanwhile by other warps).
 __device__ __forceinline__ unsigned long long ld_key(const unsigned long long* key) {
     unsigned long long v;

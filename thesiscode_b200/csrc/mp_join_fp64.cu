@@ -782,14 +782,6 @@ constexpr int kSeedThreads = 128;
 constexpr int kSeedChunk = 128;
 constexpr int kSeedPrefixChunk = 192;
 
-// 8-byte asynchronous copy that writes zero where !inside.
-__device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
-                 "r"(inside ? 8 : 0)
-                 : "memory");
-}
-
 template <int C>
 __global__ void __launch_bounds__(kSeedThreads)
     fp64_seed_kernel(const Fp64BandParams P, const double* __restrict__ Ah, int64_t nh,

@@ -75,14 +75,6 @@ __global__ void prescrimp_keys_init_kernel(unsigned long long* __restrict__ a, i
         a[i] = kNone;
 }
 
-// 8-byte asynchronous copy global -> shared that writes zero where !inside.
-static __device__ __forceinline__ void cp_async8_or_zero(double* dst, const double* src, bool inside) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
-                 "r"(inside ? 8 : 0)
-                 : "memory");
-}
-
 // Query rows: CTA b covers windows [wt*256, wt*256+256) and queries
 // [qt*32, qt*32+32), wt = b % window tiles, qt = b / window tiles (a 1-D grid,
 // so any number of queries fits).  The dot products are a matrix product,
