@@ -156,7 +156,10 @@ __device__ __forceinline__ void welford_chunk(const double* __restrict__ A, int6
 // units in the last place of a/b, a - b q is exact in one fused operation, and
 // RN(q + r (a - b q)) is the correctly rounded quotient (Markstein 1990), because
 // with b an integer a/b stays 1/(2b) of a unit away from every rounding boundary.
-// Outside the exponents where that holds, and for 0, the division itself is used.
+// Outside the exponents where that holds the division itself is used; 0 / b is 0 either way
+// (its sign, which the mean it is added to does not take on, may differ), and has to be
+// quick: lanes past the profile's end walk zeros (n = 5,000, m = 1200: 0.55 ms a call with
+// the division for them, 0.22 without).
 // A window is flat when the last change of value up to its end lies at or before its
 // start: a running maximum over the block's stretch in place of counts over the
 // whole series.
@@ -177,7 +180,7 @@ __device__ __forceinline__ double quotient(double a, double b, double r) {
     const double q = __dmul_rn(a, r);
     const double z = __fma_rn(__fma_rn(-b, q, a), r, q);
     const double x = fabs(a);
-    if (x <= 1e-280 || x >= 1e280) return plain_division(a, b);
+    if ((x <= 1e-280 && x != 0.0) || x >= 1e280) return plain_division(a, b);
     return z;  // NaN, too
 }
 __device__ __forceinline__ void stat_block(const double* __restrict__ A, int64_t m, int64_t PL, int64_t base,
