@@ -159,7 +159,7 @@ __device__ __forceinline__ void welford_chunk(const double* __restrict__ A, int6
 // Outside the exponents where that holds the division itself is used; 0 / b is 0 either way
 // (its sign, which the mean it is added to does not take on, may differ), and has to be
 // quick: lanes past the profile's end walk zeros (n = 5,000, m = 1200: 0.55 ms a call with
-// the division for them, 0.22 without).
+// the division for them, 0.25 without).
 // A window is flat when the last change of value up to its end lies at or before its
 // start: a running maximum over the block's stretch in place of counts over the
 // whole series.
